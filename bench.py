@@ -72,8 +72,8 @@ def parse_args():
                    help="FP64 apply form: canonical rotations (4 FP64 ops per rotation-row) or the "
                         "scaled form (2 FMAs per rotation-row; a few ulps from canonical)")
     p.add_argument("--chase-mode", type=int, choices=[0, 1, 2, 3], default=None,
-                   help="solve/dense workloads (default 0) and the adjoint's forward (default 3): 0 Newton-form "
-                        "two-warp chase, 1 reference form, 2 Newton + redo, 3 multishift batches")
+                   help="solve/dense workloads (default 0) and the adjoint's forward (default 3): 0 fixed-point "
+                        "rotations, 1 reference form, 2 as 0 + redo, 3 multishift batches")
     p.add_argument("--ms-bulges", type=int, default=64, help="solve workload, chase mode 3: bulge cap of a batch")
     p.add_argument("--ms-rows", type=int, default=16, help="solve workload, chase mode 3: block rows per bulge")
     p.add_argument("--ms-release", type=int, default=4, help="solve workload, chase mode 3: steps between progress releases")

@@ -51,7 +51,7 @@ typedef struct {
     int64_t wave_launches;   /* launches of the wave-window Givens kernel                 */
     double  wave_kernel_ms;  /* their summed device time (only with kernel timing on)     */
     int64_t device_errors;   /* nonzero if a kernel's bounded wait gave up (sticky)        */
-    int64_t redone_sweeps;   /* chase sweeps run again in the reference form (see below)  */
+    int64_t redone_sweeps;   /* sweeps chase mode 2 ran again in the reference form        */
     int64_t bulge_batches;   /* multishift batches the chase ran (chase mode 3)           */
 } symeig_stats;
 
@@ -74,11 +74,12 @@ int symeig_get_stats(symeig_handle h, symeig_stats* out);
 int symeig_set_exact_order(symeig_handle h, int32_t exact_order);
 /* How the chase kernel computes its rotations.  Modes 0-2 give the same bits: the reference's
  * sweep sequence and rotations.
- * 0 (default): two warps, givensAlgorithm's plain branch from FMA-only Newton steps whose
- *   rounding is proved step by step; a sweep with an unproved step is restored and run again
- *   in the reference form (counted in redone_sweeps).
+ * 0 (default): one warp, the square root and the quotients of givensAlgorithm's plain branch in
+ *   fixed-point arithmetic on the integer pipes, correctly rounded (the other branches in the
+ *   reference form), and the products of the 2x2 update side by side in its lanes.
  * 1: the reference form (correctly rounded division and square root) on one thread.
- * 2: as 0, but every sweep is then redone in the reference form (exercises the restore).
+ * 2: as 0, but every sweep is then undone and run again in the reference form (a self-check;
+ *   counted in redone_sweeps).
  * 3: multishift.  Where a block has at least 2 * 16 rows and room for several layers, the
  *   chase runs a batch of up to 64 sweeps (symeig_set_multishift) whose shifts are nb
  *   eigenvalues of the block's trailing window of 2 nb rows (those ranked about its bottom
@@ -333,7 +334,7 @@ int symeig_syev_f64_dev(symeig_handle h, int64_t n, double* A, int64_t lda, doub
 
 /* get_rotation(f, g) -> (c, s, r) (src/simple_givens.jl:20-23, LinearAlgebra.givensAlgorithm)
  * elementwise on `count` pairs, computed on the device the way the chase computes them (the
- * proved Newton form, or the reference form when symeig_set_chase_mode(h, 1)); both give the
+ * fixed-point form, or the reference form when symeig_set_chase_mode(h, 1)); both give the
  * reference's bits.  Host arrays (copied) or, for _dev, device arrays on the handle's stream. */
 int symeig_get_rotation_f64(symeig_handle h, int64_t count, const double* f, const double* g,
                             double* c, double* s, double* r);

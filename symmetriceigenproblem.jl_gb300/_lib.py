@@ -194,7 +194,7 @@ class Handle:
         check("symeig_set_multishift_min", self._lib.symeig_set_multishift_min(self.ptr, int(min_bulges)))
 
     def set_chase_mode(self, mode):
-        """0: Newton-form two-warp chase (default); 1: reference form; 2: Newton form with
+        """0: fixed-point rotations on one warp (default); 1: reference form; 2: as 0 with
         every sweep redone in the reference form -- these give the reference's bits; 3: the
         multishift chase (within the reference's error bounds)."""
         check("symeig_set_chase_mode", self._lib.symeig_set_chase_mode(self.ptr, int(mode)))

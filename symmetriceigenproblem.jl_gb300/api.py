@@ -91,7 +91,7 @@ def _colmajor_info(A):
 def get_rotation(f, g, handle: Handle | None = None, form: int = 0):
     """get_rotation(f, g) -> (c, s, r) elementwise (src/simple_givens.jl:20-23,
     LinearAlgebra.givensAlgorithm), computed on the device the way the chase computes them:
-    form 0 the proved Newton form, form 1 the reference form.  f, g: float64 numpy arrays
+    form 0 the fixed-point form, form 1 the reference form.  f, g: float64 numpy arrays
     (host) or CUDA tensors (device) of one shape."""
     dev = _is_torch(f)
     h = handle or default_handle(f.device.index if dev else 0)

@@ -4,8 +4,8 @@
 // the deflation scan (:205-222, is_offdiagonal_small :7-8), the layer capacity rule
 // (:226-230), the Wilkinson shift (:239-265) and single_shift! (:11-144) with
 // get_rotation / LinearAlgebra.givensAlgorithm (src/simple_givens.jl:20-23).  The sweep is a
-// strict dependency chain and runs on lane 0; the O(n) scans (deflation, thickest column)
-// use all 32 lanes with ballots.  Rotations go to a Julia-layout (c,s) grid: at
+// strict dependency chain and runs on one warp (sweep_warp); the O(n) scans (deflation, thickest
+// column) use all 32 lanes with ballots.  Rotations go to a Julia-layout (c,s) grid: at
 // grid[i, ++thickness[i]] as the reference records them, or (the default) at the sweep's
 // exact-order layer described at chase_kernel.
 //
@@ -20,6 +20,7 @@
 // reports CHASE_FLUSH, CHASE_CONVERGED or CHASE_MAXITER in ChaseState.
 #include "symeig_common.cuh"
 #include "givens.cuh"
+#include "givens_int.cuh"
 
 namespace symeig {
 
@@ -144,32 +145,166 @@ __device__ void single_shift(double* __restrict__ dv, double* __restrict__ ev, i
     }
 }
 
-// ---- the sweep on two warps, Newton-form rotations -------------------------------------
+// ---- the sweep on one warp ---------------------------------------------------------------
 //
 // single_shift! is one dependency chain per step: (f, g) -> r = sqrt(f^2 + g^2) -> c = f/r,
-// s = g/r -> the 2x2 update -> next (f, g).  On GB300 one warp issues an FP64 instruction
-// about every 64-90 cycles whatever their dependences, and the SM runs a few such warps at
-// once, so the step time is set by the FP64 instructions on the warp that carries the chain.
-// Here (the fastest split measured)
-//   warp 0 (the chain): the rotation by givens_nr_core (14 FP64 instructions), the four
-//           products of the 2x2 update that give the next f (B11', B12', B11'*s, B12'') and
-//           the next bulge g = s*ev[i+1] with g*g;
-//   warp 1: next B21 = c*ev[i+1] and the B21'/B22'/B22'' half of the update (-> next B11),
-//           B11'', the rounding proof of warp 0's rotation, every store and the record.
-// They trade values through a two-slot shared mailbox (slot = step parity) and two named
-// barriers, each used producer -> consumer (bar.arrive / bar.sync) and each strictly
-// alternating: warp 0 waits for B(i-1) before it arrives at CS(i), and warp 1 arrives at
-// B(i) only after CS(i).
-// Warp 0 does not wait for the proof.  Warp 1 records a failed proof (none was seen in 10^9
-// random rotations; see givens.cuh) and the kernel then restores the sweep's entries from a
-// copy taken before it and runs the sweep again in the reference form (single_shift), so the
-// result is bit-identical either way.  Steps whose (f, g) are outside the Newton form's range
-// take givens_fast on warp 0 and skip the proof.
+// s = g/r -> the 2x2 update -> next (f, g).  On GB300 a dependent FP64 instruction costs 64
+// cycles and a warp has one in flight at a time, whatever its active lanes; an FP64 result that
+// an integer instruction or a shuffle reads costs 40 more.  So a step is built of few FP64
+// instructions, each doing several products in different lanes:
+//   the rotation on the integer pipes in every lane (givens_int.cuh),
+//   level 1  p1 = m1 a1:        s B21 | s B22 | -s B11 | -s B21 | s B23 (next bulge) | -0
+//   level 2  v2 = c a2 + p1:    B11'  | B12'  | B21'   | B22'   | (bulge)            | c B23
+//   level 3  p3 = v2 m3:     -B11' s  | B12' s| -B21' s|        | bulge^2            |
+//   level 4  v4 = oth c + p3:  B12''  | B11'' | B22''                  (oth = v2 of lane ^ 1)
+//   lane (of 8)                  0    |   1   |   2    |   3    |   4                |   5
+// then x = B12''^2 + bulge^2 for the next rotation: six FP64 levels.  B22'' (lane 2) and c B23
+// (lane 5) are the next step's B11 and B21.  The lanes' operands are picked by bit masks: the
+// same selections written as ternaries compiled to divergent branches and cost 330 cycles.
+// The step's results go to memory during the next step: lane 1 stores dv, lane 2 ev, lanes 4
+// and 5 the pair (c, s), one masked store.  Measured 1077 cycles per step, against 1802 for the
+// two-warp Newton form this replaces and 1130 for a split over four warps with named barriers
+// (the warps' FP64 instructions queue for the SM's one unit).
+//
+// Step i (1-based, from .. to-1) is the reference's first rotation for i = from and its loop
+// body otherwise; both have the same 2x2 update.  Of the entries the reference writes and
+// later overwrites within the sweep only the final ones are stored: dv[from-1 .. to-1]
+// (0-based), ev[from-1 .. to-3] = the norms r of steps from+1 .. to-1 and ev[to-2] = the last
+// B12''.  The grid slot of rotation i is column `layer` (ONE_LAYER: exact order) or
+// thick[i-1] + 1 (the reference's placement; thick is updated by the caller after the sweep).
+// Every rotation is givensAlgorithm's, correctly rounded, so the bits are the reference's.
+__device__ __forceinline__ double lane_sel(uint32_t mask, double a, double b)
+{
+    const uint32_t lo = ((uint32_t)__double2loint(a) & mask) | ((uint32_t)__double2loint(b) & ~mask);
+    const uint32_t hi = ((uint32_t)__double2hiint(a) & mask) | ((uint32_t)__double2hiint(b) & ~mask);
+    return __hiloint2double((int)hi, (int)lo);
+}
+
+// x with the sign bit cleared where `keep` lacks it and flipped where `flip` has it
+__device__ __forceinline__ double lane_sign(double x, uint32_t keep, uint32_t flip)
+{
+    return __hiloint2double((int)(((uint32_t)__double2hiint(x) & keep) ^ flip), __double2loint(x));
+}
+
+// Store forced to a predicated instruction (no branch).
+__device__ __forceinline__ void st_if(double* p, double v, bool pred)
+{
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q st.global.f64 [%0], %1;\n\t}"
+                 ::"l"(p), "d"(v), "r"((unsigned)pred) : "memory");
+}
+
+__device__ __forceinline__ double lane_get(double v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
+
+// The lanes' roles (lane & 7) as masks and sign bits.
+struct SweepLanes {
+    uint32_t m0, m1, m2, m3, m4, m5;  // all ones in the lane of that role
+    uint32_t keep1, flip1, flip3;     // signs of s in levels 1 and 3
+};
+
+__device__ __forceinline__ SweepLanes sweep_lanes()
+{
+    const int role = threadIdx.x & 7;
+    const uint32_t sg = 0x80000000u;
+    SweepLanes L;
+    L.m0 = role == 0 ? ~0u : 0u;
+    L.m1 = role == 1 ? ~0u : 0u;
+    L.m2 = role == 2 ? ~0u : 0u;
+    L.m3 = role == 3 ? ~0u : 0u;
+    L.m4 = role == 4 ? ~0u : 0u;
+    L.m5 = role == 5 ? ~0u : 0u;
+    L.keep1 = role == 5 ? ~sg : ~0u;   // |s| times -0 is -0, so lane 5's level 2 is c B23 exactly
+    L.flip1 = (role == 2 || role == 3) ? sg : 0u;
+    L.flip3 = (role == 0 || role == 2) ? sg : 0u;
+    return L;
+}
+
+// Levels 1 to 4 of a step (see above): v2, v4 per lane, and the next bulge g with gg = g^2.
+__device__ __forceinline__ void sweep_update(const SweepLanes& L, double c, double s, double a1, double a2,
+                                             double nz, double& v2, double& v4, double& g, double& gg)
+{
+    const double p1 = __fma_rn(lane_sign(s, L.keep1, L.flip1), a1, nz);
+    v2 = __fma_rn(c, a2, p1);
+    const double m3 = lane_sel(L.m4, p1, lane_sign(s, ~0u, L.flip3));
+    const double p3 = __fma_rn(v2, m3, nz);
+    const double oth = __shfl_xor_sync(0xffffffffu, v2, 1);
+    v4 = __fma_rn(oth, c, p3);
+    g = lane_get(p1, 4);
+    gg = lane_get(p3, 4);
+}
+
+template <bool ONE_LAYER>
+__device__ void sweep_warp(double* __restrict__ dv, double* __restrict__ ev, int64_t from, int64_t to,
+                           double mu, double* __restrict__ grid, const int32_t* __restrict__ thick,
+                           int64_t rows, int32_t layer, double nz)
+{
+    const int lane = threadIdx.x & 31, role = lane & 7;
+    const SweepLanes L = sweep_lanes();
+    const int steps = (int)(to - from);
+    const double H11 = dv[from - 1], H21 = ev[from - 1];
+    double f = __dsub_rn(H11, mu), g = H21;
+    double x = __dadd_rn(mulz(f, f, nz), mulz(g, g, nz));
+    double B22n = dv[from], B23n = 2 <= steps ? ev[from] : 0.0;
+    double v4 = H11, v2 = H21;   // lane 2's v4 is B11, lane 5's v2 is B21
+    // where this lane's result of the step before the current one goes
+    double* out = role == 1 ? dv + from - 2 : role == 2 ? ev + from - 3
+                                            : grid + 2 * ((from - 2) + (int64_t)(layer - 1) * rows) + (role == 5);
+    const int out_step = role >= 4 ? 2 : 1;
+    const bool stores = lane == 1 || lane == 2 || lane == 4 || lane == 5;
+    const double *ld = dv + from + 1, *le = ev + from + 1;   // entries of step k + 1
+    double c_out = 0.0, s_out = 0.0, r_out = 0.0;
+    int32_t t_out = 0, t_cur = 0, t_next = 0;   // thick of the stored, the current and the next rotation
+    if (!ONE_LAYER) t_cur = thick[from - 1];
+#pragma unroll 1
+    for (int k = 0; k < steps; ++k) {
+        const double B22 = B22n, B23 = B23n;
+        double c, s, r;
+        IntRot K;
+        givens_int(f, g, x, c, s, r, K);
+        B22n = k + 2 <= steps ? *ld : 0.0;
+        B23n = k + 3 <= steps ? *le : 0.0;
+        ++ld;
+        ++le;
+        if (!ONE_LAYER) t_next = k + 2 <= steps ? thick[from + k] : 0;
+        const double B11 = lane_get(v4, 2), B21 = lane_get(v2, 5);
+        {
+            const double v = lane_sel(L.m1, v4, lane_sel(L.m2, r_out, lane_sel(L.m4, c_out, s_out)));
+            double* p = out;
+            if (!ONE_LAYER && role >= 4) p += (int64_t)(t_out + 1 - layer) * 2 * rows;
+            st_if(p, v, stores && k > 0 && !(role == 2 && k == 1));
+            out += out_step;
+        }
+        const double a1 = lane_sel(L.m1, B22, lane_sel(L.m2, B11, lane_sel(L.m5, -0.0, lane_sel(L.m4, B23, B21))));
+        const double a2 = lane_sel(L.m0, B11, lane_sel(L.m3, B22, lane_sel(L.m5, B23, lane_sel(L.m4, 0.0, B21))));
+        double gn, ggn;
+        sweep_update(L, c, s, a1, a2, nz, v2, v4, gn, ggn);
+        if (__any_sync(0xffffffffu, !K.in_range || K.undecided != 0u)) {
+            const Rot3 o = givens_fix(f, g, K, nz);
+            c = o.c; s = o.s; r = o.r;
+            sweep_update(L, c, s, a1, a2, nz, v2, v4, gn, ggn);
+        }
+        f = lane_get(v4, 0);
+        x = __dadd_rn(mulz(f, f, nz), ggn);
+        g = gn;
+        c_out = c; s_out = s; r_out = r;
+        t_out = t_cur;
+        t_cur = t_next;
+    }
+    {
+        const double v = lane_sel(L.m1, v4, lane_sel(L.m2, r_out, lane_sel(L.m4, c_out, s_out)));
+        double* p = out;
+        if (!ONE_LAYER && role >= 4) p += (int64_t)(t_out + 1 - layer) * 2 * rows;
+        st_if(p, v, stores && !(role == 2 && steps == 1));
+        st_if(dv + to - 1, v4, lane == 2);
+        st_if(ev + to - 2, f, lane == 0);
+    }
+    __syncwarp();
+}
+
+// Two-warp mailbox and named barriers of the bulges' sweep (sweep_bulge_2w).
 enum : int { kBarCS = 1, kBarB = 2 };
 
 struct NrMail {
-    double c, s, r, x, f, g;  // warp 0 -> 1 (kBarCS); r with the sign convention applied
-    int32_t slow;             // 1: (c, s, r) from givens_fast, nothing to prove
+    double c, s, r;           // warp 0 -> 1 (kBarCS); r with the sign convention applied
     double b22pp, e_next;     // warp 1 -> 0 (kBarB): next B11, next B21
 };
 
@@ -180,103 +315,6 @@ __device__ __forceinline__ void nb_sync(int id)
 __device__ __forceinline__ void nb_arrive(int id)
 {
     asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory");
-}
-
-// single_shift!(H, from, to, mu, givens, layer_thickness) (src/bulge_chasing.jl:11-144) by
-// both warps of the CTA.  Step i (1-based, from .. to-1) is the reference's first rotation
-// for i = from and its loop body otherwise; both have the same 2x2 update.  Of the entries the
-// reference writes and later overwrites within the sweep only the final ones are stored:
-// dv[from-1 .. to-1] (0-based), ev[from-1 .. to-3] = the norms r of steps from+1 .. to-1 and
-// ev[to-2] = the last B12''.  The grid slot of rotation i is column `layer` (exact order) or
-// thick[i-1] + 1 (the reference's placement; thick is updated by the caller after the sweep).
-// *fail is set when a Newton-form rotation could not be proved.
-__device__ void sweep_nr_2w(double* __restrict__ dv, double* __restrict__ ev, int64_t from,
-                            int64_t to, double mu, double* __restrict__ grid,
-                            const int32_t* __restrict__ thick, int64_t rows, int32_t layer,
-                            double nz, NrMail* mail, int32_t* fail)
-{
-    const int warp = threadIdx.x >> 5;
-    const bool lead = (threadIdx.x & 31) == 0;
-    const double H11 = dv[from - 1], H21 = ev[from - 1];
-    if (warp == 0) {
-        double f = __dsub_rn(H11, mu), g = H21, gg = mulz(H21, H21, nz);
-        double B11 = H11, B21 = H21;
-        double B22n = dv[from];                                  // dv[i+1] (1-based) for step i
-        double B23n = (from + 2 <= to) ? ev[from] : 0.0;         // ev[i+1] (1-based) for step i
-        for (int64_t i = from; i <= to - 1; ++i) {
-            const double B22 = B22n, B23 = B23n;
-            if (i + 1 <= to - 1) B22n = dv[i + 1];
-            if (i + 3 <= to) B23n = ev[i + 1];
-            // the Newton form whatever the range (no branch before the chain), then the
-            // reference form when the inputs are out of its range
-            const NrRot o = givens_nr_core(f, g, gg, nz);
-            double c = o.c, s = o.s, r = o.r;
-            int32_t slow = 0;
-            if (!nr_in_range(f, g)) {
-                givens_fast(f, g, c, s, r, nz);
-                slow = 1;
-            }
-            if (i > from) {
-                nb_sync(kBarB);
-                const NrMail& pv = mail[(i - 1) & 1];
-                B11 = pv.b22pp;
-                B21 = pv.e_next;
-            }
-            NrMail& mb = mail[i & 1];
-            mb.c = c; mb.s = s; mb.r = r; mb.x = o.x; mb.f = f; mb.g = g; mb.slow = slow;
-            nb_arrive(kBarCS);
-            const double B11p = __fma_rn(c, B11, mulz(s, B21, nz));
-            const double B12p = __fma_rn(c, B21, mulz(s, B22, nz));
-            f = __fma_rn(B12p, c, -mulz(B11p, s, nz));
-            g = (i + 2 <= to) ? mulz(s, B23, nz) : 0.0;
-            gg = mulz(g, g, nz);
-        }
-    } else {
-        double B11 = H11, B21 = H21;
-        double B22n = dv[from];
-        double B23n = (from + 2 <= to) ? ev[from] : 0.0;
-        int32_t thn = layer <= 0 ? thick[from - 1] : 0;
-        bool bad = false;
-        for (int64_t i = from; i <= to - 1; ++i) {
-            const double B22 = B22n, B23 = B23n;
-            const int32_t th = thn;
-            if (i + 1 <= to - 1) B22n = dv[i + 1];
-            if (i + 3 <= to) B23n = ev[i + 1];
-            if (layer <= 0 && i + 1 <= to - 1) thn = thick[i];
-            nb_sync(kBarCS);
-            NrMail& mb = mail[i & 1];
-            const double c = mb.c, s = mb.s, r = mb.r, x = mb.x, f = mb.f, g = mb.g;
-            const int32_t slow = mb.slow;
-            const double e_next = (i + 2 <= to) ? mulz(c, B23, nz) : 0.0;
-            const double sB21 = mulz(s, B21, nz);
-            const double B21p = __fma_rn(c, B21, -mulz(s, B11, nz));
-            const double B22p = __fma_rn(c, B22, -sB21);
-            const double B22pp = __fma_rn(B22p, c, -mulz(B21p, s, nz));
-            if (i < to - 1) {
-                mb.b22pp = B22pp;
-                mb.e_next = e_next;
-                nb_arrive(kBarB);
-            }
-            const double B11p = __fma_rn(c, B11, sB21);
-            const double B12p = __fma_rn(c, B21, mulz(s, B22, nz));
-            const double B11pp = __fma_rn(B11p, c, mulz(B12p, s, nz));
-            if (!slow && !givens_nr_proved(f, g, x, c, s, r)) bad = true;
-            if (lead) {
-                dv[i - 1] = B11pp;
-                if (i > from) ev[i - 2] = r;
-                const int32_t L = layer > 0 ? layer : th + 1;
-                *reinterpret_cast<double2*>(grid + 2 * ((i - 1) + (int64_t)(L - 1) * rows)) =
-                    make_double2(c, s);
-                if (i == to - 1) {
-                    dv[i] = B22pp;
-                    ev[i - 1] = __fma_rn(B12p, c, -mulz(B11p, s, nz));
-                }
-            }
-            B11 = B22pp;
-            B21 = e_next;
-        }
-        if (lead && bad) *fail = 1;
-    }
 }
 
 constexpr int kScanUnroll = 8;  // chunks of 32 entries per round of the deflation scan
@@ -483,9 +521,10 @@ __device__ void batch_shifts_solve(const double* __restrict__ dv, int64_t to, in
     }
 }
 
-// The bulges of a batch.  Bulge j (CTA j) runs the two-warp sweep of sweep_nr_2w (same split,
-// mailbox and barriers) with shift shifts[j] over the batch's block, a few steps behind bulge
-// j-1, reading only what bulge j-1 has stored: step k of a sweep stores dv[k-1] and ev[k-2] (0-based; its last step also
+// The bulges of a batch.  Bulge j (CTA j) runs a sweep on two warps -- warp 0 the rotation and
+// the products that lead to the next one, warp 1 the rest of the update and the stores, values
+// traded through a two-slot mailbox and two alternating named barriers -- with shift shifts[j]
+// over the batch's block, a few steps behind bulge j-1, reading only what bulge j-1 has stored: step k of a sweep stores dv[k-1] and ev[k-2] (0-based; its last step also
 // dv[k] and ev[k-1]), so before its loads for step i+1 (dv[i+1], ev[i+1]) bulge j needs bulge
 // j-1 through step min(i+3, to-1).  The helper warp's store thread releases the bulge's
 // progress every (prog_mask + 1) steps and at its last step (st.release.gpu); the next bulge's
@@ -652,8 +691,10 @@ bulge_batch_kernel(const ChaseState* __restrict__ st, double* __restrict__ dv,
 
 // One flush: the reference's inner loop from `to = last_block_ends_at` until the matrix is
 // split into converged parts, every block has reached max_layers, or iter > maxiter.
-// Warp 0 runs the control flow and the O(n) scans with ballots; each sweep runs on both
-// warps (sweep_nr_2w) after both copy the entries it may change to `bak` (2n doubles).
+// Warp 0 runs the control flow, the O(n) scans with ballots and the sweeps (sweep_warp); warp 1
+// shares the O(n) updates and the shift solve.  In chase modes 1 and 2 every sweep runs in the
+// reference form on one thread (mode 2: after the warp's sweep, undone from the copy `bak`, 2n
+// doubles, of the entries it may change).
 //
 // Exact-order placement (st->exact_order != 0).  The reference applies a flush's grid in
 // layer-major order, which equals the order the chase made the rotations only while every
@@ -677,9 +718,7 @@ chase_kernel(ChaseState* __restrict__ st, double* __restrict__ dv, double* __res
              double* __restrict__ grid, int32_t* __restrict__ thick, int32_t* __restrict__ place,
              double* __restrict__ bak, BulgeScratch* __restrict__ bs, int32_t resume_only)
 {
-    __shared__ NrMail mail[2];
     __shared__ Decision dec;
-    __shared__ int32_t fail;
     __shared__ float ms_d[kWinMax], ms_e2[kWinMax], ms_ea[kWinMax];
     __shared__ double ms_dd[kWinMax], ms_ee2[kWinMax];
     __shared__ ShiftWindow swin;
@@ -721,7 +760,6 @@ chase_kernel(ChaseState* __restrict__ st, double* __restrict__ dv, double* __res
             place[q] = L0 > 0 ? L0 + nbk - 1 : t;
         }
     }
-    if (threadIdx.x == 0) fail = 0;
     __syncthreads();
 
     bool did = resume && st->r_did != 0;
@@ -845,17 +883,21 @@ chase_kernel(ChaseState* __restrict__ st, double* __restrict__ dv, double* __res
         if (d.action == 1) {
             // entries the sweep may change: dv[from-1 .. to-1], ev[from-1 .. to-2] (0-based)
             const int64_t q0 = d.from - 1, q1 = d.to - 1;
-            bool redo = mode == 1;
-            if (mode != 1) {
+            const bool redo = mode == 1 || mode == 2;
+            if (mode == 2) {
                 for (int64_t q = q0 + threadIdx.x; q <= q1; q += 64) {
                     bak[q] = dv[q];
                     if (q < q1) bak[n + q] = ev[q];
                 }
                 __syncthreads();
-                sweep_nr_2w(dv, ev, d.from, d.to, d.mu, grid, thick, rows, d.layer, nz, mail, &fail);
+            }
+            if (mode != 1) {
+                if (warp == 0) {
+                    if (d.layer > 0) sweep_warp<true>(dv, ev, d.from, d.to, d.mu, grid, thick, rows, d.layer, nz);
+                    else sweep_warp<false>(dv, ev, d.from, d.to, d.mu, grid, thick, rows, d.layer, nz);
+                }
                 __syncthreads();
-                redo = fail != 0 || mode == 2;
-                if (redo) {
+                if (mode == 2) {
                     for (int64_t q = q0 + threadIdx.x; q <= q1; q += 64) {
                         dv[q] = bak[q];
                         if (q < q1) ev[q] = bak[n + q];
@@ -868,7 +910,6 @@ chase_kernel(ChaseState* __restrict__ st, double* __restrict__ dv, double* __res
                 __syncthreads();
                 if (threadIdx.x == 0)
                     single_shift<false>(dv, ev, d.from, d.to, d.mu, grid, thick, place, rows, d.layer, nz);
-                if (threadIdx.x == 0) fail = 0;
             } else {
                 for (int64_t q = q0 + threadIdx.x; q < q1; q += 64) {
                     const int32_t t = thick[q] + 1;
@@ -1028,8 +1069,8 @@ chase_batched_kernel(const BatchMat* __restrict__ mats, const int32_t* __restric
     chase_flush_lane(st, d + mt.doff, e + mt.eoff, grids + mt.goff, thick + mt.doff, place + mt.doff);
 }
 
-// get_rotation(f, g) (src/simple_givens.jl:20-23) elementwise: form 0 the chase's Newton form
-// (givens_nr), form 1 the reference form (givens).
+// get_rotation(f, g) (src/simple_givens.jl:20-23) elementwise: form 0 as the chase computes it
+// (givens_int.cuh), form 1 the reference form (givens).
 __global__ void get_rotation_kernel(int64_t count, const double* __restrict__ f,
                                     const double* __restrict__ g, double* __restrict__ c,
                                     double* __restrict__ s, double* __restrict__ r, int32_t form,
@@ -1040,7 +1081,10 @@ __global__ void get_rotation_kernel(int64_t count, const double* __restrict__ f,
         const double fi = f[i], gi = g[i];
         double ci, si, ri;
         if (form == 1) givens(fi, gi, ci, si, ri);
-        else givens_nr(fi, gi, mulz(gi, gi, nz), ci, si, ri, nz);
+        else {
+            const Rot3 o = givens_any(fi, gi, nz);
+            ci = o.c; si = o.s; ri = o.r;
+        }
         c[i] = ci;
         s[i] = si;
         r[i] = ri;

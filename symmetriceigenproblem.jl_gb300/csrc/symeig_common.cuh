@@ -93,8 +93,8 @@ struct ChaseState {
     int64_t total_rotations;
     int64_t early_flushes;       // flushes ended because a sweep's layer exceeded grid_layers
     double  neg_zero;            // -0.0, supplied at run time (see mulz in givens.cuh)
-    int32_t chase_mode;          // 0 Newton-form two-warp sweeps, 1 reference form on one
-                                 // thread, 2 Newton form with every sweep redone (tests)
+    int32_t chase_mode;          // 0 fixed-point rotations, 1 reference form on one
+                                 // thread, 2 as 0 with every sweep redone as 1 (tests)
     int32_t pad0;
     int64_t redone_sweeps;       // sweeps run again in the reference form (cumulative)
     // chase_mode 3: the pending batch and the flush's loop state to resume after it
@@ -204,7 +204,7 @@ cudaError_t launch_tridiag_unscale(double* A, int64_t lda, int64_t n, double* d,
 // a[i] * b[i] elementwise: form 0 the canonical apply's integer-pipe products, 1 the FP64 pipe.
 cudaError_t launch_mul_rn(int64_t count, const double* a, const double* b, double* out, int32_t form,
                           cudaStream_t stream);
-// givensAlgorithm elementwise on device arrays (form 0 Newton form, 1 reference form).
+// givensAlgorithm elementwise on device arrays (form 0 as the chase, 1 reference form).
 cudaError_t launch_get_rotation(int64_t count, const double* f, const double* g, double* c,
                                 double* s, double* r, int32_t form, cudaStream_t stream);
 // resume_only: run only if a multishift batch is pending resumption (else return at once).

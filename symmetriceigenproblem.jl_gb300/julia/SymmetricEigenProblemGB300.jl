@@ -197,7 +197,7 @@ end
 set_apply_form!(form::Integer) =
     check(:symeig_set_apply_form, ccall((:symeig_set_apply_form, libsymeig), Cint, (Ptr{Cvoid}, Int32), handle(), form))
 
-"""0: Newton-form two-warp chase (default); 1: reference form; 2: Newton form with every
+"""0: fixed-point rotations on one warp (default); 1: reference form; 2: as 0 with every
 sweep redone in the reference form -- these three give the reference's bits.  3: multishift
 batches of concurrent bulges (within the reference's error bounds, not its bits; about 8x
 faster at n = 16384)."""
