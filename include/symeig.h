@@ -192,7 +192,7 @@ int symeig_apply_givens_f32_dev(symeig_handle h, float* A, int64_t lda, int64_t 
  * column-major, leading dimension n_i, overwritten with Q_i * prod(G)) at
  * Q[sum_{j<i} n_j^2 ...]; Q may be NULL (eigenvalues only).  n, converged and iters are host
  * arrays of count entries.  The reference has no batched entry point; this replaces a loop of
- * qr_algorithm! calls.  Matrices run one flush per round: a one-lane-per-matrix chase, then
+ * qr_algorithm! calls.  Matrices run one flush per round: a one-warp-per-matrix chase, then
  * a persistent wave-kernel launch over a device-built queue of (matrix, row tile) items.  Each
  * round's apply runs beside the next round's chase (double-buffered rotation grids); the
  * rounds are captured as CUDA graphs and replayed until every matrix has finished.  Device

@@ -3,9 +3,9 @@
 //
 // The reference solves one matrix per call (src/bulge_chasing.jl:146).  A batch here runs
 // in rounds; each round is one flush of every unfinished matrix:
-//   1. chase: one lane per matrix runs the reference's inner loop until its rotation buffer
-//      is full or it converges (chase.cu, chase_batched_kernel).  Lanes are assigned in
-//      order of decreasing n so that a warp's 32 chases sweep similar lengths.
+//   1. chase: one warp per matrix runs the reference's inner loop until its rotation buffer
+//      is full or it converges (chase.cu, chase_batched_kernel).  Warps are assigned in
+//      order of decreasing n, so that the longest chases start first.
 //   2. worklist (one CTA): for every matrix with rotations, the column range and layer
 //      count of its flush, its number of row tiles, and exclusive prefix sums of tiles per
 //      (pass, size class) -- the work queue of (matrix, row-tile) items -- and the number of
@@ -348,7 +348,7 @@ int qr_batched_dev(int device, cudaStream_t stream, int64_t count, const int64_t
         s.neg_zero = -0.0;
         states[i] = s;
     }
-    // lanes in order of decreasing n (stable), so that a warp's chases have similar lengths
+    // warps in order of decreasing n (stable), so that the longest chases start first
     std::vector<int32_t> order(count);
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return n[a] > n[b]; });
@@ -405,8 +405,8 @@ int qr_batched_dev(int device, cudaStream_t stream, int64_t count, const int64_t
         // Rounds are pipelined: round r's apply (its rotations in grid buffer r % 2) runs beside
         // round r + 1's chase (into the other buffer).  The chase never reads Q and the apply
         // never reads the chase states: the work list snapshots round r's flushes before the
-        // next chase starts.  The lane-per-matrix chase is as long as the batch's largest
-        // sweeps and holds few warps, the apply fills the GPU, so the two overlap well.
+        // next chase starts.  The chase's warps wait on long dependent chains, the apply fills
+        // the pipes, so the two overlap well.
         // Round 0's chase runs first; graph b (b = r % 2) then runs, per round r,
         //   work list (round r) -> [ tables + wave passes on buffer b  ||  chase into buffer 1-b ]
         // and copies the number of matrices still active after chase r to the host.  The loop

@@ -79,8 +79,6 @@ __device__ __forceinline__ void record(double* grid, int32_t* thick, int32_t* pl
 // single_shift!(H, from, to, mu, givens, layer_thickness) (src/bulge_chasing.jl:11-144).
 // dv/ev are 0-based arrays; from/to 1-based.  Values the sweep itself produced travel in
 // registers; only untouched entries are loaded.
-// NR = true computes each rotation by givens_nr (proved Newton form, else the reference form).
-template <bool NR>
 __device__ void single_shift(double* __restrict__ dv, double* __restrict__ ev, int64_t from,
                              int64_t to, double mu, double* __restrict__ grid,
                              int32_t* __restrict__ thick, int32_t* __restrict__ place,
@@ -88,8 +86,7 @@ __device__ void single_shift(double* __restrict__ dv, double* __restrict__ ev, i
 {
     const double H11 = dv[from - 1], H21 = ev[from - 1], H22 = dv[from];
     double c, s, nrm;
-    if (NR) givens_nr(__dsub_rn(H11, mu), H21, mulz(H21, H21, nz), c, s, nrm, nz);
-    else givens_fast(__dsub_rn(H11, mu), H21, c, s, nrm, nz);
+    givens_fast(__dsub_rn(H11, mu), H21, c, s, nrm, nz);
     const double H11p = fsum(c, H11, s, H21, nz);
     const double H21p = fdif(c, H21, s, H11, nz);
     const double H12p = fsum(c, H21, s, H22, nz);
@@ -120,8 +117,7 @@ __device__ void single_shift(double* __restrict__ dv, double* __restrict__ ev, i
         // prefetch for step i+1: dv[i+2], ev[i+2] (1-based)
         if (i + 1 <= to - 1) B22_n = dv[i + 1];
         if (i + 3 <= to) B23_n = ev[i + 1];
-        if (NR) givens_nr(p1, bulge, mulz(bulge, bulge, nz), c, s, nrm, nz);
-        else givens_fast(p1, bulge, c, s, nrm, nz);
+        givens_fast(p1, bulge, c, s, nrm, nz);
         ev[i - 2] = nrm;
         const double B21 = e_next;
         const double B11p = fsum(c, B11, s, B21, nz);
@@ -321,9 +317,59 @@ constexpr int kScanUnroll = 8;  // chunks of 32 entries per round of the deflati
 
 __device__ __forceinline__ int32_t warp_max(int32_t v)
 {
+    return __reduce_max_sync(0xffffffffu, v);
+}
+
+// The start of the unreduced block that ends at `to`: the largest j+1 with is_small(j), j in
+// [start, to-1], or start.  kScanUnroll chunks of 32 per round: their loads are issued
+// together, so a long block costs one memory latency per 32 * kScanUnroll entries.
+__device__ __forceinline__ int64_t block_start(const double* dv, const double* ev, int64_t start, int64_t to,
+                                               double tol)
+{
+    const int lane = threadIdx.x & 31;
+    for (int64_t base = to - 1; base >= start; base -= 32 * kScanUnroll) {
+        bool sm[kScanUnroll];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
+        for (int u = 0; u < kScanUnroll; ++u) {
+            const int64_t j = base - 32 * u - lane;
+            sm[u] = (j >= start) && is_small(dv, ev, j, tol);
+        }
+#pragma unroll
+        for (int u = 0; u < kScanUnroll; ++u) {
+            const unsigned mask = __ballot_sync(0xffffffffu, sm[u]);
+            if (mask) return base - 32 * u - (__ffs(mask) - 1) + 1;
+        }
+    }
+    return start;
+}
+
+// max(0, a[lo .. hi]) by a warp
+__device__ __forceinline__ int32_t warp_range_max(const int32_t* a, int64_t lo, int64_t hi)
+{
+    int32_t v = 0;
+#pragma unroll 8
+    for (int64_t q = lo + (threadIdx.x & 31); q <= hi; q += 32) v = max(v, a[q]);
+    return warp_max(v);
+}
+
+// The exact-order layer of a sweep over [from, to] (see chase_kernel), and the identity in the
+// slots the jump to it skips.
+__device__ __forceinline__ int32_t exact_layer(const int32_t* place, int64_t from, int64_t to, int64_t n)
+{
+    int32_t L = warp_range_max(place, from - 1, to - 2);
+    if (to <= n - 1) L = max(L, place[to - 1]);
+    if (from >= 2) L = max(L, place[from - 2] - 1);
+    return L + 1;
+}
+__device__ __forceinline__ void fill_skipped(double* grid, const int32_t* place, int64_t from, int64_t to,
+                                             int32_t layer, int64_t rows)
+{
+    for (int64_t q = from - 1 + (threadIdx.x & 31); q <= to - 2; q += 32)
+        for (int32_t g = place[q] + 1; g < layer; ++g) {
+            double* p = grid + 2 * (q + (int64_t)(g - 1) * rows);
+            p[0] = 1.0;
+            p[1] = 0.0;
+        }
 }
 
 // ---- multishift batches (chase_mode 3) -----------------------------------------------------
@@ -778,62 +824,26 @@ chase_kernel(ChaseState* __restrict__ st, double* __restrict__ dv, double* __res
             } else if (to <= start) {
                 d.action = 0;
             } else {
-                // from = largest j+1 with is_small(j), j in [start, to-1]; start if none.
-                // kScanUnroll chunks of 32 per round: their loads are issued together, so a
-                // long block costs one memory latency per 32 * kScanUnroll entries.
-                int64_t from = start;
-                for (int64_t base = to - 1; base >= start; base -= 32 * kScanUnroll) {
-                    bool sm[kScanUnroll];
-#pragma unroll
-                    for (int u = 0; u < kScanUnroll; ++u) {
-                        const int64_t j = base - 32 * u - lane;
-                        sm[u] = (j >= start) && is_small(dv, ev, j, tol);
-                    }
-                    bool found = false;
-#pragma unroll
-                    for (int u = 0; u < kScanUnroll; ++u) {
-                        const unsigned mask = __ballot_sync(0xffffffffu, sm[u]);
-                        if (!found && mask) {
-                            from = base - 32 * u - (__ffs(mask) - 1) + 1;
-                            found = true;
-                        }
-                    }
-                    if (found) break;
-                }
+                const int64_t from = block_start(dv, ev, start, to, tol);
                 if (from == to) {
                     if (lane == 0) ev[from - 2] = 0.0;
                     if (to == lbe) lbe -= 1;
                     to -= 1;
                 } else {
-                    int32_t mx = 0;
-#pragma unroll 8
-                    for (int64_t q = from - 1 + lane; q <= to - 1; q += 32) mx = max(mx, thick[q]);
-                    mx = warp_max(mx);
+                    const int32_t mx = warp_range_max(thick, from - 1, to - 1);
                     if (mx == max_layers) {
                         to = from - 1;
                     } else {
                         int32_t layer = 0;
                         bool go = true;
                         if (exact) {
-                            int32_t L = 0;
-#pragma unroll 8
-                            for (int64_t q = from - 1 + lane; q <= to - 2; q += 32) L = max(L, place[q]);
-                            L = warp_max(L);
-                            if (to <= n - 1) L = max(L, place[to - 1]);
-                            if (from >= 2) L = max(L, place[from - 2] - 1);
-                            layer = L + 1;
+                            layer = exact_layer(place, from, to, n);
                             if (layer > grid_layers) {
                                 early = 1;
                                 go = false;
                                 d.action = 0;
                             } else {
-                                // slots skipped by the jump to `layer` hold the identity
-                                for (int64_t q = from - 1 + lane; q <= to - 2; q += 32)
-                                    for (int32_t g = place[q] + 1; g < layer; ++g) {
-                                        double* p = grid + 2 * (q + (int64_t)(g - 1) * rows);
-                                        p[0] = 1.0;
-                                        p[1] = 0.0;
-                                    }
+                                fill_skipped(grid, place, from, to, layer, rows);
                             }
                         }
                         if (go) {
@@ -909,7 +919,7 @@ chase_kernel(ChaseState* __restrict__ st, double* __restrict__ dv, double* __res
                 // the reference form on one thread; it updates thick/place itself
                 __syncthreads();
                 if (threadIdx.x == 0)
-                    single_shift<false>(dv, ev, d.from, d.to, d.mu, grid, thick, place, rows, d.layer, nz);
+                    single_shift(dv, ev, d.from, d.to, d.mu, grid, thick, place, rows, d.layer, nz);
             } else {
                 for (int64_t q = q0 + threadIdx.x; q < q1; q += 64) {
                     const int32_t t = thick[q] + 1;
@@ -966,22 +976,25 @@ chase_kernel(ChaseState* __restrict__ st, double* __restrict__ dv, double* __res
     }
 }
 
-// ---- batched chase: one lane per matrix --------------------------------------------------
+// ---- batched chase: one warp per matrix ---------------------------------------------------
 //
-// A chase step is a chain of ~55 dependent FP64 operations, and on GB300 an FP64 instruction
-// occupies its sub-partition's FP64 unit for 64 cycles whether 1 or 32 lanes are active.  So
-// for many independent matrices each lane runs its own matrix's flush: 32 chases share every
-// FP64 instruction.  The host sorts matrices by size so that a warp's lanes sweep similar
-// lengths.  The scans (deflation, thickest column, exact-order layer) are serial per lane.
+// Each warp runs its own matrix's flush with the one-warp sweep: its six FP64 instructions per
+// step (64 cycles each) leave the FP64 unit of the SM room for the warps beside it, the scans
+// use all lanes, and no matrix waits for another's sweep length.  One lane per matrix, which
+// this replaces, shared every FP64 instruction among 32 chases but ran the warp's longest
+// sweeps and serial scans for all of them (256 matrices of n = 32 .. 320 with FP64 Q, the whole
+// call: 354 ms, 79 ms with one warp per matrix).
 
-// One flush of one matrix (the same steps, in the same order, as chase_kernel).
-__device__ void chase_flush_lane(ChaseState* __restrict__ st, double* __restrict__ dv,
+// One flush of one matrix by one warp (the same steps, in the same order, as chase_kernel).
+__device__ void chase_flush_warp(ChaseState* __restrict__ st, double* __restrict__ dv,
                                  double* __restrict__ ev, double* __restrict__ grid,
                                  int32_t* __restrict__ thick, int32_t* __restrict__ place)
 {
+    const int lane = threadIdx.x & 31;
     const int64_t n = st->n;
     const int64_t start = st->start;
     const double tol = st->tol;
+    const double nz = st->neg_zero;
     const int32_t max_layers = st->max_layers;
     const int32_t grid_layers = st->grid_layers;
     const bool exact = st->exact_order != 0;
@@ -990,10 +1003,11 @@ __device__ void chase_flush_lane(ChaseState* __restrict__ st, double* __restrict
     int64_t lbe = st->last_block_ends_at;
     const int64_t rows = n > 1 ? n - 1 : 1;
 
-    for (int64_t q = 0; q < n; ++q) {
+    for (int64_t q = lane; q < n; q += 32) {
         thick[q] = 0;
         place[q] = 0;
     }
+    __syncwarp();
     bool did = false;
     int64_t rotations = 0, min_from = n + 1, max_to = 0, early = 0;
     int32_t status = CHASE_RUNNING;
@@ -1001,35 +1015,32 @@ __device__ void chase_flush_lane(ChaseState* __restrict__ st, double* __restrict
     for (;;) {
         if (iter > maxiter) { status = CHASE_MAXITER; break; }
         if (to <= start) break;
-        int64_t from = to;
-        while (from > start && !is_small(dv, ev, from - 1, tol)) from -= 1;
+        const int64_t from = block_start(dv, ev, start, to, tol);
         if (from == to) {
-            ev[from - 2] = 0.0;
+            if (lane == 0) ev[from - 2] = 0.0;
+            __syncwarp();
             if (to == lbe) lbe -= 1;
             to -= 1;
         } else {
-            int32_t mx = 0;
-            for (int64_t q = from - 1; q <= to - 1; ++q) mx = max(mx, thick[q]);
+            const int32_t mx = warp_range_max(thick, from - 1, to - 1);
             if (mx == max_layers) {
                 to = from - 1;
             } else {
                 int32_t layer = 0;
                 if (exact) {
-                    int32_t L = 0;
-                    for (int64_t q = from - 1; q <= to - 2; ++q) L = max(L, place[q]);
-                    if (to <= n - 1) L = max(L, place[to - 1]);
-                    if (from >= 2) L = max(L, place[from - 2] - 1);
-                    layer = L + 1;
+                    layer = exact_layer(place, from, to, n);
                     if (layer > grid_layers) { early = 1; break; }
-                    for (int64_t q = from - 1; q <= to - 2; ++q)
-                        for (int32_t g = place[q] + 1; g < layer; ++g) {
-                            double* p = grid + 2 * (q + (int64_t)(g - 1) * rows);
-                            p[0] = 1.0;
-                            p[1] = 0.0;
-                        }
+                    fill_skipped(grid, place, from, to, layer, rows);
                 }
                 const double mu = wilkinson_shift(dv[to - 2], dv[to - 1], ev[to - 2]);
-                single_shift<true>(dv, ev, from, to, mu, grid, thick, place, rows, layer, st->neg_zero);
+                if (layer > 0) sweep_warp<true>(dv, ev, from, to, mu, grid, thick, rows, layer, nz);
+                else sweep_warp<false>(dv, ev, from, to, mu, grid, thick, rows, layer, nz);
+                for (int64_t q = from - 1 + lane; q < to - 1; q += 32) {
+                    const int32_t t = thick[q] + 1;
+                    thick[q] = t;
+                    place[q] = layer > 0 ? layer : t;
+                }
+                __syncwarp();
                 did = true;
                 iter += 1;
                 rotations += to - from;
@@ -1039,34 +1050,37 @@ __device__ void chase_flush_lane(ChaseState* __restrict__ st, double* __restrict
         }
         if (to <= start) break;
     }
-    int32_t kmax = 0;
-    for (int64_t q = 0; q < n; ++q) kmax = max(kmax, place[q]);
-    if (status == CHASE_RUNNING) status = did ? CHASE_FLUSH : CHASE_CONVERGED;
-    st->status = status;
-    st->iter = iter;
-    st->last_block_ends_at = lbe;
-    st->rotations = rotations;
-    st->min_from = min_from;
-    st->max_to = max_to;
-    st->max_thickness = kmax;
-    st->total_rotations += rotations;
-    st->early_flushes += early;
+    const int32_t kmax = warp_range_max(place, 0, n - 1);
+    if (lane == 0) {
+        if (status == CHASE_RUNNING) status = did ? CHASE_FLUSH : CHASE_CONVERGED;
+        st->status = status;
+        st->iter = iter;
+        st->last_block_ends_at = lbe;
+        st->rotations = rotations;
+        st->min_from = min_from;
+        st->max_to = max_to;
+        st->max_thickness = kmax;
+        st->total_rotations += rotations;
+        st->early_flushes += early;
+    }
 }
 
-__global__ void __launch_bounds__(32)
+constexpr int kBatchWarps = 4;   // matrices per CTA, one on each SM sub-partition
+
+__global__ void __launch_bounds__(32 * kBatchWarps)
 chase_batched_kernel(const BatchMat* __restrict__ mats, const int32_t* __restrict__ order,
                      int32_t count, ChaseState* __restrict__ states, double* __restrict__ d,
                      double* __restrict__ e, double* __restrict__ grids,
                      int32_t* __restrict__ thick, int32_t* __restrict__ place)
 {
-    const int32_t k = blockIdx.x * 32 + threadIdx.x;
+    const int32_t k = blockIdx.x * kBatchWarps + (threadIdx.x >> 5);
     if (k >= count) return;
     const int32_t i = order[k];
     ChaseState* st = states + i;
     const int32_t s0 = st->status;
     if (s0 == CHASE_CONVERGED || s0 == CHASE_MAXITER) return;
     const BatchMat mt = mats[i];
-    chase_flush_lane(st, d + mt.doff, e + mt.eoff, grids + mt.goff, thick + mt.doff, place + mt.doff);
+    chase_flush_warp(st, d + mt.doff, e + mt.eoff, grids + mt.goff, thick + mt.doff, place + mt.doff);
 }
 
 // get_rotation(f, g) (src/simple_givens.jl:20-23) elementwise: form 0 as the chase computes it
@@ -1128,7 +1142,7 @@ cudaError_t launch_chase_batched(const BatchMat* mats, const int32_t* order, int
                                  int32_t* thick, int32_t* place, cudaStream_t stream)
 {
     if (count <= 0) return cudaSuccess;
-    chase_batched_kernel<<<(count + 31) / 32, 32, 0, stream>>>(mats, order, count, states, d, e,
+    chase_batched_kernel<<<(count + kBatchWarps - 1) / kBatchWarps, 32 * kBatchWarps, 0, stream>>>(mats, order, count, states, d, e,
                                                                grids, thick, place);
     return cudaGetLastError();
 }

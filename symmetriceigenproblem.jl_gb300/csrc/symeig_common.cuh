@@ -229,7 +229,7 @@ struct BatchMat {
     int32_t pad;
 };
 
-// One flush of every unfinished matrix of a batch, one lane per matrix, lanes in `order`.
+// One flush of every unfinished matrix of a batch, one warp per matrix, warps in `order`.
 cudaError_t launch_chase_batched(const BatchMat* mats, const int32_t* order, int32_t count,
                                  ChaseState* states, double* d, double* e, double* grids,
                                  int32_t* thick, int32_t* place, cudaStream_t stream);
