@@ -228,6 +228,57 @@ __device__ __forceinline__ void sweep_update(const SweepLanes& L, double c, doub
     gg = lane_get(p3, 4);
 }
 
+// What a sweep carries from step to step: the next rotation's (f, g) and x = f^2 + g^2, the
+// lanes' v2 and v4, and the last rotation.
+struct SweepRegs {
+    double f, g, x, v2, v4, c, s, r;
+};
+
+// H11, H21: dv[from], ev[from] (1-based) of the sweep's block.
+__device__ __forceinline__ SweepRegs sweep_begin(double H11, double H21, double mu, double nz)
+{
+    SweepRegs S;
+    S.f = __dsub_rn(H11, mu);
+    S.g = H21;
+    S.x = __dadd_rn(mulz(S.f, S.f, nz), mulz(H21, H21, nz));
+    S.v4 = H11;   // lane 2's v4 is B11, lane 5's v2 is B21
+    S.v2 = H21;
+    S.c = S.s = S.r = 0.0;
+    return S;
+}
+
+// This lane's result of the last step: lane 1 B11'', lane 2 r, lane 4 c, lane 5 s.
+__device__ __forceinline__ double sweep_result(const SweepLanes& L, const SweepRegs& S)
+{
+    return lane_sel(L.m1, S.v4, lane_sel(L.m2, S.r, lane_sel(L.m4, S.c, S.s)));
+}
+
+// One step with the entries B22 = dv[i+1], B23 = ev[i+1] (1-based i).  `emit` puts the last
+// step's result away, beside this step's rotation.
+template <typename Emit>
+__device__ __forceinline__ void sweep_step(const SweepLanes& L, SweepRegs& S, double B22, double B23, double nz,
+                                           Emit emit)
+{
+    double c, s, r;
+    IntRot K;
+    givens_int(S.f, S.g, S.x, c, s, r, K);
+    const double B11 = lane_get(S.v4, 2), B21 = lane_get(S.v2, 5);
+    emit(sweep_result(L, S));
+    const double a1 = lane_sel(L.m1, B22, lane_sel(L.m2, B11, lane_sel(L.m5, -0.0, lane_sel(L.m4, B23, B21))));
+    const double a2 = lane_sel(L.m0, B11, lane_sel(L.m3, B22, lane_sel(L.m5, B23, lane_sel(L.m4, 0.0, B21))));
+    double g, gg;
+    sweep_update(L, c, s, a1, a2, nz, S.v2, S.v4, g, gg);
+    if (__any_sync(0xffffffffu, !K.in_range || K.undecided != 0u)) {
+        const Rot3 o = givens_fix(S.f, S.g, K, nz);
+        c = o.c; s = o.s; r = o.r;
+        sweep_update(L, c, s, a1, a2, nz, S.v2, S.v4, g, gg);
+    }
+    S.f = lane_get(S.v4, 0);
+    S.x = __dadd_rn(mulz(S.f, S.f, nz), gg);
+    S.g = g;
+    S.c = c; S.s = s; S.r = r;
+}
+
 template <bool ONE_LAYER>
 __device__ void sweep_warp(double* __restrict__ dv, double* __restrict__ ev, int64_t from, int64_t to,
                            double mu, double* __restrict__ grid, const int32_t* __restrict__ thick,
@@ -236,81 +287,38 @@ __device__ void sweep_warp(double* __restrict__ dv, double* __restrict__ ev, int
     const int lane = threadIdx.x & 31, role = lane & 7;
     const SweepLanes L = sweep_lanes();
     const int steps = (int)(to - from);
-    const double H11 = dv[from - 1], H21 = ev[from - 1];
-    double f = __dsub_rn(H11, mu), g = H21;
-    double x = __dadd_rn(mulz(f, f, nz), mulz(g, g, nz));
+    SweepRegs S = sweep_begin(dv[from - 1], ev[from - 1], mu, nz);
     double B22n = dv[from], B23n = 2 <= steps ? ev[from] : 0.0;
-    double v4 = H11, v2 = H21;   // lane 2's v4 is B11, lane 5's v2 is B21
     // where this lane's result of the step before the current one goes
     double* out = role == 1 ? dv + from - 2 : role == 2 ? ev + from - 3
                                             : grid + 2 * ((from - 2) + (int64_t)(layer - 1) * rows) + (role == 5);
     const int out_step = role >= 4 ? 2 : 1;
     const bool stores = lane == 1 || lane == 2 || lane == 4 || lane == 5;
     const double *ld = dv + from + 1, *le = ev + from + 1;   // entries of step k + 1
-    double c_out = 0.0, s_out = 0.0, r_out = 0.0;
     int32_t t_out = 0, t_cur = 0, t_next = 0;   // thick of the stored, the current and the next rotation
     if (!ONE_LAYER) t_cur = thick[from - 1];
+    auto put = [&](double v, bool first, bool second) {
+        double* p = out;
+        if (!ONE_LAYER && role >= 4) p += (int64_t)(t_out + 1 - layer) * 2 * rows;
+        st_if(p, v, stores && !first && !(role == 2 && second));   // the first rotation has no r entry
+        out += out_step;
+    };
 #pragma unroll 1
     for (int k = 0; k < steps; ++k) {
         const double B22 = B22n, B23 = B23n;
-        double c, s, r;
-        IntRot K;
-        givens_int(f, g, x, c, s, r, K);
         B22n = k + 2 <= steps ? *ld : 0.0;
         B23n = k + 3 <= steps ? *le : 0.0;
         ++ld;
         ++le;
         if (!ONE_LAYER) t_next = k + 2 <= steps ? thick[from + k] : 0;
-        const double B11 = lane_get(v4, 2), B21 = lane_get(v2, 5);
-        {
-            const double v = lane_sel(L.m1, v4, lane_sel(L.m2, r_out, lane_sel(L.m4, c_out, s_out)));
-            double* p = out;
-            if (!ONE_LAYER && role >= 4) p += (int64_t)(t_out + 1 - layer) * 2 * rows;
-            st_if(p, v, stores && k > 0 && !(role == 2 && k == 1));
-            out += out_step;
-        }
-        const double a1 = lane_sel(L.m1, B22, lane_sel(L.m2, B11, lane_sel(L.m5, -0.0, lane_sel(L.m4, B23, B21))));
-        const double a2 = lane_sel(L.m0, B11, lane_sel(L.m3, B22, lane_sel(L.m5, B23, lane_sel(L.m4, 0.0, B21))));
-        double gn, ggn;
-        sweep_update(L, c, s, a1, a2, nz, v2, v4, gn, ggn);
-        if (__any_sync(0xffffffffu, !K.in_range || K.undecided != 0u)) {
-            const Rot3 o = givens_fix(f, g, K, nz);
-            c = o.c; s = o.s; r = o.r;
-            sweep_update(L, c, s, a1, a2, nz, v2, v4, gn, ggn);
-        }
-        f = lane_get(v4, 0);
-        x = __dadd_rn(mulz(f, f, nz), ggn);
-        g = gn;
-        c_out = c; s_out = s; r_out = r;
+        sweep_step(L, S, B22, B23, nz, [&](double v) { put(v, k == 0, k == 1); });
         t_out = t_cur;
         t_cur = t_next;
     }
-    {
-        const double v = lane_sel(L.m1, v4, lane_sel(L.m2, r_out, lane_sel(L.m4, c_out, s_out)));
-        double* p = out;
-        if (!ONE_LAYER && role >= 4) p += (int64_t)(t_out + 1 - layer) * 2 * rows;
-        st_if(p, v, stores && !(role == 2 && steps == 1));
-        st_if(dv + to - 1, v4, lane == 2);
-        st_if(ev + to - 2, f, lane == 0);
-    }
+    put(sweep_result(L, S), false, steps == 1);
+    st_if(dv + to - 1, S.v4, lane == 2);
+    st_if(ev + to - 2, S.f, lane == 0);
     __syncwarp();
-}
-
-// Two-warp mailbox and named barriers of the bulges' sweep (sweep_bulge_2w).
-enum : int { kBarCS = 1, kBarB = 2 };
-
-struct NrMail {
-    double c, s, r;           // warp 0 -> 1 (kBarCS); r with the sign convention applied
-    double b22pp, e_next;     // warp 1 -> 0 (kBarB): next B11, next B21
-};
-
-__device__ __forceinline__ void nb_sync(int id)
-{
-    asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory");
-}
-__device__ __forceinline__ void nb_arrive(int id)
-{
-    asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory");
 }
 
 constexpr int kScanUnroll = 8;  // chunks of 32 entries per round of the deflation scan
@@ -567,23 +575,27 @@ __device__ void batch_shifts_solve(const double* __restrict__ dv, int64_t to, in
     }
 }
 
-// The bulges of a batch.  Bulge j (CTA j) runs a sweep on two warps -- warp 0 the rotation and
-// the products that lead to the next one, warp 1 the rest of the update and the stores, values
-// traded through a two-slot mailbox and two alternating named barriers -- with shift shifts[j]
-// over the batch's block, a few steps behind bulge j-1, reading only what bulge j-1 has stored: step k of a sweep stores dv[k-1] and ev[k-2] (0-based; its last step also
-// dv[k] and ev[k-1]), so before its loads for step i+1 (dv[i+1], ev[i+1]) bulge j needs bulge
-// j-1 through step min(i+3, to-1).  The helper warp's store thread releases the bulge's
-// progress every (prog_mask + 1) steps and at its last step (st.release.gpu); the next bulge's
-// warps read it with ld.acquire.gpu only when the value they hold is too small, and read
-// dv/ev through L2 (ld.global.cg), never from a stale L1 line.  Bulge j waits only for bulge
+// The bulges of a batch.  Bulge j (CTA j) runs the one-warp sweep with shift shifts[j] over the
+// batch's block, a few steps behind bulge j-1, reading only what bulge j-1 has stored: step k of
+// a sweep stores dv[k-1] and ev[k-2] (0-based; its last step also dv[k] and ev[k-1]), so the
+// entries of step i (dv[i], ev[i]) need bulge j-1 through step min(i+2, to-1).
+// Three warps.  The sweep's warp (0) touches only shared memory: warp 1 fetches the entries of
+// the next steps as far as bulge j-1's progress allows, warp 2 stores the results and releases
+// the bulge's own progress (st.release.gpu, whose fence would hold the sweep for about 700
+// cycles).  They work in chunks of `every` steps, two buffers each way, handed over by named
+// barriers, each used by one producer (bar.arrive) and one consumer (bar.sync) that strictly
+// alternate: full[b] before a buffer is read, empty[b] before it is written again.
+// Warp 1 reads the progress word with ld.acquire.gpu only when the value it holds is too small,
+// and dv/ev through L2 (ld.global.cg), never from a stale L1 line.  Bulge j waits only for bulge
 // j-1 and the CTAs are co-resident (one cooperative launch), so the waits form one chain that
-// starts at bulge 0, which waits for none.  Every wait is bounded (about 2 s of SM clock): one
-// that gives up sets the device error word, and the warp carries on without waiting, so the
-// two warps' barrier protocol still completes; the call then reports the error.
-// The rotation is givens_nr_core (reference form out of its range) without the rounding
-// proof: the batch is not the reference's sweep sequence, so there are no bits to match.
+// starts at bulge 0, which waits for none.  Every wait on another bulge is bounded (about 2 s of
+// SM clock): one that gives up sets the device error word, and the warp carries on without
+// waiting, so the barriers still complete; the call then reports the error.
 // `hold` (the test hook of symeig_set_test_stall, bulge 0 only) withholds every release, so
 // the next bulge's wait runs out.
+// With the two-warp Newton sweep that waited, loaded and stored by itself a step cost 1.15 us:
+// the whole n = 2000 multishift solve took 175 ms and takes 137 ms, n = 3001 with FP32 Q and a
+// random diagonal 514 and 348 ms.
 
 __device__ __forceinline__ long long ld_acquire_gpu(const long long* p)
 {
@@ -626,102 +638,126 @@ struct PipeWait {
     }
 };
 
-__device__ void sweep_bulge_2w(double* __restrict__ dv, double* __restrict__ ev, int64_t from,
-                               int64_t to, double mu, double* __restrict__ grid,
-                               const int32_t* __restrict__ thick, int64_t rows, int32_t layer,
-                               int32_t jofs, double nz, NrMail* mail, PipeWait pw,
-                               long long* __restrict__ my_prog, int64_t prog_mask, bool hold)
+constexpr int kMaxRelease = 64;   // largest chunk (symeig_set_multishift's release_every)
+enum : int { kBarInFull = 1, kBarInEmpty = 3, kBarOutFull = 5, kBarOutEmpty = 7 };   // two each
+
+__device__ __forceinline__ void nb_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+__device__ __forceinline__ void nb_arrive(int id) { asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory"); }
+
+struct BulgeRing {
+    double2 in[2][kMaxRelease];       // (dv[i], ev[i]) of the chunk's steps
+    double out[2][kMaxRelease][4];    // (B11'', r, c, s)
+    double first[2];                  // dv[from-1], ev[from-1]
+    double last[2];                   // the last step's B22'', B12''
+};
+
+__device__ __forceinline__ void bulge_sweep(BulgeRing& R, int steps, int every, double mu, double nz)
 {
-    const int warp = threadIdx.x >> 5;
-    const bool lead = (threadIdx.x & 31) == 0;
-    pw.until(min(from + 2, to - 1));
-    const double H11 = __ldcg(dv + from - 1), H21 = __ldcg(ev + from - 1);
-    if (warp == 0) {
-        double f = __dsub_rn(H11, mu), g = H21, gg = mulz(H21, H21, nz);
-        double B11 = H11, B21 = H21;
-        double B22n = __ldcg(dv + from);
-        double B23n = (from + 2 <= to) ? __ldcg(ev + from) : 0.0;
-        for (int64_t i = from; i <= to - 1; ++i) {
-            const double B22 = B22n, B23 = B23n;
-            pw.until(min(i + 3, to - 1));
-            if (i + 1 <= to - 1) B22n = __ldcg(dv + i + 1);
-            if (i + 3 <= to) B23n = __ldcg(ev + i + 1);
-            const NrRot o = givens_nr_core(f, g, gg, nz);
-            double c = o.c, s = o.s, r = o.r;
-            if (!nr_in_range(f, g)) givens_fast(f, g, c, s, r, nz);
-            if (i > from) {
-                nb_sync(kBarB);
-                const NrMail& pv = mail[(i - 1) & 1];
-                B11 = pv.b22pp;
-                B21 = pv.e_next;
+    const int lane = threadIdx.x & 31, role = lane & 7;
+    const SweepLanes L = sweep_lanes();
+    const bool stores = lane == 1 || lane == 2 || lane == 4 || lane == 5;
+    const int item = role == 1 ? 0 : role == 2 ? 1 : role == 4 ? 2 : 3;
+    const uint32_t out0 = (uint32_t)__cvta_generic_to_shared(&R.out[0][0][item]);
+    nb_sync(kBarInFull);
+    SweepRegs S = sweep_begin(R.first[0], R.first[1], mu, nz);
+    uint32_t at = out0;   // where the last step's result goes
+    int b = 0;
+    for (int k0 = 0; k0 < steps; k0 += every, b ^= 1) {
+        if (k0 > 0) nb_sync(kBarInFull + b);
+        if (k0 >= 2 * every) nb_sync(kBarOutEmpty + b);
+        const int len = min(every, steps - k0);
+        const double2* in = R.in[b];
+#pragma unroll 1
+        for (int q = 0; q < len; ++q) {
+            const double2 B = in[q];
+            sweep_step(L, S, B.x, B.y, nz, [&](double v) {
+                asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q st.shared.f64 [%0], %1;\n\t}"
+                             ::"r"(at), "d"(v), "r"((unsigned)(stores && k0 + q > 0)) : "memory");
+            });
+            if (q == 0 && k0 > 0) {
+                __syncwarp();
+                nb_arrive(kBarOutFull + (b ^ 1));
             }
-            NrMail& mb = mail[i & 1];
-            mb.c = c; mb.s = s; mb.r = r;
-            nb_arrive(kBarCS);
-            const double B11p = __fma_rn(c, B11, mulz(s, B21, nz));
-            const double B12p = __fma_rn(c, B21, mulz(s, B22, nz));
-            f = __fma_rn(B12p, c, -mulz(B11p, s, nz));
-            g = (i + 2 <= to) ? mulz(s, B23, nz) : 0.0;
-            gg = mulz(g, g, nz);
+            at = out0 + (uint32_t)((b * kMaxRelease + q) * 4 * sizeof(double));
         }
-    } else {
-        double B11 = H11, B21 = H21;
-        double B22n = __ldcg(dv + from);
-        double B23n = (from + 2 <= to) ? __ldcg(ev + from) : 0.0;
-        int32_t thn = layer <= 0 ? thick[from - 1] : 0;
-        for (int64_t i = from; i <= to - 1; ++i) {
-            const double B22 = B22n, B23 = B23n;
-            const int32_t th = thn;
-            pw.until(min(i + 3, to - 1));
-            if (i + 1 <= to - 1) B22n = __ldcg(dv + i + 1);
-            if (i + 3 <= to) B23n = __ldcg(ev + i + 1);
-            if (layer <= 0 && i + 1 <= to - 1) thn = thick[i];
-            nb_sync(kBarCS);
-            const NrMail& mb = mail[i & 1];
-            const double c = mb.c, s = mb.s, r = mb.r;
-            const double e_next = (i + 2 <= to) ? mulz(c, B23, nz) : 0.0;
-            const double sB21 = mulz(s, B21, nz);
-            const double B21p = __fma_rn(c, B21, -mulz(s, B11, nz));
-            const double B22p = __fma_rn(c, B22, -sB21);
-            const double B22pp = __fma_rn(B22p, c, -mulz(B21p, s, nz));
-            if (i < to - 1) {
-                NrMail& mo = mail[i & 1];
-                mo.b22pp = B22pp;
-                mo.e_next = e_next;
-                nb_arrive(kBarB);
-            }
-            const double B11p = __fma_rn(c, B11, sB21);
-            const double B12p = __fma_rn(c, B21, mulz(s, B22, nz));
-            const double B11pp = __fma_rn(B11p, c, mulz(B12p, s, nz));
-            if (lead) {
-                dv[i - 1] = B11pp;
-                if (i > from) ev[i - 2] = r;
-                const int32_t L = layer > 0 ? layer : th + 1 + jofs;
-                *reinterpret_cast<double2*>(grid + 2 * ((i - 1) + (int64_t)(L - 1) * rows)) =
-                    make_double2(c, s);
-                if (i == to - 1) {
-                    dv[i] = B22pp;
-                    ev[i - 1] = __fma_rn(B12p, c, -mulz(B11p, s, nz));
-                }
-                if (!hold && (i == to - 1 || ((i - from) & prog_mask) == prog_mask)) st_release_gpu(my_prog, i);
-            }
-            B11 = B22pp;
-            B21 = e_next;
+        if (k0 + 2 * every < steps) nb_arrive(kBarInEmpty + b);   // only a buffer that is filled again
+    }
+    if (stores) {
+        const double v = sweep_result(L, S);
+        asm volatile("st.shared.f64 [%0], %1;" ::"r"(at), "d"(v) : "memory");
+    }
+    if (lane == 2) R.last[0] = S.v4;
+    if (lane == 0) R.last[1] = S.f;
+    __syncwarp();
+    nb_arrive(kBarOutFull + (b ^ 1));
+}
+
+__device__ __forceinline__ void bulge_fetch(BulgeRing& R, const double* __restrict__ dv, const double* __restrict__ ev,
+                                            int64_t from, int64_t to, int steps, int every, PipeWait pw)
+{
+    const int lane = threadIdx.x & 31;
+    int b = 0;
+    for (int k0 = 0; k0 < steps; k0 += every, b ^= 1) {
+        const int len = min(every, steps - k0);
+        if (k0 >= 2 * every) nb_sync(kBarInEmpty + b);
+        // the chunk's last step is i = from + k0 + len - 1
+        pw.until(min(from + k0 + len + 1, to - 1));
+        if (k0 == 0 && lane == 0) {
+            R.first[0] = __ldcg(dv + from - 1);
+            R.first[1] = __ldcg(ev + from - 1);
         }
+        for (int q = lane; q < len; q += 32) {
+            const int64_t i = from + k0 + q;
+            R.in[b][q] = make_double2(__ldcg(dv + i), i + 2 <= to ? __ldcg(ev + i) : 0.0);
+        }
+        __syncwarp();
+        nb_arrive(kBarInFull + b);
     }
 }
 
-// One CTA of two warps per bulge; dynamic shared memory (kBatchSmem) keeps one CTA per SM, so
+__device__ __forceinline__ void bulge_store(BulgeRing& R, double* __restrict__ dv, double* __restrict__ ev, int64_t from,
+                                            int64_t to, double* __restrict__ grid, const int32_t* __restrict__ thick,
+                                            int64_t rows, int32_t layer, int32_t jofs, int steps, int every,
+                                            long long* __restrict__ my_prog, bool hold)
+{
+    const int lane = threadIdx.x & 31;
+    int b = 0;
+    for (int k0 = 0; k0 < steps; k0 += every, b ^= 1) {
+        const int len = min(every, steps - k0);
+        nb_sync(kBarOutFull + b);
+        for (int t = lane; t < 4 * len; t += 32) {
+            const int q = t >> 2, item = t & 3;
+            const int64_t i = from + k0 + q;   // 1-based step
+            const double v = R.out[b][q][item];
+            if (item == 0) {
+                dv[i - 1] = v;
+            } else if (item == 1) {
+                if (k0 + q > 0) ev[i - 2] = v;
+            } else {
+                const int32_t Lr = layer > 0 ? layer : thick[i - 1] + 1 + jofs;
+                grid[2 * ((i - 1) + (int64_t)(Lr - 1) * rows) + (item - 2)] = v;
+            }
+        }
+        if (k0 + every >= steps && lane == 0) {
+            dv[to - 1] = R.last[0];
+            ev[to - 2] = R.last[1];
+        }
+        __syncwarp();
+        if (k0 + 2 * every < steps) nb_arrive(kBarOutEmpty + b);
+        if (!hold && lane == 0) st_release_gpu(my_prog, from + k0 + len - 1);
+    }
+}
+
+// One CTA of three warps per bulge; dynamic shared memory (kBatchSmem) keeps one CTA per SM, so
 // no two bulges share an SM's FP64 unit.
 constexpr int kBatchSmem = 120 * 1024;
 
-__global__ void __launch_bounds__(64, 1)
-bulge_batch_kernel(const ChaseState* __restrict__ st, double* __restrict__ dv,
-                   double* __restrict__ ev, double* __restrict__ grid,
+__global__ void __launch_bounds__(96, 1)
+bulge_batch_kernel(const ChaseState* __restrict__ st, double* dv, double* ev, double* __restrict__ grid,
                    const int32_t* __restrict__ thick, BulgeScratch* __restrict__ bs,
                    int* __restrict__ err)
 {
-    __shared__ NrMail mail[2];
+    __shared__ BulgeRing ring;
     const int j = blockIdx.x;
     if (st->status != CHASE_BATCH) return;  // a launch queued ahead after the batches ended
     const int32_t nb = st->b_bulges;
@@ -729,10 +765,16 @@ bulge_batch_kernel(const ChaseState* __restrict__ st, double* __restrict__ dv,
     const int64_t n = st->n, from = st->b_from, to = st->b_to;
     const int64_t rows = n > 1 ? n - 1 : 1;
     const int32_t L0 = st->b_layer0;
-    PipeWait pw{j > 0 ? &bs->prog[j - 1] : nullptr, err, -1};
-    sweep_bulge_2w(dv, ev, from, to, bs->shifts[j], grid, thick, rows, L0 > 0 ? L0 + j : 0, j,
-                   st->neg_zero, mail, pw, &bs->prog[j], (int64_t)st->ms_prog_mask,
-                   st->test_stall != 0 && j == 0);
+    const int steps = (int)(to - from), every = st->ms_prog_mask + 1;
+    const int warp = threadIdx.x >> 5;
+    if (warp == 0) {
+        bulge_sweep(ring, steps, every, bs->shifts[j], st->neg_zero);
+    } else if (warp == 1) {
+        bulge_fetch(ring, dv, ev, from, to, steps, every, PipeWait{j > 0 ? &bs->prog[j - 1] : nullptr, err, -1});
+    } else {
+        bulge_store(ring, dv, ev, from, to, grid, thick, rows, L0 > 0 ? L0 + j : 0, j, steps, every, &bs->prog[j],
+                    st->test_stall != 0 && j == 0);
+    }
 }
 
 // One flush: the reference's inner loop from `to = last_block_ends_at` until the matrix is
@@ -1133,7 +1175,7 @@ cudaError_t launch_bulge_batch(const ChaseState* state, double* d, double* e, do
                                           kBatchSmem);
     if (ce != cudaSuccess) return ce;
     void* args[] = {(void*)&state, (void*)&d, (void*)&e, (void*)&grid, (void*)&thick, (void*)&bs, (void*)&err};
-    return cudaLaunchCooperativeKernel((const void*)bulge_batch_kernel, dim3((unsigned)bulges), dim3(64), args,
+    return cudaLaunchCooperativeKernel((const void*)bulge_batch_kernel, dim3((unsigned)bulges), dim3(96), args,
                                        (size_t)kBatchSmem, stream);
 }
 

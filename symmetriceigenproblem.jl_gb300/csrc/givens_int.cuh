@@ -2,8 +2,8 @@
 // root and the two quotients on the integer pipes.
 //
 // On GB300 a dependent FP64 instruction costs 64 cycles, a 32-bit integer one 4 to 5 and a
-// 32 x 32 -> 64-bit multiply-add about 5.  The FMA-only Newton form (givens.cuh) is a chain of
-// ten FP64 instructions after x = f^2 + g^2 (719 cycles measured); here one table seed (18
+// 32 x 32 -> 64-bit multiply-add about 5.  Newton steps in FP64 are a chain of ten instructions
+// after x = f^2 + g^2 (719 cycles measured); here one table seed (18
 // cycles) and fixed-point arithmetic on 64-bit integers give r = RN(sqrt x), c = RN(f/r) and
 // s = RN(g/r) in 307 cycles, each from an interval that holds the exact value.  Where an
 // interval straddles a rounding boundary (3.8 % of the rotations of a chase) givens_exact
@@ -51,8 +51,9 @@ __device__ __forceinline__ uint64_t mulhi64(uint64_t a, uint64_t b)
     return mulw(hi32(a), hi32(b)) + hi32(p1) + hi32(p2);
 }
 
-// nr_in_range on the high words: the exponent fields alone decide it (zero, infinity and NaN
-// are out of range).
+// The fixed-point form's range, from the high words: max(|f|, |g|) in [2^-450, 2^450) and
+// min >= 2^-400 max by the exponent fields (so f, g are nonzero and finite, givensAlgorithm takes
+// its plain branch, x and r are normal and |c|, |s| >= 2^-401).
 __device__ __forceinline__ bool in_range_hi(uint32_t fh, uint32_t gh)
 {
     const uint32_t ef = (fh >> 20) & 0x7FFu, eg = (gh >> 20) & 0x7FFu;

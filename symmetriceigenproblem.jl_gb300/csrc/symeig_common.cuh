@@ -212,7 +212,7 @@ cudaError_t launch_chase(ChaseState* state, double* d, double* e, double* grid, 
                          int32_t* place, double* bak, BulgeScratch* bs, int32_t resume_only,
                          cudaStream_t stream);
 // The pending multishift batch of `state`, if its status is CHASE_BATCH (else the launch
-// returns at once): `bulges` (>= the batch's) CTAs of two warps in one cooperative launch,
+// returns at once): `bulges` (>= the batch's) CTAs of three warps in one cooperative launch,
 // one bulge each.  A bounded wait that gives up sets *err.
 cudaError_t launch_bulge_batch(const ChaseState* state, double* d, double* e, double* grid,
                                const int32_t* thick, BulgeScratch* bs, int* err, int32_t bulges,
