@@ -18,7 +18,7 @@ ROOT = PKG.parent
 CSRC = PKG / "csrc"
 OUT = PKG / "_build"
 LIB = OUT / "libsymeig.so"
-SOURCES = ["apply.cu", "chase.cu", "api.cu", "peak.cu", "noalloc.cu", "batched.cu", "adjoint.cu", "sytrd.cu"]
+SOURCES = ["apply.cu", "apply_f64.cu", "apply_f32.cu", "chase.cu", "api.cu", "peak.cu", "noalloc.cu", "batched.cu", "adjoint.cu", "sytrd.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
               "-Xcompiler", "-Wall", "-Xcompiler", "-Wextra", "-Xcompiler", "-Wno-unused-parameter",
@@ -84,7 +84,7 @@ def build(force: bool = False, verbose: bool = False, extra_flags: list[str] | N
 # batched apply) compiled with -DSYMEIG_DEVICE_CHECKS and linked with the default build's other
 # objects into _build/libsymeig_checked.so.  A debugging aid: every global access of a wave
 # tile is checked against its pass's extent and a failed check is reported as SYMEIG_ERR_DEVICE.
-CHECKED_SOURCES = ["apply.cu", "batched.cu"]
+CHECKED_SOURCES = ["apply.cu", "apply_f64.cu", "apply_f32.cu", "batched.cu"]
 CHECKED_LIB = OUT / "libsymeig_checked.so"
 
 

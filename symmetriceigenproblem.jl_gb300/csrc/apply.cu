@@ -21,9 +21,7 @@ using wave::kThreads;
 // Tile shapes.  Each covers 64 layers per pass, except FP64 shape 3 (128).
 //   shape 0 = 8 lane groups of 8 layers: 4 rows per warp -- at m = 16384, 4096 warps, all
 //             resident at <= 7 CTAs of 4 warps per SM (register budget 73), 6 or 7 warps per
-//             SM sub-partition.  The FP64 shape below 9728 rows: the FP64 unit (2 FMA per SM
-//             per clock on GB300) is the limit and this shape balances it best; from there
-//             its CTAs of 27 warps (shape 2) even out the SMs' loads.
+//             SM sub-partition.
 //   shape 1 = 4 lane groups of 16 layers: 8 rows per warp, twice the rotations per wave for
 //             the same per-wave overhead (shuffle, Q load/store, address arithmetic).  For
 //             FP32 the overhead per rotation matters more than the coarser balance.
@@ -32,7 +30,8 @@ using wave::kThreads;
 //             128-bit broadcast read of 4 or 8 distinct addresses) carries half the load per
 //             rotation-row, and each thread has two independent rotation chains.  Shape 2
 //             runs as shape 4 (below) from 15000 rows on.
-// By default (kAutoShape) the rows of the launch choose the shape (resolve_shape).
+// They run when tuned to, for forms 1 and 2 of the FP64 apply and for the fixed-scratch apply; the
+// default (kAutoShape) runs the fused-wave tile instead (use_fused).
 template <typename T, int S> struct Cfg;
 // MINB: CTAs per SM the launch bounds ask for; MINB_INT the same for the FP64 kernels whose
 // products run on the integer pipes (int_mul.cuh: about 95 registers with one row per thread).
@@ -71,21 +70,16 @@ constexpr int64_t kWideRows = 15000;
 // (measured, 64 layers on m x m: 556 against 642 GFLOP/s at m = 2000, 916 against 710 at
 // m = 4096), and the products stay on the FP64 pipe; both give the same bits.
 constexpr int64_t kIntMulRows = 3072;
-// The tile shape by precision ([0] FP64, [1] FP32): a shape index, or kAutoShape (the default)
-// for the shape chosen by the rows of the launch.  Measured at n = 4096, k = 64 for m = 1024 ..
-// 16384 (TFLOP/s):
-//   FP32  m:      2048   4096   6144   8192  12288  15000  16384
-//         shape 0  8.60  15.10  18.77  19.64  19.82  21.44  23.25
-//         shape 1  6.92  13.75  16.30  21.55  24.30  22.01  23.94
-//         shape 4  3.32   6.62   9.95  13.26  19.86  24.25  26.31   (shape 2: within 8 % of 4)
-//   FP64  shape 0  0.67   0.81   0.90   0.88   0.84   1.39*  1.51*  (* as shape 2)
-//         shape 2  0.10   0.38   0.57   0.76   1.14   1.39   1.51
+// The tile shape by precision ([0] FP64, [1] FP32): a shape index, or kAutoShape (the default):
+// the fused-wave tile (use_fused), and for FP64 calls that do not take it a shape chosen by the
+// rows of the launch.  Measured at n = 4096, k = 64 for m = 1024 .. 16384 (TFLOP/s):
+//   m:            2048   4096   6144   8192  12288  15000  16384
+//   FP64 shape 0  0.67   0.81   0.90   0.88   0.84   1.39*  1.51*  (* as shape 2)
+//        shape 2  0.10   0.38   0.57   0.76   1.14   1.39   1.51
 // The 27-warp FP64 shape runs one CTA of 108 rows per SM, so it pays once m gives it about 90
-// of the 152 SMs; FP32 shape 0 wins while its 16-row CTAs are needed to fill the SMs, shape 1
-// in between, and the 14-warp shape 4 from about 14000 rows.
+// of the 152 SMs.
 constexpr int kAutoShape = -1;
 constexpr int64_t kAutoWideRows64 = 9728;       // FP64: shape 0 below, shape 2 from here
-constexpr int64_t kAutoRows32[2] = {7168, 14336};  // FP32: shape 0 below [0], 1 below [1], 4 from [1]
 int g_shape[2] = {kAutoShape, kAutoShape};
 
 // FP64: passes of more than 64 layers in the canonical form run as one 128-layer pass of
@@ -109,9 +103,16 @@ template <typename T> int resolve_shape(int64_t m, int64_t layers = 64, int form
         if (s == 3) return deep_ok ? 3 : 0;
         return (s == 0 && m >= kWideRows) ? 2 : s;
     } else {
-        if (s == kAutoShape) return m < kAutoRows32[0] ? 0 : (m < kAutoRows32[1] ? 1 : 4);
+        if (s == kAutoShape) return 0;   // the fused-wave tile takes every FP32 call
         return (s == 2 && m >= kWideRows) ? 4 : s;
     }
+}
+
+// The auto choice runs the fused-wave tile (apply_fused.cuh) for FP32 and for canonical FP64
+// rotations; a tuned shape, forms 1 and 2 and the fixed-scratch apply run the shapes above.
+template <typename T> bool use_fused(int form, int fixed_table = 0)
+{
+    return !fixed_table && g_shape[sizeof(T) == 8 ? 0 : 1] == kAutoShape && (sizeof(T) == 4 || form == 0);
 }
 
 template <typename Tsrc, typename T, int S>
@@ -418,10 +419,11 @@ cudaError_t launch_mul_rn(int64_t count, const double* a, const double* b, doubl
     return cudaGetLastError();
 }
 
-// Layers per pass of an apply of `layers` layers to m rows in `form`: 128 where the 128-layer
-// FP64 shape takes it, else 64.
+// Layers per pass of an apply of `layers` layers to m rows in `form`: the fused tile's, or 128
+// where the 128-layer FP64 shape takes it, else 64.
 template <typename T> int64_t apply_layers_per_pass(int64_t m, int64_t layers, int form)
 {
+    if (use_fused<T>(form)) return fused_layers_per_pass<T>(m, layers);
     if constexpr (sizeof(T) == 8)
         if (resolve_shape<T>(m, layers, form) == 3) return 128;
     return 64;
@@ -447,7 +449,7 @@ template <typename T> size_t apply_table_bytes(int64_t n_loc, int64_t layers)
         const int64_t passes = layers > 64 ? (layers + 63) / 64 : 1;
         b += (size_t)passes * scaled_slot_bytes(n_loc);
     }
-    return b;
+    return std::max(b, fused_table_bytes<T>(n_loc, layers));
 }
 
 cudaError_t launch_scaled_recurrences(const double* grid, int64_t grid_rows, const int32_t* place,
@@ -642,6 +644,8 @@ cudaError_t apply_pass(T* Q, int64_t ldq, int64_t m, const Tsrc* grid, int64_t g
                        const int32_t* place, const ApplyPass& pass, void* table, int* err,
                        cudaStream_t stream, cudaEvent_t ev_begin, cudaEvent_t ev_end, int what)
 {
+    if (use_fused<T>(pass.form, pass.fixed_table))
+        return fused_pass<Tsrc, T>(Q, ldq, m, grid, grid_rows, place, pass, table, err, stream, ev_begin, ev_end, what);
     const int s = resolve_shape<T>(m, pass.layers, pass.form);
     if constexpr (sizeof(T) == 8) {
         if (s == 2)
@@ -675,8 +679,9 @@ cudaError_t apply_host_segmented(T* dQ, int64_t m, const T* d_cs, const ApplyPas
 {
     if (pass.n_loc < 2 || pass.layers <= 0 || m <= 0) return cudaSuccess;
     if (pass.layers > 64 || pass.c0 != 0 || pass.L0 != 0) return cudaErrorInvalidValue;
-    // segmented launches exist for FP64 shapes 0 and 2 and FP32 shapes 0, 1, 2 and 4 (every
-    // shape the auto choice takes); other tunings take the unpipelined path
+    if (use_fused<T>(pass.form)) return fused_host_segmented<T>(dQ, m, d_cs, pass, table, err, stream, io);
+    // segmented launches exist for FP64 shapes 0 and 2 and FP32 shapes 0, 1, 2 and 4; other tunings
+    // take the unpipelined path
     const int s = resolve_shape<T>(m);
     if constexpr (sizeof(T) == 8) {
         if (s == 2) return host_segmented_shape<T, 2>(dQ, m, d_cs, pass, table, err, stream, io);
@@ -716,7 +721,7 @@ template <typename T> size_t apply_segment_state_bytes(int64_t m)
         b = std::max(b, state_bytes<T, 3>(m));
         b = std::max(b, state_bytes<T, 4>(m));
     }
-    return b;
+    return std::max(b, fused_state_bytes<T>(m));
 }
 template size_t apply_segment_state_bytes<double>(int64_t);
 template size_t apply_segment_state_bytes<float>(int64_t);

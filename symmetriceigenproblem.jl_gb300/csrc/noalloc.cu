@@ -107,6 +107,7 @@ extern "C" int symeig_apply_givens_f64_noalloc(double* A, int64_t lda, int64_t m
     cudaStream_t s = (cudaStream_t)stream;
     for (int64_t L0 = 0; L0 < k; L0 += per) {
         ApplyPass pass{0, n, L0, k - L0 < per ? k - L0 : per};
+        pass.fixed_table = 1;
         if (apply_pass<double, double>(A, lda, m, cs, n - 1, nullptr, pass, table, err, s) != cudaSuccess)
             return SYMEIG_ERR_CUDA;
     }

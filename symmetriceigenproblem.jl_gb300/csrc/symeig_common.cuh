@@ -132,6 +132,7 @@ struct ApplyPass {
     int32_t stall = 0; // test hook: > 0 stops the table copies from that chunk on (see wave_tile)
     int32_t rec = 0;   // form 1: 1 if launch_scaled_recurrences already filled scratch slot `slot`
     int32_t slot = 0;  // form 1: the pass's scratch slot (its index within the flush)
+    int32_t fixed_table = 0;  // 1: the table must fit apply_canonical_table_bytes (64-layer shapes)
 };
 
 // The scaled form's column-scale recurrences of all passes of [L0, L0 + layers) in one launch
@@ -183,6 +184,18 @@ cudaError_t apply_host_segmented(T* dQ, int64_t m, const T* d_cs, const ApplyPas
                                  cudaStream_t stream, const HostStream& io);
 template <typename T> size_t apply_segment_state_bytes(int64_t m);
 template <typename T> bool apply_host_segmented_supported(int64_t m);
+
+// The fused-wave tile (apply_fused.cuh), the default of FP32 and of canonical FP64 rotations.
+template <typename T> int64_t fused_layers_per_pass(int64_t m, int64_t layers);
+template <typename T> size_t fused_table_bytes(int64_t n_loc, int64_t layers);
+template <typename T> size_t fused_state_bytes(int64_t m);
+template <typename Tsrc, typename T>
+cudaError_t fused_pass(T* Q, int64_t ldq, int64_t m, const Tsrc* grid, int64_t grid_rows, const int32_t* place,
+                       const ApplyPass& pass, void* table, int* err, cudaStream_t stream, cudaEvent_t ev_begin,
+                       cudaEvent_t ev_end, int what);
+template <typename T>
+cudaError_t fused_host_segmented(T* dQ, int64_t m, const T* d_cs, const ApplyPass& pass, void* table, int* err,
+                                 cudaStream_t stream, const HostStream& io);
 
 // Tile shape of the single-matrix wave kernel per precision (see apply.cu).
 void apply_set_shape(int fp64, int shape);
