@@ -37,7 +37,11 @@ using wave::st_pred;
 
 constexpr int kSms = 152;   // GB300
 
-// PD: iterations group 0 reads ahead.  NI: iterations per chunk of the table.
+// PD: iterations group 0 reads ahead.  NI: iterations per chunk of the table, as many as two
+// chunks of 23 KB hold: two CTA barriers per chunk keep the warps together (16384 x 8192, 64
+// layers: 31.2 ms with 9 KB chunks, 30.8 with 22 KB; without barriers, each warp waiting by itself
+// and the last one refilling a slot, 31.3 and 31.0 ms, the warps then share no instruction
+// fetches).
 template <typename T, int KB_, int G_, int F_>
 struct Shape {
     using P2 = typename Pair<T>::type;
@@ -46,7 +50,7 @@ struct Shape {
     static constexpr int LAYERS = KB * G;
     static constexpr int GSTRIDE = KB * F * (int)sizeof(P2) + 16;   // padded: the groups' pairs lie in other banks
     static constexpr int ITER = G * GSTRIDE;
-    static constexpr int NI = SHIFT ? (ITER >= 6144 ? 2 : ITER >= 2048 ? 4 : 8) : D * (D * ITER <= 8192 ? 2 : 1);
+    static constexpr int NI = SHIFT ? (23552 / ITER < 16 ? 23552 / ITER : 16) : D * (D * ITER <= 8192 ? 2 : 1);
     static constexpr int PD = SHIFT ? 1 : D;
     static constexpr int CHUNK = NI * ITER;
     // warps per CTA that fit an SM's registers: 72 per thread for FP64 (KB <= 8), FP32 up to 122
