@@ -400,9 +400,7 @@ __device__ __forceinline__ void fill_skipped(double* grid, const int32_t* place,
 // exponent of p_i leaves [-600, 600]: over 128 rows of a window whose diagonal lies close to
 // the shift, the unscaled p_i underflows (about 1e-362 in case A), which made every Newton
 // step non-finite and left the shifts at FP32 accuracy.  Warp 0 of the controller sets up the
-// window (batch_shifts_setup), then every thread of the CTA solves for its shifts
-// (batch_shifts_solve); sd, se2, sea (FP32) and dd, ee2 (FP64) are
-// kShiftWindow * kMaxBulges-entry shared arrays.
+// window (batch_shifts_setup) and each bulge's CTA solves for its own shift (bulge_shift).
 constexpr int kShiftWindow = 2;
 constexpr int kWinMax = kShiftWindow * kMaxBulges;
 
@@ -421,17 +419,17 @@ __device__ __forceinline__ int window_count32(const float* sd, const float* se2,
     return cnt;
 }
 
-// p(x), p'(x) and the number of eigenvalues below x of the scaled window (dd, ee2), in FP64.
-__device__ __forceinline__ void char_poly(const double* __restrict__ dd, const double* __restrict__ ee2, int w,
-                                          double x, double& p, double& dp, int& below)
+// p(x), p'(x) and the number of eigenvalues below x of the scaled window, in FP64, step by step:
+// dd the diagonal, nbb[i] = -e_{i-1}^2.  The windows that meet an exact zero of a leading minor.
+__device__ __noinline__ void char_poly(const double* dd, const double* nbb, int w, double x, double& p, double& dp,
+                                       int& below)
 {
     double p0 = 1.0, p1 = dd[0] - x, q0 = 0.0, q1 = -1.0;
     int cnt = p1 < 0.0;
     for (int i = 1; i < w; ++i) {
-        const double aa = dd[i] - x, bb = ee2[i - 1];
-        const double t = -bb * p0, u = -bb * q0 - p1;
-        const double p2 = __fma_rn(aa, p1, t);
-        const double q2 = __fma_rn(aa, q1, u);
+        const double aa = dd[i] - x, nb = nbb[i];
+        const double p2 = __fma_rn(aa, p1, __dmul_rn(nb, p0));
+        const double q2 = __fma_rn(aa, q1, __fma_rn(nb, q0, -p1));
         // a sign change of the leading minors is an eigenvalue below x; an exact zero takes
         // the sign opposite to its predecessor's (the pivot convention of the FP32 counts)
         cnt += (p2 == 0.0) ? 1 : ((p2 < 0.0) != (p1 < 0.0));
@@ -454,17 +452,10 @@ __device__ __forceinline__ void char_poly(const double* __restrict__ dd, const d
     below = cnt;
 }
 
-// What batch_shifts_setup leaves for batch_shifts_solve (shared memory).
-struct ShiftWindow {
-    int32_t w, k0, ex, trivial;
-    float lo, hi;
-};
-
-// Warp 0: load and scale the window into the shared arrays, its Gershgorin interval, and the
-// rank k0 of the first shift.
+// Warp 0 of the controller: the scaled window into bs, its Gershgorin interval, and the rank of the
+// first shift.  sd, se2, sea: kWinMax-entry shared arrays.
 __device__ void batch_shifts_setup(const double* __restrict__ dv, const double* __restrict__ ev, int64_t from,
-                                   int64_t to, int nb, ShiftWindow& sw, float* sd, float* se2, float* sea,
-                                   double* dd, double* ee2)
+                                   int64_t to, int nb, BulgeScratch* __restrict__ bs, float* sd, float* se2, float* sea)
 {
     const int lane = threadIdx.x & 31;
     constexpr int H = kWinMax / 32;
@@ -484,10 +475,8 @@ __device__ void batch_shifts_setup(const double* __restrict__ dv, const double* 
     for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     if (!(mx > 0.0) || !isfinite(mx)) {
         // a zero block is already diagonal; a non-finite one is left to the sweep
-        if (lane == 0) {
-            sw.w = w;
-            sw.trivial = 1;
-        }
+        for (int j = lane; j < nb; j += 32) bs->shifts[j] = dv[to - nb + j];
+        if (lane == 0) bs->win_trivial = 1;
         __syncwarp();
         return;
     }
@@ -501,8 +490,10 @@ __device__ void batch_shifts_setup(const double* __restrict__ dv, const double* 
         sd[q] = (float)dsc;
         se2[q] = ef * ef;
         sea[q] = fabsf(ef);
-        dd[q] = dsc;
-        ee2[q] = esc * esc;
+        if (q < w) {
+            bs->win_d[q] = dsc;
+            bs->win_e[q] = esc;
+        }
     }
     __syncwarp();
     // Gershgorin interval of the window
@@ -524,55 +515,145 @@ __device__ void batch_shifts_setup(const double* __restrict__ dv, const double* 
     int k0 = 0;
     if (w > nb) k0 = min(max(window_count32(sd, se2, w, sd[w - 1]) - nb / 2, 0), w - nb);
     if (lane == 0) {
-        sw.w = w;
-        sw.k0 = k0;
-        sw.ex = ex;
-        sw.trivial = 0;
-        sw.lo = lo - 1e-6f;
-        sw.hi = hi + 1e-6f;
+        bs->win_w = w;
+        bs->win_k0 = k0;
+        bs->win_ex = ex;
+        bs->win_trivial = 0;
+        bs->win_lo = lo - 1e-6f;
+        bs->win_hi = hi + 1e-6f;
     }
     __syncwarp();
 }
 
-// All threads of the CTA (after a barrier that follows the setup): thread j finds shift j,
-// j + blockDim.x, ...  FP32 bisection to a bracket, then the safeguarded FP64 Newton iteration.
-__device__ void batch_shifts_solve(const double* __restrict__ dv, int64_t to, int nb, const ShiftWindow& sw,
-                                   double* __restrict__ shifts, const float* sd, const float* se2,
-                                   const double* dd, const double* ee2)
+// A bulge's copy of the window.
+struct ShiftSmem {
+    float sd[kWinMax], se2[kWinMax];
+    double dd[kWinMax], nbb[kWinMax + 1];      // diagonal; nbb[i] = -e_{i-1}^2, nbb[0] = 0
+    double aa[kWinMax + 1], p[kWinMax + 1];    // dd - x; the leading minors at x
+};
+
+// p(x), p'(x) and the count by one warp: even lanes carry the minors, odd lanes their derivatives one
+// step behind, so a step is two FP64 instructions for both (p_i = aa p_{i-1} + RN(nbb p_{i-2}),
+// q_i = aa q_{i-1} + RN(nbb q_{i-2} - p_{i-1}), char_poly's operations).  The rescaling is
+// checked every eight steps against 2^+-300 (a step shrinks a minor by less than 2^-105 and grows it
+// by less than 4) and changes no bit of p / p'.
+__device__ __forceinline__ void char_poly_warp(ShiftSmem& sm, int w, double x, double& p, double& dp, int& below)
 {
-    if (sw.trivial) {
-        for (int j = threadIdx.x; j < nb; j += blockDim.x) shifts[j] = dv[to - nb + j];
+    const int lane = threadIdx.x & 31;
+    const bool odd = lane & 1;
+    for (int i = lane; i < w; i += 32) sm.aa[i] = __dsub_rn(sm.dd[i], x);
+    if (lane == 0) sm.aa[w] = 0.0;
+    __syncwarp();
+    const double* aa = sm.aa - odd;
+    const double* bb = sm.nbb - odd;
+    const uint32_t m = odd ? ~0u : 0u;
+    double z0 = odd ? 0.0 : 1.0, z1 = odd ? 0.0 : sm.aa[0];
+    if (lane == 0) sm.p[0] = z1;
+#pragma unroll 1
+    for (int s = 1; s <= w; ++s) {
+        const double up = __shfl_sync(0xffffffffu, z0, lane & 30);
+        const double add = lane_sel(m, lane_sign(up, ~0u, 0x80000000u), -0.0);
+        const double z2 = __fma_rn(aa[s], z1, __fma_rn(bb[s], z0, add));
+        z0 = z1;
+        z1 = z2;
+        if (lane == 0) sm.p[s] = z2;
+        if ((s & 7) == 0) {
+            const int hi = __shfl_sync(0xffffffffu, __double2hiint(z1), 0);
+            const int e = ((hi >> 20) & 0x7FF) - 1023;
+            if ((e > 300 && e < 1024) || (e < -300 && e > -1023)) {
+                const double sc = __longlong_as_double((long long)(1023 - e) << 52);   // 2^-e, exact
+                z0 *= sc;
+                z1 *= sc;
+            }
+        }
+    }
+    __syncwarp();
+    p = lane_get(z0, 0);
+    dp = lane_get(z1, 1);
+    int cnt = 0;
+    bool zero = false;
+    for (int i = lane; i < w; i += 32) {
+        const double pi = sm.p[i];
+        zero |= pi == 0.0;
+        cnt += (pi < 0.0) != (i > 0 && sm.p[i - 1] < 0.0);
+    }
+    if (__any_sync(0xffffffffu, zero)) {
+        char_poly(sm.dd, sm.nbb, w, x, p, dp, below);
         return;
     }
-    const int w = sw.w;
-    for (int j = threadIdx.x; j < nb; j += blockDim.x) {
-        const int k = sw.k0 + j;
-        float a = sw.lo, b = sw.hi;
-        for (int it = 0; it < 40; ++it) {
-            const float mid = 0.5f * (a + b);
-            if (!(mid > a && mid < b)) break;
-            if (window_count32(sd, se2, w, mid) > k) b = mid;
-            else a = mid;
-        }
-        // FP64 refinement inside a bracket kept by FP64 Sturm counts
-        double A = (double)a - 4e-7, B = (double)b + 4e-7;
-        double x = 0.5 * ((double)a + (double)b);
-        for (int it = 0; it < 5; ++it) {
-            double p, dp;
-            int below;
-            char_poly(dd, ee2, w, x, p, dp, below);
-            if (below > k) B = x;
-            else A = x;
-            const double step = p / dp;
-            // converged: a step below the last bits ends the iteration first (such a step can
-            // land on the bracket's edge, which the safeguard below would turn into a jump)
-            if (fabs(step) <= 4e-16 * fabs(x) + 1e-300) break;
-            double xn = x - step;
-            if (!(xn > A && xn < B)) xn = 0.5 * (A + B);
-            x = xn;
-        }
-        shifts[j] = ldexp(x, sw.ex);
+    below = __reduce_add_sync(0xffffffffu, cnt);
+}
+
+// Shift j of the batch, by one warp of bulge j's CTA, every CTA at once: FP32 bisection to a bracket,
+// five levels a round (lane n of 1 .. 31 counts at the midpoint a bisection would reach at node n
+// of its tree, so the path is the bisection's), then the safeguarded FP64 Newton iteration.  One
+// thread per shift in the controller, 40 levels and both recurrences in sequence, took about
+// 285 us for 64 shifts of a 128-row window (n = 2000 multishift solve 125 ms, 113 ms this way).
+__device__ double bulge_shift(const BulgeScratch* bs, int j, ShiftSmem& sm)
+{
+    const int lane = threadIdx.x & 31;
+    if (bs->win_trivial) return bs->shifts[j];
+    const int w = bs->win_w, k = bs->win_k0 + j;
+    for (int q = lane; q < w; q += 32) {
+        const double d = bs->win_d[q], e = bs->win_e[q];
+        const float ef = (float)e;
+        sm.sd[q] = (float)d;
+        sm.se2[q] = ef * ef;
+        sm.dd[q] = d;
+        sm.nbb[q + 1] = -(e * e);
     }
+    if (lane == 0) sm.nbb[0] = 0.0;
+    __syncwarp();
+    float a = bs->win_lo, b = bs->win_hi;
+    const int depth = 31 - __clz(lane | 1);
+    for (int it = 0; it < 40; it += 5) {
+        float na = a, nb = b, mid = 0.0f;
+        bool valid = lane > 0;
+        for (int l = 0; l <= depth; ++l) {
+            mid = 0.5f * (na + nb);
+            valid = valid && mid > na && mid < nb;
+            if (l < depth) {
+                if ((lane >> (depth - 1 - l)) & 1) na = mid;
+                else nb = mid;
+            }
+        }
+        const unsigned above = __ballot_sync(0xffffffffu, window_count32(sm.sd, sm.se2, w, mid) > k);
+        const unsigned ok = __ballot_sync(0xffffffffu, valid);
+        bool done = false;
+        for (int l = 0, node = 1; l < 5; ++l) {
+            if (!((ok >> node) & 1u)) {
+                done = true;
+                break;
+            }
+            mid = 0.5f * (a + b);
+            if ((above >> node) & 1u) {
+                b = mid;
+                node = 2 * node;
+            } else {
+                a = mid;
+                node = 2 * node + 1;
+            }
+        }
+        if (done) break;
+    }
+    // FP64 refinement inside a bracket kept by FP64 Sturm counts
+    double A = (double)a - 4e-7, B = (double)b + 4e-7;
+    double x = 0.5 * ((double)a + (double)b);
+    for (int it = 0; it < 5; ++it) {
+        double p, dp;
+        int below;
+        char_poly_warp(sm, w, x, p, dp, below);
+        if (below > k) B = x;
+        else A = x;
+        const double step = p / dp;
+        // converged: a step below the last bits ends the iteration first (such a step can
+        // land on the bracket's edge, which the safeguard below would turn into a jump)
+        if (fabs(step) <= 4e-16 * fabs(x) + 1e-300) break;
+        double xn = x - step;
+        if (!(xn > A && xn < B)) xn = 0.5 * (A + B);
+        x = xn;
+    }
+    return ldexp(x, bs->win_ex);
 }
 
 // The bulges of a batch.  Bulge j (CTA j) runs the one-warp sweep with shift shifts[j] over the
@@ -758,6 +839,7 @@ bulge_batch_kernel(const ChaseState* __restrict__ st, double* dv, double* ev, do
                    int* __restrict__ err)
 {
     __shared__ BulgeRing ring;
+    __shared__ ShiftSmem shift;
     const int j = blockIdx.x;
     if (st->status != CHASE_BATCH) return;  // a launch queued ahead after the batches ended
     const int32_t nb = st->b_bulges;
@@ -768,7 +850,7 @@ bulge_batch_kernel(const ChaseState* __restrict__ st, double* dv, double* ev, do
     const int steps = (int)(to - from), every = st->ms_prog_mask + 1;
     const int warp = threadIdx.x >> 5;
     if (warp == 0) {
-        bulge_sweep(ring, steps, every, bs->shifts[j], st->neg_zero);
+        bulge_sweep(ring, steps, every, bulge_shift(bs, j, shift), st->neg_zero);
     } else if (warp == 1) {
         bulge_fetch(ring, dv, ev, from, to, steps, every, PipeWait{j > 0 ? &bs->prog[j - 1] : nullptr, err, -1});
     } else {
@@ -780,7 +862,7 @@ bulge_batch_kernel(const ChaseState* __restrict__ st, double* dv, double* ev, do
 // One flush: the reference's inner loop from `to = last_block_ends_at` until the matrix is
 // split into converged parts, every block has reached max_layers, or iter > maxiter.
 // Warp 0 runs the control flow, the O(n) scans with ballots and the sweeps (sweep_warp); warp 1
-// shares the O(n) updates and the shift solve.  In chase modes 1 and 2 every sweep runs in the
+// shares the O(n) updates.  In chase modes 1 and 2 every sweep runs in the
 // reference form on one thread (mode 2: after the warp's sweep, undone from the copy `bak`, 2n
 // doubles, of the entries it may change).
 //
@@ -808,8 +890,6 @@ chase_kernel(ChaseState* __restrict__ st, double* __restrict__ dv, double* __res
 {
     __shared__ Decision dec;
     __shared__ float ms_d[kWinMax], ms_e2[kWinMax], ms_ea[kWinMax];
-    __shared__ double ms_dd[kWinMax], ms_ee2[kWinMax];
-    __shared__ ShiftWindow swin;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int64_t n = st->n;
@@ -902,7 +982,7 @@ chase_kernel(ChaseState* __restrict__ st, double* __restrict__ dv, double* __res
                                 if (nbl < ms_min) nbl = 1;
                             }
                             if (nbl >= 2) {
-                                batch_shifts_setup(dv, ev, from, to, (int)nbl, swin, ms_d, ms_e2, ms_ea, ms_dd, ms_ee2);
+                                batch_shifts_setup(dv, ev, from, to, (int)nbl, bs, ms_d, ms_e2, ms_ea);
                                 d.bulges = (int32_t)nbl;
                                 d.action = 3;
                             } else {
@@ -928,8 +1008,7 @@ chase_kernel(ChaseState* __restrict__ st, double* __restrict__ dv, double* __res
         const Decision d = dec;
         last = d;
         if (d.action == 3) {
-            // the batch's shifts, one per thread, then the batch runs in its own launch
-            batch_shifts_solve(dv, d.to, d.bulges, swin, bs->shifts, ms_d, ms_e2, ms_dd, ms_ee2);
+            // the batch runs in its own launch
             break;
         }
         if (d.action == 1) {

@@ -68,10 +68,13 @@ constexpr int kDefaultProgEvery = 4;
 constexpr int kDefaultMinBulges = 2;
 constexpr int kBatchesAhead = 8;
 
-// Device scratch of a batch: the bulges' shifts and their progress words.
+// Device scratch of a batch: the bulges' progress words and the shift window (chase.cu).
 struct BulgeScratch {
-    double shifts[kMaxBulges];
     long long prog[kMaxBulges];  // last step whose stores a bulge has released
+    double shifts[kMaxBulges];   // the shifts, where the window is trivial
+    double win_d[2 * kMaxBulges], win_e[2 * kMaxBulges];   // its scaled diagonal and off-diagonal
+    int32_t win_w, win_k0, win_ex, win_trivial;   // rows, rank of the first shift, scale, see chase.cu
+    float win_lo, win_hi;        // Gershgorin interval
 };
 
 struct ChaseState {
