@@ -34,16 +34,28 @@ __device__ __forceinline__ bool is_small(const double* dv, const double* ev, int
     return fabs(ev[j - 1]) <= __dmul_rn(tol, __dadd_rn(fabs(dv[j - 1]), fabs(dv[j])));
 }
 
-// Wilkinson shift from the trailing 2x2 block [a c; c b] (src/bulge_chasing.jl:239-265).
+// False only where is_small is false, from the exponent fields: |e| >= 2^(xe-1023), while
+// tol (|d_j| + |d_j+1|) < 2^(xt-1023+1) 2^(max(xd)-1023+2).  An FP64 instruction costs 64 cycles,
+// so the scan runs the exact test only where this cannot decide.
+__device__ __forceinline__ bool maybe_small(double e, double d0, double d1, int32_t xt)
+{
+    const int32_t xe = (__double2hiint(e) >> 20) & 0x7FF;
+    const int32_t xd = max((__double2hiint(d0) >> 20) & 0x7FF, (__double2hiint(d1) >> 20) & 0x7FF);
+    return xe == 0 || xe < xt + xd - 1020;
+}
+
+// Wilkinson shift from the trailing 2x2 block [a c; c b] (src/bulge_chasing.jl:239-265), by a
+// warp: the three divisions by the scale in three lanes at once (650 cycles each).
 __device__ __forceinline__ double wilkinson_shift(double a, double b, double c)
 {
+    const int lane = threadIdx.x & 31;
     const double scale = __dadd_rn(__dadd_rn(fabs(a), __dmul_rn(2.0, fabs(c))), fabs(b));
-    const double H11 = __ddiv_rn(a, scale), H12 = __ddiv_rn(c, scale), H22 = __ddiv_rn(b, scale);
-    const double t = __ddiv_rn(__dadd_rn(H11, H22), 2.0);
+    const double q = __ddiv_rn(lane == 0 ? a : lane == 1 ? c : b, scale);
+    const double H11 = __shfl_sync(0xffffffffu, q, 0), H12 = __shfl_sync(0xffffffffu, q, 1),
+                 H22 = __shfl_sync(0xffffffffu, q, 2);
+    const double t = __dmul_rn(__dadd_rn(H11, H22), 0.5);   // (H11 + H22) / 2
     const double p = __dmul_rn(__dsub_rn(H11, t), __dsub_rn(H22, t));
-    const double q = __dmul_rn(H12, H12);
-    const double d = __dsub_rn(p, q);
-    const double sq = __dsqrt_rn(fabs(d));
+    const double sq = __dsqrt_rn(fabs(__dsub_rn(p, __dmul_rn(H12, H12))));
     const double l1 = __dadd_rn(t, sq), l2 = __dsub_rn(t, sq);
     const double lam = fabs(__dsub_rn(H22, l1)) < fabs(__dsub_rn(H22, l2)) ? l1 : l2;
     return __dmul_rn(lam, scale);
@@ -158,7 +170,7 @@ __device__ void single_shift(double* __restrict__ dv, double* __restrict__ ev, i
 // (lane 5) are the next step's B11 and B21.  The lanes' operands are picked by bit masks: the
 // same selections written as ternaries compiled to divergent branches and cost 330 cycles.
 // The step's results go to memory during the next step: lane 1 stores dv, lane 2 ev, lanes 4
-// and 5 the pair (c, s), one masked store.  Measured 1077 cycles per step, against 1802 for the
+// and 5 the pair (c, s), one masked store.  Measured 890 to 1040 cycles per step, against 1802 for the
 // two-warp Newton form this replaces and 1130 for a split over four warps with named barriers
 // (the warps' FP64 instructions queue for the SM's one unit).
 //
@@ -214,20 +226,6 @@ __device__ __forceinline__ SweepLanes sweep_lanes()
     return L;
 }
 
-// Levels 1 to 4 of a step (see above): v2, v4 per lane, and the next bulge g with gg = g^2.
-__device__ __forceinline__ void sweep_update(const SweepLanes& L, double c, double s, double a1, double a2,
-                                             double nz, double& v2, double& v4, double& g, double& gg)
-{
-    const double p1 = __fma_rn(lane_sign(s, L.keep1, L.flip1), a1, nz);
-    v2 = __fma_rn(c, a2, p1);
-    const double m3 = lane_sel(L.m4, p1, lane_sign(s, ~0u, L.flip3));
-    const double p3 = __fma_rn(v2, m3, nz);
-    const double oth = __shfl_xor_sync(0xffffffffu, v2, 1);
-    v4 = __fma_rn(oth, c, p3);
-    g = lane_get(p1, 4);
-    gg = lane_get(p3, 4);
-}
-
 // What a sweep carries from step to step: the next rotation's (f, g) and x = f^2 + g^2, the
 // lanes' v2 and v4, and the last rotation.
 struct SweepRegs {
@@ -254,28 +252,42 @@ __device__ __forceinline__ double sweep_result(const SweepLanes& L, const SweepR
 }
 
 // One step with the entries B22 = dv[i+1], B23 = ev[i+1] (1-based i).  `emit` puts the last
-// step's result away, beside this step's rotation.
-template <typename Emit>
+// step's result away, `fetch` starts the loads of the next step's entries.
+// The order of the statements matters: the compiler keeps the shuffles and memory operations
+// about where they stand, and these wait in one queue with the FP64 instructions.  96 orders were
+// timed in place, all with the same results (n = 750 default solve 180 to 215 ms, eigenvalues of
+// n = 1500 by multishift 52 to 58 ms, 256 small ones in a batch 60 to 74 ms); this one is best
+// or near it in all three.
+template <typename Emit, typename Fetch>
 __device__ __forceinline__ void sweep_step(const SweepLanes& L, SweepRegs& S, double B22, double B23, double nz,
-                                           Emit emit)
+                                           Emit emit, Fetch fetch)
 {
+    // the lanes' operands that the entries alone give; the others are B11 or B21
+    const double e1 = lane_sel(L.m1, B22, lane_sel(L.m5, -0.0, B23)), e2 = lane_sel(L.m3, B22, lane_sel(L.m5, B23, 0.0));
+    const double B11 = lane_get(S.v4, 2), B21 = lane_get(S.v2, 5);
     double c, s, r;
     IntRot K;
     givens_int(S.f, S.g, S.x, c, s, r, K);
-    const double B11 = lane_get(S.v4, 2), B21 = lane_get(S.v2, 5);
+    fetch();
     emit(sweep_result(L, S));
-    const double a1 = lane_sel(L.m1, B22, lane_sel(L.m2, B11, lane_sel(L.m5, -0.0, lane_sel(L.m4, B23, B21))));
-    const double a2 = lane_sel(L.m0, B11, lane_sel(L.m3, B22, lane_sel(L.m5, B23, lane_sel(L.m4, 0.0, B21))));
-    double g, gg;
-    sweep_update(L, c, s, a1, a2, nz, S.v2, S.v4, g, gg);
+    const double a1 = lane_sel(L.m1 | L.m4 | L.m5, e1, lane_sel(L.m2, B11, B21));
+    const double a2 = lane_sel(L.m3 | L.m4 | L.m5, e2, lane_sel(L.m0, B11, B21));
+    double p1 = __fma_rn(lane_sign(s, L.keep1, L.flip1), a1, nz);
+    double v2 = __fma_rn(c, a2, p1);
+    double p3 = __fma_rn(v2, lane_sel(L.m4, p1, lane_sign(s, ~0u, L.flip3)), nz);
+    double v4 = __fma_rn(__shfl_xor_sync(0xffffffffu, v2, 1), c, p3);
     if (__any_sync(0xffffffffu, !K.in_range || K.undecided != 0u)) {
         const Rot3 o = givens_fix(S.f, S.g, K, nz);
         c = o.c; s = o.s; r = o.r;
-        sweep_update(L, c, s, a1, a2, nz, S.v2, S.v4, g, gg);
+        p1 = __fma_rn(lane_sign(s, L.keep1, L.flip1), a1, nz);
+        v2 = __fma_rn(c, a2, p1);
+        p3 = __fma_rn(v2, lane_sel(L.m4, p1, lane_sign(s, ~0u, L.flip3)), nz);
+        v4 = __fma_rn(__shfl_xor_sync(0xffffffffu, v2, 1), c, p3);
     }
-    S.f = lane_get(S.v4, 0);
-    S.x = __dadd_rn(mulz(S.f, S.f, nz), gg);
-    S.g = g;
+    const double f = lane_get(v4, 0), g = lane_get(p1, 4), gg = lane_get(p3, 4);
+    S.x = __dadd_rn(mulz(f, f, nz), gg);
+    S.v2 = v2; S.v4 = v4;
+    S.f = f; S.g = g;
     S.c = c; S.s = s; S.r = r;
 }
 
@@ -305,13 +317,14 @@ __device__ void sweep_warp(double* __restrict__ dv, double* __restrict__ ev, int
     };
 #pragma unroll 1
     for (int k = 0; k < steps; ++k) {
-        const double B22 = B22n, B23 = B23n;
-        B22n = k + 2 <= steps ? *ld : 0.0;
-        B23n = k + 3 <= steps ? *le : 0.0;
-        ++ld;
-        ++le;
-        if (!ONE_LAYER) t_next = k + 2 <= steps ? thick[from + k] : 0;
-        sweep_step(L, S, B22, B23, nz, [&](double v) { put(v, k == 0, k == 1); });
+        sweep_step(L, S, B22n, B23n, nz, [&](double v) { put(v, k == 0, k == 1); },
+                   [&] {
+                       B22n = k + 2 <= steps ? *ld : 0.0;
+                       B23n = k + 3 <= steps ? *le : 0.0;
+                       ++ld;
+                       ++le;
+                       if (!ONE_LAYER) t_next = k + 2 <= steps ? thick[from + k] : 0;
+                   });
         t_out = t_cur;
         t_cur = t_next;
     }
@@ -335,16 +348,19 @@ __device__ __forceinline__ int64_t block_start(const double* dv, const double* e
                                                double tol)
 {
     const int lane = threadIdx.x & 31;
+    const int32_t xt = (__double2hiint(tol) >> 20) & 0x7FF;
     for (int64_t base = to - 1; base >= start; base -= 32 * kScanUnroll) {
-        bool sm[kScanUnroll];
+        bool may[kScanUnroll];
 #pragma unroll
         for (int u = 0; u < kScanUnroll; ++u) {
             const int64_t j = base - 32 * u - lane;
-            sm[u] = (j >= start) && is_small(dv, ev, j, tol);
+            may[u] = j >= start && maybe_small(ev[j - 1], dv[j - 1], dv[j], xt);
         }
 #pragma unroll
         for (int u = 0; u < kScanUnroll; ++u) {
-            const unsigned mask = __ballot_sync(0xffffffffu, sm[u]);
+            if (!__any_sync(0xffffffffu, may[u])) continue;
+            const int64_t j = base - 32 * u - lane;
+            const unsigned mask = __ballot_sync(0xffffffffu, may[u] && is_small(dv, ev, j, tol));
             if (mask) return base - 32 * u - (__ffs(mask) - 1) + 1;
         }
     }
@@ -360,15 +376,32 @@ __device__ __forceinline__ int32_t warp_range_max(const int32_t* a, int64_t lo, 
     return warp_max(v);
 }
 
-// The exact-order layer of a sweep over [from, to] (see chase_kernel), and the identity in the
-// slots the jump to it skips.
-__device__ __forceinline__ int32_t exact_layer(const int32_t* place, int64_t from, int64_t to, int64_t n)
+// What a sweep over [from, to] meets: the thickest column, the exact-order layer (see chase_kernel)
+// and the least filled slot among its rotations' columns.
+struct SweepRoom {
+    int32_t thickest, layer, least;
+};
+__device__ __forceinline__ SweepRoom sweep_room(const int32_t* thick, const int32_t* place, int64_t from, int64_t to,
+                                                int64_t n)
 {
-    int32_t L = warp_range_max(place, from - 1, to - 2);
-    if (to <= n - 1) L = max(L, place[to - 1]);
-    if (from >= 2) L = max(L, place[from - 2] - 1);
-    return L + 1;
+    int32_t t = 0, hi = 0, lo = INT32_MAX;
+    const int32_t after = to <= n - 1 ? place[to - 1] : 0, before = from >= 2 ? place[from - 2] - 1 : 0;
+#pragma unroll 4
+    for (int64_t q = from - 1 + (threadIdx.x & 31); q <= to - 1; q += 32) {
+        t = max(t, thick[q]);
+        if (q < to - 1) {
+            const int32_t p = place[q];
+            hi = max(hi, p);
+            lo = min(lo, p);
+        }
+    }
+    SweepRoom r;
+    r.thickest = warp_max(t);
+    r.layer = 1 + max(warp_max(hi), max(after, before));
+    r.least = __reduce_min_sync(0xffffffffu, lo);
+    return r;
 }
+// The identity in the slots the jump to `layer` skips.
 __device__ __forceinline__ void fill_skipped(double* grid, const int32_t* place, int64_t from, int64_t to,
                                              int32_t layer, int64_t rows)
 {
@@ -754,7 +787,7 @@ __device__ __forceinline__ void bulge_sweep(BulgeRing& R, int steps, int every, 
             sweep_step(L, S, B.x, B.y, nz, [&](double v) {
                 asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q st.shared.f64 [%0], %1;\n\t}"
                              ::"r"(at), "d"(v), "r"((unsigned)(stores && k0 + q > 0)) : "memory");
-            });
+            }, [] {});
             if (q == 0 && k0 > 0) {
                 __syncwarp();
                 nb_arrive(kBarOutFull + (b ^ 1));
@@ -952,19 +985,20 @@ chase_kernel(ChaseState* __restrict__ st, double* __restrict__ dv, double* __res
                     if (to == lbe) lbe -= 1;
                     to -= 1;
                 } else {
-                    const int32_t mx = warp_range_max(thick, from - 1, to - 1);
+                    const SweepRoom room = sweep_room(thick, place, from, to, n);
+                    const int32_t mx = room.thickest;
                     if (mx == max_layers) {
                         to = from - 1;
                     } else {
                         int32_t layer = 0;
                         bool go = true;
                         if (exact) {
-                            layer = exact_layer(place, from, to, n);
+                            layer = room.layer;
                             if (layer > grid_layers) {
                                 early = 1;
                                 go = false;
                                 d.action = 0;
-                            } else {
+                            } else if (room.least < layer - 1) {
                                 fill_skipped(grid, place, from, to, layer, rows);
                             }
                         }
@@ -1143,15 +1177,15 @@ __device__ void chase_flush_warp(ChaseState* __restrict__ st, double* __restrict
             if (to == lbe) lbe -= 1;
             to -= 1;
         } else {
-            const int32_t mx = warp_range_max(thick, from - 1, to - 1);
-            if (mx == max_layers) {
+            const SweepRoom room = sweep_room(thick, place, from, to, n);
+            if (room.thickest == max_layers) {
                 to = from - 1;
             } else {
                 int32_t layer = 0;
                 if (exact) {
-                    layer = exact_layer(place, from, to, n);
+                    layer = room.layer;
                     if (layer > grid_layers) { early = 1; break; }
-                    fill_skipped(grid, place, from, to, layer, rows);
+                    if (room.least < layer - 1) fill_skipped(grid, place, from, to, layer, rows);
                 }
                 const double mu = wilkinson_shift(dv[to - 2], dv[to - 1], ev[to - 2]);
                 if (layer > 0) sweep_warp<true>(dv, ev, from, to, mu, grid, thick, rows, layer, nz);
@@ -1186,7 +1220,7 @@ __device__ void chase_flush_warp(ChaseState* __restrict__ st, double* __restrict
     }
 }
 
-constexpr int kBatchWarps = 4;   // matrices per CTA, one on each SM sub-partition
+constexpr int kBatchWarps = 4;   // most matrices per CTA, one on each SM sub-partition
 
 __global__ void __launch_bounds__(32 * kBatchWarps)
 chase_batched_kernel(const BatchMat* __restrict__ mats, const int32_t* __restrict__ order,
@@ -1194,7 +1228,7 @@ chase_batched_kernel(const BatchMat* __restrict__ mats, const int32_t* __restric
                      double* __restrict__ e, double* __restrict__ grids,
                      int32_t* __restrict__ thick, int32_t* __restrict__ place)
 {
-    const int32_t k = blockIdx.x * kBatchWarps + (threadIdx.x >> 5);
+    const int32_t k = (int32_t)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
     if (k >= count) return;
     const int32_t i = order[k];
     ChaseState* st = states + i;
@@ -1263,8 +1297,10 @@ cudaError_t launch_chase_batched(const BatchMat* mats, const int32_t* order, int
                                  int32_t* thick, int32_t* place, cudaStream_t stream)
 {
     if (count <= 0) return cudaSuccess;
-    chase_batched_kernel<<<(count + kBatchWarps - 1) / kBatchWarps, 32 * kBatchWarps, 0, stream>>>(mats, order, count, states, d, e,
-                                                               grids, thick, place);
+    // a small batch spreads over the SMs: chases on one SM queue for its FP64 unit
+    const int32_t warps = count <= 152 ? 1 : count <= 304 ? 2 : kBatchWarps;
+    chase_batched_kernel<<<(unsigned)((count + warps - 1) / warps), 32 * warps, 0, stream>>>(mats, order, count, states, d,
+                                                                                            e, grids, thick, place);
     return cudaGetLastError();
 }
 
