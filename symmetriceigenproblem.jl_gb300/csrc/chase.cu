@@ -1297,8 +1297,10 @@ cudaError_t launch_chase_batched(const BatchMat* mats, const int32_t* order, int
                                  int32_t* thick, int32_t* place, cudaStream_t stream)
 {
     if (count <= 0) return cudaSuccess;
-    // a small batch spreads over the SMs: chases on one SM queue for its FP64 unit
-    const int32_t warps = count <= 152 ? 1 : count <= 304 ? 2 : kBatchWarps;
+    // One matrix per SM while there are enough SMs (chases on one SM queue for its FP64 unit: 16 of
+    // n = 50 .. 250 31.3 against 32.1 ms).  From there four, so that the round's apply beside
+    // it has SMs of its own (256 of n = 200 .. 256, FP64 Q: 68.5 ms, 77.2 with two per CTA).
+    const int32_t warps = count <= 152 ? 1 : kBatchWarps;
     chase_batched_kernel<<<(unsigned)((count + warps - 1) / warps), 32 * warps, 0, stream>>>(mats, order, count, states, d,
                                                                                             e, grids, thick, place);
     return cudaGetLastError();
