@@ -10,8 +10,10 @@
 // autograd Function of the host bindings.  Q is the solver's output, so no rotation history
 // is stored.
 //
-// Two FP64 tensor-core GEMMs (dmma_tile.cuh: mma.sync m8n8k4 .f64, the FP64 MMA of sm_103a;
-// tcgen05 has no f64 kind) with fused epilogues:
+// Two FP64 GEMMs with fused epilogues, on the bf16 tensor cores by exact slices (sliced_gemm.cuh)
+// from n = kSlicedMin on, else (and where Q is localized or an operand holds an infinity or NaN,
+// which the device decides) on the FP64 MMA
+// (dmma_tile.cuh: mma.sync m8n8k4 .f64; tcgen05 has no f64 kind):
 //   1. G = Q^T gQ, epilogue M_ij = i == j ? glam_i : G_ij / (lam_j - lam_i), M stored.
 //   2. P = Q M, epilogue: per row i the partial sums over the CTA's columns k of
 //        P_ik Q_ik (-> dd_i),  P_ik Q_{i+1,k} and P_ik Q_{i-1,k} (-> de_i, de_{i-1}),
@@ -20,9 +22,12 @@
 // A batch of matrices of one order runs with blockIdx.z = matrix.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "symeig.h"
 #include "symeig_common.cuh"
 #include "dmma_tile.cuh"
+#include "sliced_gemm.cuh"
 
 namespace symeig {
 namespace {
@@ -36,8 +41,9 @@ __global__ void __launch_bounds__(kAdjThreads)
 adjoint_m_kernel(const double* __restrict__ Q, int64_t ldq, const double* __restrict__ gQ,
                  int64_t ldg, const double* __restrict__ lam, const double* __restrict__ glam,
                  int64_t n, double* __restrict__ Mout, int64_t strideQ, int64_t strideG,
-                 int64_t strideM)
+                 int64_t strideM, const int* __restrict__ only_if)
 {
+    if (only_if && !only_if[blockIdx.z]) return;   // the sliced kernel did it
     __shared__ dmma::Smem sm;
     const int64_t z = blockIdx.z;
     Q += z * strideQ;
@@ -77,8 +83,9 @@ adjoint_m_kernel(const double* __restrict__ Q, int64_t ldq, const double* __rest
 __global__ void __launch_bounds__(kAdjThreads)
 adjoint_p_kernel(const double* __restrict__ Q, int64_t ldq, const double* __restrict__ M,
                  int64_t n, double* __restrict__ part, int64_t strideQ, int64_t strideM,
-                 int64_t stridePart)
+                 int64_t stridePart, const int* __restrict__ only_if)
 {
+    if (only_if && !only_if[blockIdx.z]) return;
     __shared__ dmma::Smem sm;
     __shared__ double red[3][2][BM];
     const int64_t z = blockIdx.z;
@@ -135,14 +142,15 @@ adjoint_p_kernel(const double* __restrict__ Q, int64_t ldq, const double* __rest
 }
 
 // 3. dd_i = sum_tiles part0[i];  de_i = sum_tiles (part1[i] + part2[i+1]).
+// part holds the FP64 MMA's column tiles, or with `fallback` given and clear the sliced kernel's.
 __global__ void adjoint_reduce_kernel(const double* __restrict__ part, int64_t n, double* __restrict__ gd,
-                                      double* __restrict__ ge, int64_t stridePart)
+                                      double* __restrict__ ge, int64_t stridePart, const int* __restrict__ fallback)
 {
     const int64_t z = blockIdx.y;
     part += z * stridePart;
     gd += z * n;
     ge += z * (n > 1 ? n - 1 : 0);
-    const int64_t tiles = (n + BN - 1) / BN;
+    const int64_t tiles = fallback && !fallback[blockIdx.y] ? (n + sliced::BN - 1) / sliced::BN : (n + BN - 1) / BN;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         double sd = 0.0, se = 0.0;
         for (int64_t t = 0; t < tiles; ++t) {
@@ -151,6 +159,110 @@ __global__ void adjoint_reduce_kernel(const double* __restrict__ part, int64_t n
         }
         gd[i] = sd;
         if (i + 1 < n) ge[i] = se;
+    }
+}
+
+// ---- the same on the bf16 tensor cores (sliced_gemm.cuh) -------------------------------------
+
+// 1. as adjoint_m_kernel.  A: planes of Q's columns with exponents ea; B: of gQ's columns with eb.
+__global__ void __launch_bounds__(sliced::kThreads, 1)
+sliced_m_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B, const int* __restrict__ ea,
+                const int* __restrict__ eb, const double* __restrict__ lam, const double* __restrict__ glam, int64_t n,
+                int64_t rows, int64_t kp, int64_t pstride, double* __restrict__ Mout, const int* __restrict__ fallback)
+{
+    extern __shared__ __align__(128) unsigned char smem[];
+    if (fallback[blockIdx.z]) return;
+    const int64_t z = blockIdx.z;
+    lam += z * n;
+    glam += z * n;
+    Mout += z * n * n;
+    const int64_t i0 = (int64_t)blockIdx.y * sliced::BM, j0 = (int64_t)blockIdx.x * sliced::BN;
+    double acc[4][4][4];
+    sliced::tile_product(A + z * pstride, B + z * pstride, rows, kp, i0, j0, smem, acc);
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+#pragma unroll
+        for (int h = 0; h < 4; h += 2) {
+            const int64_t i = i0 + sliced::tile_row(x, h);
+            if (i >= n) continue;
+            const int e = ea[z * n + i];
+            const double li = lam[i];
+#pragma unroll
+            for (int y = 0; y < 4; ++y)
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const int64_t j = j0 + sliced::tile_col(y, q);
+                    if (j >= n) continue;
+                    double v;
+                    if (i == j) {
+                        v = glam[i];
+                    } else {
+                        const double gap = lam[j] - li;
+                        v = gap != 0.0 ? scalbn(acc[x][y][h + q], e + eb[z * n + j]) / gap : 0.0;
+                    }
+                    Mout[i + j * n] = v;
+                }
+        }
+}
+
+// 2. as adjoint_p_kernel.  A: planes of Q's rows with exponents ea; B: of M's columns with eb.
+__global__ void __launch_bounds__(sliced::kThreads, 1)
+sliced_p_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B, const int* __restrict__ ea,
+                const int* __restrict__ eb, const double* __restrict__ Q, int64_t n, int64_t rows, int64_t kp,
+                int64_t pstride, double* __restrict__ part, int64_t stridePart, const int* __restrict__ fallback)
+{
+    extern __shared__ __align__(128) unsigned char smem[];
+    if (fallback[blockIdx.z]) return;
+    double(*red)[4][sliced::BM] = reinterpret_cast<double(*)[4][sliced::BM]>(smem);   // [3], in the ring
+    const int64_t z = blockIdx.z;
+    Q += z * n * n;
+    part += z * stridePart;
+    const int64_t i0 = (int64_t)blockIdx.y * sliced::BM, k0 = (int64_t)blockIdx.x * sliced::BN;
+    double acc[4][4][4];
+    sliced::tile_product(A + z * pstride, B + z * pstride, rows, kp, i0, k0, smem, acc);
+    const int tig = threadIdx.x & 3, wcol = (threadIdx.x >> 5) & 3;
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+#pragma unroll
+        for (int h = 0; h < 4; h += 2) {
+            const int r = sliced::tile_row(x, h);
+            const int64_t i = i0 + r;
+            double sd = 0.0, su = 0.0, sl = 0.0;
+            if (i < n) {
+                const int e = ea[z * n + i];
+#pragma unroll
+                for (int y = 0; y < 4; ++y)
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        const int64_t k = k0 + sliced::tile_col(y, q);
+                        if (k >= n) continue;
+                        const double p = scalbn(acc[x][y][h + q], e + eb[z * n + k]);
+                        sd = fma(p, Q[i + k * n], sd);
+                        if (i + 1 < n) su = fma(p, Q[i + 1 + k * n], su);
+                        if (i >= 1) sl = fma(p, Q[i - 1 + k * n], sl);
+                    }
+            }
+            // the 4 lanes of a group hold the same row: sum them
+#pragma unroll
+            for (int o = 1; o < 4; o <<= 1) {
+                sd += __shfl_xor_sync(0xffffffffu, sd, o);
+                su += __shfl_xor_sync(0xffffffffu, su, o);
+                sl += __shfl_xor_sync(0xffffffffu, sl, o);
+            }
+            if (tig == 0) {
+                red[0][wcol][r] = sd;
+                red[1][wcol][r] = su;
+                red[2][wcol][r] = sl;
+            }
+        }
+    __syncthreads();
+    const int64_t tiles = (n + sliced::BN - 1) / sliced::BN;
+    for (int r = threadIdx.x; r < sliced::BM; r += blockDim.x) {
+        const int64_t i = i0 + r;
+        if (i >= n) continue;
+#pragma unroll
+        for (int t = 0; t < 3; ++t)
+            part[((int64_t)t * tiles + blockIdx.x) * n + i] = (red[t][0][r] + red[t][1][r]) + (red[t][2][r] + red[t][3][r]);
     }
 }
 
@@ -179,11 +291,40 @@ __global__ void adjoint_lambda_only_kernel(const double* __restrict__ Q, int64_t
 
 }  // namespace
 
+// From this order on the products run on the bf16 tensor cores; below it the padding to 128 x 128
+// tiles, the slicing and its launches cost more than the FP64 pipe takes.  One matrix, FP64 MMA against
+// sliced: n = 130 427 / 491 us, 160 470 / 486, 192 545 / 487, 256 700 / 557, 512 1314 / 880, 1024 4.78 / 1.54 ms,
+// 2047 32.8 / 5.5, 4096 252 / 35.  Batches: 64 of n = 100 611 / 631 us, 49 of 192 1441 / 1167,
+// 25 of 257 3226 / 1469.  The rule leaves the count out, so that a matrix has the same bits alone and
+// in a batch.
+static constexpr int64_t kSlicedMin = 192;
+// Matrices sliced at once: their planes take at most this many bytes (one matrix always fits).
+static constexpr int64_t kSlicedBytes = (int64_t)512 << 20;
+
+// Above it the rows leave the grid's y range (slice_columns_kernel).
+static constexpr int64_t kSlicedMax = 65408;
+
+bool adjoint_sliced(int64_t n) { return n >= kSlicedMin && n <= kSlicedMax; }
+
+static int64_t sliced_group(int64_t count, int64_t n)
+{
+    const int64_t per = 2 * 2 * sliced::plane_values(n, n);
+    return std::max<int64_t>(1, std::min<int64_t>(count, kSlicedBytes / per));
+}
+
+// The scratch after M and the partials: two operands' planes, their exponents, two flags a matrix.
+static int64_t sliced_scratch_doubles(int64_t count, int64_t n)
+{
+    const int64_t g = sliced_group(count, n);
+    return g * (2 * sliced::plane_values(n, n) * 2 + 2 * (n + 1) * (int64_t)sizeof(int)) / 8 + 64;
+}
+
 // Device-pointer adjoint for `count` matrices of order n stored back to back (Q, gQ with
 // leading dimension n and stride n*n; lam, glam, gd with stride n; ge with stride n-1).
-// scratch: count * (n*n + 3*ceil(n/64)*n) doubles.
+// scratch: adjoint_scratch_doubles(count, n, use_sliced) doubles; use_sliced only where adjoint_sliced(n).
 int adjoint_dev(cudaStream_t s, int64_t count, int64_t n, const double* lam, const double* Q,
-                const double* glam, const double* gQ, double* gd, double* ge, double* scratch)
+                const double* glam, const double* gQ, double* gd, double* ge, double* scratch,
+                bool use_sliced)
 {
     if (count <= 0 || n <= 0) return SYMEIG_OK;
     const int64_t tiles = (n + BN - 1) / BN;
@@ -197,16 +338,55 @@ int adjoint_dev(cudaStream_t s, int64_t count, int64_t n, const double* lam, con
     double* Mbuf = scratch;
     double* part = scratch + count * strideM;
     const dim3 grid((unsigned)tiles, (unsigned)((n + BM - 1) / BM), (unsigned)count);
-    adjoint_m_kernel<<<grid, kAdjThreads, 0, s>>>(Q, n, gQ, n, lam, glam, n, Mbuf, strideQ, strideQ, strideM);
-    adjoint_p_kernel<<<grid, kAdjThreads, 0, s>>>(Q, n, Mbuf, n, part, strideQ, strideM, stridePart);
-    adjoint_reduce_kernel<<<dim3((unsigned)((n + 255) / 256), (unsigned)count), 256, 0, s>>>(part, n, gd, ge, stridePart);
+    if (!use_sliced) {
+        adjoint_m_kernel<<<grid, kAdjThreads, 0, s>>>(Q, n, gQ, n, lam, glam, n, Mbuf, strideQ, strideQ, strideM, nullptr);
+        adjoint_p_kernel<<<grid, kAdjThreads, 0, s>>>(Q, n, Mbuf, n, part, strideQ, strideM, stridePart, nullptr);
+        adjoint_reduce_kernel<<<dim3((unsigned)((n + 255) / 256), (unsigned)count), 256, 0, s>>>(part, n, gd, ge, stridePart, nullptr);
+        return cudaGetLastError() == cudaSuccess ? SYMEIG_OK : SYMEIG_ERR_CUDA;
+    }
+    if (cudaFuncSetAttribute(sliced_m_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sliced::kSmem) != cudaSuccess ||
+        cudaFuncSetAttribute(sliced_p_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sliced::kSmem) != cudaSuccess)
+        return SYMEIG_ERR_CUDA;
+    const int64_t group = sliced_group(count, n), rows = sliced::pad_rows(n), kp = sliced::pad_k(n);
+    const int64_t pstride = sliced::plane_values(n, n);
+    // 256-byte aligned: the planes' 16-byte pieces
+    unsigned char* base = (unsigned char*)(((uintptr_t)(part + count * stridePart) + 255) & ~(uintptr_t)255);
+    __nv_bfloat16* PA = (__nv_bfloat16*)base;
+    __nv_bfloat16* PB = PA + group * pstride;
+    int* ea = (int*)(PB + group * pstride);
+    int* eb = ea + group * n;
+    int* flag = eb + group * n;
+    const int64_t ntiles = (n + sliced::BN - 1) / sliced::BN;
+    for (int64_t z = 0; z < count; z += group) {
+        const unsigned g = (unsigned)std::min<int64_t>(group, count - z);
+        const double *Qz = Q + z * strideQ, *Gz = gQ + z * strideQ, *lz = lam + z * n, *glz = glam + z * n;
+        double *Mz = Mbuf + z * strideM, *pz = part + z * stridePart;
+        double* gez = ge ? ge + z * (n - 1) : nullptr;
+        const dim3 fgrid(grid.x, grid.y, g), sgrid((unsigned)ntiles, (unsigned)ntiles, g);
+        const dim3 cgrid((unsigned)((kp / 8 + 255) / 256), (unsigned)rows, g);
+        if (cudaMemsetAsync(flag, 0, 2 * group * sizeof(int), s) != cudaSuccess) return SYMEIG_ERR_CUDA;
+        sliced::column_exponents_kernel<<<dim3((unsigned)n, g), 256, 0, s>>>(Qz, n, n, strideQ, ea, n, true, flag);
+        sliced::column_exponents_kernel<<<dim3((unsigned)n, g), 256, 0, s>>>(Gz, n, n, strideQ, eb, n, false, flag);
+        sliced::slice_columns_kernel<<<cgrid, 256, 0, s>>>(Qz, n, n, strideQ, ea, n, rows, kp, PA, pstride, flag);
+        sliced::slice_columns_kernel<<<cgrid, 256, 0, s>>>(Gz, n, n, strideQ, eb, n, rows, kp, PB, pstride, flag);
+        sliced_m_kernel<<<sgrid, sliced::kThreads, sliced::kSmem, s>>>(PA, PB, ea, eb, lz, glz, n, rows, kp, pstride, Mz, flag);
+        adjoint_m_kernel<<<fgrid, kAdjThreads, 0, s>>>(Qz, n, Gz, n, lz, glz, n, Mz, strideQ, strideQ, strideM, flag);
+        sliced::row_exponents_kernel<<<dim3((unsigned)((n + 31) / 32), g), 256, 0, s>>>(Qz, n, n, strideQ, ea, n, true, flag + group);
+        sliced::column_exponents_kernel<<<dim3((unsigned)n, g), 256, 0, s>>>(Mz, n, n, strideM, eb, n, false, flag + group);
+        sliced::slice_rows_kernel<<<dim3((unsigned)((kp + 63) / 64), (unsigned)((rows + 31) / 32), g), 256, 0, s>>>(
+            Qz, n, n, strideQ, ea, n, rows, kp, PA, pstride, flag + group);
+        sliced::slice_columns_kernel<<<cgrid, 256, 0, s>>>(Mz, n, n, strideM, eb, n, rows, kp, PB, pstride, flag + group);
+        sliced_p_kernel<<<sgrid, sliced::kThreads, sliced::kSmem, s>>>(PA, PB, ea, eb, Qz, n, rows, kp, pstride, pz, stridePart, flag + group);
+        adjoint_p_kernel<<<fgrid, kAdjThreads, 0, s>>>(Qz, n, Mz, n, pz, strideQ, strideM, stridePart, flag + group);
+        adjoint_reduce_kernel<<<dim3((unsigned)((n + 255) / 256), g), 256, 0, s>>>(pz, n, gd + z * n, gez, stridePart, flag + group);
+    }
     return cudaGetLastError() == cudaSuccess ? SYMEIG_OK : SYMEIG_ERR_CUDA;
 }
 
-int64_t adjoint_scratch_doubles(int64_t count, int64_t n)
+int64_t adjoint_scratch_doubles(int64_t count, int64_t n, bool use_sliced)
 {
     const int64_t tiles = (n + BN - 1) / BN;
-    return count * (n * n + 3 * tiles * n);
+    return count * (n * n + 3 * tiles * n) + (use_sliced ? sliced_scratch_doubles(count, n) : 0);
 }
 
 }  // namespace symeig

@@ -1026,9 +1026,19 @@ int symeig_eig_adjoint_f64_dev(symeig_handle h, int64_t count, int64_t n, const 
     if (count == 0 || n == 0) return SYMEIG_OK;
     if (!lam || !Q || !glam || !gd || (n > 1 && !ge)) return SYMEIG_ERR_NULL;
     begin_call(h);
-    if (gQ) CK(h->cs.ensure((size_t)adjoint_scratch_doubles(count, n) * sizeof(double)));
+    bool use_sliced = gQ && adjoint_sliced(n);
+    if (use_sliced) {
+        const cudaError_t e = h->cs.ensure((size_t)adjoint_scratch_doubles(count, n, true) * sizeof(double));
+        if (e == cudaErrorMemoryAllocation) {
+            (void)cudaGetLastError();   // no room for the planes: the FP64 MMA needs M alone
+            use_sliced = false;
+        } else {
+            CK(e);
+        }
+    }
+    if (gQ && !use_sliced) CK(h->cs.ensure((size_t)adjoint_scratch_doubles(count, n, false) * sizeof(double)));
     auto t0 = std::chrono::steady_clock::now();
-    rc = adjoint_dev(h->stream, count, n, lam, Q, glam, gQ, gd, ge, (double*)h->cs.ptr);
+    rc = adjoint_dev(h->stream, count, n, lam, Q, glam, gQ, gd, ge, (double*)h->cs.ptr, use_sliced);
     h->stats.total_ms =
         std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     return rc;
