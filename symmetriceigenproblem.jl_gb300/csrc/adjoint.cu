@@ -168,102 +168,98 @@ __global__ void adjoint_reduce_kernel(const double* __restrict__ part, int64_t n
 __global__ void __launch_bounds__(sliced::kThreads, 1)
 sliced_m_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B, const int* __restrict__ ea,
                 const int* __restrict__ eb, const double* __restrict__ lam, const double* __restrict__ glam, int64_t n,
-                int64_t rows, int64_t kp, int64_t pstride, double* __restrict__ Mout, const int* __restrict__ fallback)
+                int64_t rows, int64_t kp, int64_t pstride, double* __restrict__ Mout, double* __restrict__ park,
+                int* __restrict__ fallback)
 {
-    extern __shared__ __align__(128) unsigned char smem[];
-    if (fallback[blockIdx.z]) return;
+    extern __shared__ __align__(1024) unsigned char smem[];
     const int64_t z = blockIdx.z;
+    const bool skip = fallback[z] != 0;
+    if (__syncthreads_or(skip)) return;
     lam += z * n;
     glam += z * n;
     Mout += z * n * n;
+    park += ((z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * sliced::BM * sliced::BN;
     const int64_t i0 = (int64_t)blockIdx.y * sliced::BM, j0 = (int64_t)blockIdx.x * sliced::BN;
-    double acc[4][4][4];
-    sliced::tile_product(A + z * pstride, B + z * pstride, rows, kp, i0, j0, smem, acc);
+    double acc[64];
+    if (!sliced::tile_product(A + z * pstride, B + z * pstride, rows, kp, i0, j0, smem, park, acc)) {
+        if (threadIdx.x == 0) fallback[z] = 1;
+        return;
+    }
+    const int64_t i = i0 + sliced::tile_row();
+    if (threadIdx.x >= sliced::kEpiThreads || i >= n) return;
+    const int e = ea[z * n + i];
+    const double li = lam[i];
 #pragma unroll
-    for (int x = 0; x < 4; ++x)
-#pragma unroll
-        for (int h = 0; h < 4; h += 2) {
-            const int64_t i = i0 + sliced::tile_row(x, h);
-            if (i >= n) continue;
-            const int e = ea[z * n + i];
-            const double li = lam[i];
-#pragma unroll
-            for (int y = 0; y < 4; ++y)
-#pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    const int64_t j = j0 + sliced::tile_col(y, q);
-                    if (j >= n) continue;
-                    double v;
-                    if (i == j) {
-                        v = glam[i];
-                    } else {
-                        const double gap = lam[j] - li;
-                        v = gap != 0.0 ? scalbn(acc[x][y][h + q], e + eb[z * n + j]) / gap : 0.0;
-                    }
-                    Mout[i + j * n] = v;
-                }
+    for (int q = 0; q < 64; ++q) {
+        const int64_t j = j0 + sliced::tile_col() + q;
+        if (j >= n) continue;
+        double v;
+        if (i == j) {
+            v = glam[i];
+        } else {
+            const double gap = lam[j] - li;
+            v = gap != 0.0 ? scalbn(acc[q], e + eb[z * n + j]) / gap : 0.0;
         }
+        Mout[i + j * n] = v;
+    }
 }
 
 // 2. as adjoint_p_kernel.  A: planes of Q's rows with exponents ea; B: of M's columns with eb.
 __global__ void __launch_bounds__(sliced::kThreads, 1)
 sliced_p_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B, const int* __restrict__ ea,
                 const int* __restrict__ eb, const double* __restrict__ Q, int64_t n, int64_t rows, int64_t kp,
-                int64_t pstride, double* __restrict__ part, int64_t stridePart, const int* __restrict__ fallback)
+                int64_t pstride, double* __restrict__ part, int64_t stridePart, double* __restrict__ park,
+                int* __restrict__ fallback)
 {
-    extern __shared__ __align__(128) unsigned char smem[];
-    if (fallback[blockIdx.z]) return;
-    double(*red)[4][sliced::BM] = reinterpret_cast<double(*)[4][sliced::BM]>(smem);   // [3], in the ring
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ double red[3][2][sliced::BM];
     const int64_t z = blockIdx.z;
+    const bool skip = fallback[z] != 0;
+    if (__syncthreads_or(skip)) return;
     Q += z * n * n;
     part += z * stridePart;
+    park += ((z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * sliced::BM * sliced::BN;
     const int64_t i0 = (int64_t)blockIdx.y * sliced::BM, k0 = (int64_t)blockIdx.x * sliced::BN;
-    double acc[4][4][4];
-    sliced::tile_product(A + z * pstride, B + z * pstride, rows, kp, i0, k0, smem, acc);
-    const int tig = threadIdx.x & 3, wcol = (threadIdx.x >> 5) & 3;
+    double acc[64];
+    if (!sliced::tile_product(A + z * pstride, B + z * pstride, rows, kp, i0, k0, smem, park, acc)) {
+        if (threadIdx.x == 0) fallback[z] = 1;
+        return;
+    }
+    const int r = sliced::tile_row();
+    if (threadIdx.x < sliced::kEpiThreads) {
+        const int64_t i = i0 + r;
+        double sd = 0.0, su = 0.0, sl = 0.0;
+        if (i < n) {
+            const int e = ea[z * n + i];
+            // eight columns at a time: shorter sums round less
 #pragma unroll
-    for (int x = 0; x < 4; ++x)
+            for (int q0 = 0; q0 < 64; q0 += 8) {
+                double td = 0.0, tu = 0.0, tl = 0.0;
 #pragma unroll
-        for (int h = 0; h < 4; h += 2) {
-            const int r = sliced::tile_row(x, h);
-            const int64_t i = i0 + r;
-            double sd = 0.0, su = 0.0, sl = 0.0;
-            if (i < n) {
-                const int e = ea[z * n + i];
-#pragma unroll
-                for (int y = 0; y < 4; ++y)
-#pragma unroll
-                    for (int q = 0; q < 2; ++q) {
-                        const int64_t k = k0 + sliced::tile_col(y, q);
-                        if (k >= n) continue;
-                        const double p = scalbn(acc[x][y][h + q], e + eb[z * n + k]);
-                        sd = fma(p, Q[i + k * n], sd);
-                        if (i + 1 < n) su = fma(p, Q[i + 1 + k * n], su);
-                        if (i >= 1) sl = fma(p, Q[i - 1 + k * n], sl);
-                    }
-            }
-            // the 4 lanes of a group hold the same row: sum them
-#pragma unroll
-            for (int o = 1; o < 4; o <<= 1) {
-                sd += __shfl_xor_sync(0xffffffffu, sd, o);
-                su += __shfl_xor_sync(0xffffffffu, su, o);
-                sl += __shfl_xor_sync(0xffffffffu, sl, o);
-            }
-            if (tig == 0) {
-                red[0][wcol][r] = sd;
-                red[1][wcol][r] = su;
-                red[2][wcol][r] = sl;
+                for (int q = q0; q < q0 + 8; ++q) {
+                    const int64_t k = k0 + sliced::tile_col() + q;
+                    if (k >= n) continue;
+                    const double p = scalbn(acc[q], e + eb[z * n + k]);
+                    td = fma(p, Q[i + k * n], td);
+                    if (i + 1 < n) tu = fma(p, Q[i + 1 + k * n], tu);
+                    if (i >= 1) tl = fma(p, Q[i - 1 + k * n], tl);
+                }
+                sd += td;
+                su += tu;
+                sl += tl;
             }
         }
+        const int half = threadIdx.x >> 7;
+        red[0][half][r] = sd;
+        red[1][half][r] = su;
+        red[2][half][r] = sl;
+    }
     __syncthreads();
     const int64_t tiles = (n + sliced::BN - 1) / sliced::BN;
-    for (int r = threadIdx.x; r < sliced::BM; r += blockDim.x) {
-        const int64_t i = i0 + r;
-        if (i >= n) continue;
+    if (threadIdx.x < sliced::BM && i0 + r < n)
 #pragma unroll
         for (int t = 0; t < 3; ++t)
-            part[((int64_t)t * tiles + blockIdx.x) * n + i] = (red[t][0][r] + red[t][1][r]) + (red[t][2][r] + red[t][3][r]);
-    }
+            part[((int64_t)t * tiles + blockIdx.x) * n + i0 + r] = red[t][0][r] + red[t][1][r];
 }
 
 // Eigenvalue-only loss (gQ = 0): dd_i = sum_k glam_k Q_ik^2, de_i = 2 sum_k glam_k Q_ik Q_{i+1,k}.
@@ -292,12 +288,12 @@ __global__ void adjoint_lambda_only_kernel(const double* __restrict__ Q, int64_t
 }  // namespace
 
 // From this order on the products run on the bf16 tensor cores; below it the padding to 128 x 128
-// tiles, the slicing and its launches cost more than the FP64 pipe takes.  One matrix, FP64 MMA against
-// sliced: n = 130 427 / 491 us, 160 470 / 486, 192 545 / 487, 256 700 / 557, 512 1314 / 880, 1024 4.78 / 1.54 ms,
-// 2047 32.8 / 5.5, 4096 252 / 35.  Batches: 64 of n = 100 611 / 631 us, 49 of 192 1441 / 1167,
-// 25 of 257 3226 / 1469.  The rule leaves the count out, so that a matrix has the same bits alone and
-// in a batch.
-static constexpr int64_t kSlicedMin = 192;
+// tiles, the slicing and its launches cost more than the FP64 pipe takes.  FP64 MMA against sliced, one
+// matrix: n = 64 239 / 234 us, 96 312 / 257, 130 427 / 299, 256 700 / 328, 512 1314 / 428, 1024 4.78 / 0.67 ms,
+// 2047 32.8 / 2.05, 4096 252 / 10.9; batches: 64 of n = 64 235 / 436 us, of 80 462 / 468, of 96 538 / 500,
+// of 130 1769 / 878, 25 of 257 3226 / 958.  The rule leaves the count out, so that a matrix has the
+// same bits alone and in a batch.
+static constexpr int64_t kSlicedMin = 96;
 // Matrices sliced at once: their planes take at most this many bytes (one matrix always fits).
 static constexpr int64_t kSlicedBytes = (int64_t)512 << 20;
 
@@ -312,11 +308,12 @@ static int64_t sliced_group(int64_t count, int64_t n)
     return std::max<int64_t>(1, std::min<int64_t>(count, kSlicedBytes / per));
 }
 
-// The scratch after M and the partials: two operands' planes, their exponents, two flags a matrix.
+// The scratch after M and the partials: two operands' planes, the tiles' small sums, the operands' exponents, two
+// flags a matrix.
 static int64_t sliced_scratch_doubles(int64_t count, int64_t n)
 {
-    const int64_t g = sliced_group(count, n);
-    return g * (2 * sliced::plane_values(n, n) * 2 + 2 * (n + 1) * (int64_t)sizeof(int)) / 8 + 64;
+    const int64_t g = sliced_group(count, n), r = sliced::pad_rows(n);
+    return g * (2 * sliced::plane_values(n, n) * 2 + r * r * (int64_t)sizeof(double) + 2 * (n + 1) * (int64_t)sizeof(int)) / 8 + 64;
 }
 
 // Device-pointer adjoint for `count` matrices of order n stored back to back (Q, gQ with
@@ -353,7 +350,8 @@ int adjoint_dev(cudaStream_t s, int64_t count, int64_t n, const double* lam, con
     unsigned char* base = (unsigned char*)(((uintptr_t)(part + count * stridePart) + 255) & ~(uintptr_t)255);
     __nv_bfloat16* PA = (__nv_bfloat16*)base;
     __nv_bfloat16* PB = PA + group * pstride;
-    int* ea = (int*)(PB + group * pstride);
+    double* park = (double*)(PB + group * pstride);
+    int* ea = (int*)(park + group * rows * rows);
     int* eb = ea + group * n;
     int* flag = eb + group * n;
     const int64_t ntiles = (n + sliced::BN - 1) / sliced::BN;
@@ -369,14 +367,14 @@ int adjoint_dev(cudaStream_t s, int64_t count, int64_t n, const double* lam, con
         sliced::column_exponents_kernel<<<dim3((unsigned)n, g), 256, 0, s>>>(Gz, n, n, strideQ, eb, n, false, flag);
         sliced::slice_columns_kernel<<<cgrid, 256, 0, s>>>(Qz, n, n, strideQ, ea, n, rows, kp, PA, pstride, flag);
         sliced::slice_columns_kernel<<<cgrid, 256, 0, s>>>(Gz, n, n, strideQ, eb, n, rows, kp, PB, pstride, flag);
-        sliced_m_kernel<<<sgrid, sliced::kThreads, sliced::kSmem, s>>>(PA, PB, ea, eb, lz, glz, n, rows, kp, pstride, Mz, flag);
+        sliced_m_kernel<<<sgrid, sliced::kThreads, sliced::kSmem, s>>>(PA, PB, ea, eb, lz, glz, n, rows, kp, pstride, Mz, park, flag);
         adjoint_m_kernel<<<fgrid, kAdjThreads, 0, s>>>(Qz, n, Gz, n, lz, glz, n, Mz, strideQ, strideQ, strideM, flag);
         sliced::row_exponents_kernel<<<dim3((unsigned)((n + 31) / 32), g), 256, 0, s>>>(Qz, n, n, strideQ, ea, n, true, flag + group);
         sliced::column_exponents_kernel<<<dim3((unsigned)n, g), 256, 0, s>>>(Mz, n, n, strideM, eb, n, false, flag + group);
         sliced::slice_rows_kernel<<<dim3((unsigned)((kp + 63) / 64), (unsigned)((rows + 31) / 32), g), 256, 0, s>>>(
             Qz, n, n, strideQ, ea, n, rows, kp, PA, pstride, flag + group);
         sliced::slice_columns_kernel<<<cgrid, 256, 0, s>>>(Mz, n, n, strideM, eb, n, rows, kp, PB, pstride, flag + group);
-        sliced_p_kernel<<<sgrid, sliced::kThreads, sliced::kSmem, s>>>(PA, PB, ea, eb, Qz, n, rows, kp, pstride, pz, stridePart, flag + group);
+        sliced_p_kernel<<<sgrid, sliced::kThreads, sliced::kSmem, s>>>(PA, PB, ea, eb, Qz, n, rows, kp, pstride, pz, stridePart, park, flag + group);
         adjoint_p_kernel<<<fgrid, kAdjThreads, 0, s>>>(Qz, n, Mz, n, pz, strideQ, strideM, stridePart, flag + group);
         adjoint_reduce_kernel<<<dim3((unsigned)((n + 255) / 256), g), 256, 0, s>>>(pz, n, gd + z * n, gez, stridePart, flag + group);
     }

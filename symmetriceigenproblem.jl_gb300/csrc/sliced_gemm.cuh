@@ -22,11 +22,15 @@
 // kernels return at once for it and the caller's FP64 MMA kernels, launched behind them
 // with the opposite test, do the work.
 //
-// The product kernel: 128 x 128 tiles, 8 warps of 64 x 32 with mma.sync m16n8k16 (bf16, FP32 sums), operand
-// tiles of 64 of the inner dimension in a three-stage shared-memory ring by cp.async.  45 plane
-// products for S = 9: 352 TFLOP/s at n = 4096, bound by ldmatrix's shared-memory reads (98 KB a
-// step of 64 for 8 warps, 768 of about 1850 cycles) beside the MMAs (1024).  With 32-deep steps and
-// FP64 sums per chunk the two products of n = 2047 took 8.3 ms instead of 5.5.
+// The product kernel: 128 x 128 tiles by tcgen05.mma (bf16, FP32 sums in TMEM), one CTA per tile.  Operands lie
+// in memory as the tensor core wants them, 128 x 64 tiles of 16 KB with the 128-byte swizzle, so one
+// bulk copy brings each.  Four levels at a time have a 128-column accumulator each, so that a plane's
+// tile is read once for all of them, 37 bytes a clock and SM at the tensor core's rate (one product at a
+// time would take 128).  Two products at n = 2047 take 2.0 ms with everything (mma.sync with 128 x 128 tiles of
+// the same operands: 5.4), at n = 4096 10.9 ms, 1130 TFLOP/s in bf16 counted over the whole call.  At
+// n = 2047 256 tiles on 152 SMs are two waves, 84 % full; a tile's own time is the products (256 cycles
+// each, 1440 of them), the sums' way out of TMEM (18 times, between which the tensor core waits) and the
+// epilogue's FP64 division.
 #pragma once
 #include <cuda_bf16.h>
 #include <cstdint>
@@ -35,11 +39,14 @@ namespace symeig {
 namespace sliced {
 
 constexpr int S = 9;                      // digit planes
-constexpr int BM = 128, BN = 128, BK = 64, STAGES = 3, kThreads = 256;
-constexpr int kTileBytes = BM * BK * 2;   // one operand tile
-constexpr int kRing = STAGES * 2 * kTileBytes;
-constexpr int kSmem = kRing + BM * BN * (int)sizeof(double);   // and the small levels' sums
-constexpr int kSmallLevels = 5;                                // levels from this one on are small
+constexpr int BM = 128, BN = 128, BK = 64;
+constexpr int kTileValues = BM * BK, kTileBytes = kTileValues * 2;   // one operand tile
+constexpr int kSlots = 13;                                // operand tiles in shared memory
+constexpr int kSmem = kSlots * kTileBytes + 1024;         // the tiles on a 1 KB boundary
+constexpr int kEpiThreads = 256;                          // warps 0-7: TMEM -> integers -> result
+constexpr int kThreads = kEpiThreads + 64;                // warp 8 copies, warp 9 issues the MMAs
+constexpr int kSmallLevels = 5;                           // levels from this one on are small
+static_assert(BM == 128 && BN == 128, "a tile is one tcgen05 shape");
 
 inline int64_t pad_rows(int64_t n) { return (n + BM - 1) / BM * BM; }
 inline int64_t pad_k(int64_t n) { return (n + BK - 1) / BK * BK; }
@@ -161,8 +168,15 @@ row_exponents_kernel(const double* __restrict__ X, int64_t ld, int64_t n, int64_
     }
 }
 
-// Planes of the columns of X: plane s, column i, inner index k at planes[(s * rows + i) * kp + k]
-// (rows, kp padded; zeros outside).  One thread per 8 inner indices.
+// Where 8 inner indices from k0 on of row i of plane s lie: 128 x 64 tiles, 16-byte pieces of a row
+// rotated by the row (the 128-byte swizzle).
+__device__ __forceinline__ int64_t plane_offset(int s, int64_t i, int64_t k0, int64_t rows, int64_t kp)
+{
+    const int r = (int)(i & (BM - 1)), c = (int)(k0 & (BK - 1)) >> 3;
+    return ((s * (rows / BM) + i / BM) * (kp / BK) + k0 / BK) * kTileValues + r * BK + ((c ^ (r & 7)) << 3);
+}
+
+// Planes of the columns of X (rows, kp padded; zeros outside).  One thread per 8 inner indices.
 static __global__ void __launch_bounds__(256)
 slice_columns_kernel(const double* __restrict__ X, int64_t ld, int64_t n, int64_t stride, const int* __restrict__ exps,
                      int64_t estride, int64_t rows, int64_t kp, __nv_bfloat16* __restrict__ planes, int64_t pstride,
@@ -184,7 +198,7 @@ slice_columns_kernel(const double* __restrict__ X, int64_t ld, int64_t n, int64_
 #pragma unroll
         for (int s = 0; s < S; ++s) out[s][q] = pack(d0[s], d1[s]);
     }
-    __nv_bfloat16* p = planes + blockIdx.z * pstride + i * kp + k0;
+    __nv_bfloat16* p = planes + blockIdx.z * pstride + plane_offset(0, i, k0, rows, kp);
 #pragma unroll
     for (int s = 0; s < S; ++s)
         *reinterpret_cast<uint4*>(p + s * rows * kp) = make_uint4(out[s][0], out[s][1], out[s][2], out[s][3]);
@@ -219,7 +233,7 @@ slice_rows_kernel(const double* __restrict__ X, int64_t ld, int64_t n, int64_t s
 #pragma unroll
         for (int s = 0; s < S; ++s) out[s][q] = pack(d0[s], d1[s]);
     }
-    __nv_bfloat16* p = planes + blockIdx.z * pstride + i * kp + k0 + c;
+    __nv_bfloat16* p = planes + blockIdx.z * pstride + plane_offset(0, i, k0 + c, rows, kp);
 #pragma unroll
     for (int s = 0; s < S; ++s)
         *reinterpret_cast<uint4*>(p + s * rows * kp) = make_uint4(out[s][0], out[s][1], out[s][2], out[s][3]);
@@ -227,186 +241,301 @@ slice_rows_kernel(const double* __restrict__ X, int64_t ld, int64_t n, int64_t s
 
 // ---- the product ---------------------------------------------------------------------------
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src)
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void mbar_init(uint64_t* b, uint32_t count)
 {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(b)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* b)
+{
+    asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.shared::cta.b64 t, [%0];\n\t}" ::"r"(smem_addr(b)) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(uint64_t* b, uint32_t bytes)
+{
+    asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 t, [%0], %1;\n\t}" ::"r"(smem_addr(b)),
+                 "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool mbar_try(uint64_t* b, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(smem_addr(b)), "r"(parity) : "memory");
+    return ok != 0;
 }
 
-__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t addr)
-{
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
-}
-
-__device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
-{
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-                 "{%0, %1, %2, %3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-// Byte offset of the 16-byte piece c (0 .. 7) of row r in an operand tile: pieces rotated so that
-// the eight rows of an ldmatrix phase fall on different banks.
-__device__ __forceinline__ uint32_t piece(int r, int c) { return (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)); }
-
-// The schedule of plane products: levels S-1 .. 0, chunks of the inner dimension, pairs (s, l - s),
-// steps of BK.
-struct Schedule {
-    int l, s, ks, chunk0, chunk1, ksteps;
-    __device__ __forceinline__ int chunk_steps() const { return 2048 / BK / (l + 1); }
-    __device__ __forceinline__ void begin(int steps)
+// The levels lo .. hi are summed in one pass over the inner dimension.  For each 64 of it (a block)
+// and each plane s of A, in order, the tiles that come in and the products done are:
+//   s = 0: A_0, B_hi .. B_lo;  s >= 1: A_s, and B_(lo - s) while that exists
+//   A_s B_t for max(0, lo - s) <= t <= hi - s; then A_s and B_(hi - s) are done with
+// so each tile comes in once a block, and at most hi - lo + 3 of them are held.
+struct Pass {
+    int lo, hi;
+    __device__ __forceinline__ int loads() const { return 2 * (hi + 1); }
+    __device__ __forceinline__ int index_a(int s) const
     {
-        ksteps = steps;
-        l = S - 1;
-        s = 0;
-        chunk0 = ks = 0;
-        chunk1 = min(chunk_steps(), ksteps);
+        return s == 0 ? 0 : hi - lo + 2 + (s <= lo ? 2 * (s - 1) : lo + s - 1);
     }
-    __device__ __forceinline__ bool done() const { return l < 0; }
-    // the next step; true when it begins a new (level, chunk)
-    __device__ __forceinline__ bool next()
-    {
-        if (++ks < chunk1) return false;
-        ks = chunk0;
-        if (++s <= l) return false;
-        s = 0;
-        chunk0 = ks = chunk1;
-        if (chunk0 >= ksteps) {
-            chunk0 = ks = 0;
-            --l;
-            if (l < 0) return true;
-        }
-        chunk1 = min(chunk0 + chunk_steps(), ksteps);
-        return true;
-    }
+    __device__ __forceinline__ int index_b(int t) const { return t >= lo ? 1 + hi - t : hi - lo + 2 + 2 * (lo - t - 1) + 1; }
+    // blocks whose sums stay below 2^23: (hi + 1) 64 2^12 each
+    __device__ __forceinline__ int chunk_blocks() const { return 32 / (hi + 1); }
+};
+constexpr int kPasses = 3;
+__device__ __forceinline__ Pass pass_of(int p)
+{
+    return p == 0 ? Pass{kSmallLevels, S - 1} : p == 1 ? Pass{1, kSmallLevels - 1} : Pass{0, 0};
+}
+static_assert(S - kSmallLevels <= 4 && kSmallLevels - 1 <= 4, "four accumulators of 128 columns");
+
+struct Control {
+    uint64_t full[kSlots], empty[kSlots], sums_full, sums_empty, drained;
+    uint32_t tmem;
+    int failed;
 };
 
-// One 128 x 128 tile of sum_{s+t<S} 2^(-12-7(s+t)) A_s B_t^T (planes as slice_*_kernel lays them out).
-// acc[x][y][h]: this thread's elements, row 64 (warp >> 2) + 16 x + (lane >> 2) + 8 (h >> 1), column
-// 32 (warp & 3) + 8 y + 2 (lane & 3) + (h & 1) of the tile.
-__device__ __forceinline__ void tile_product(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B,
-                                             int64_t rows, int64_t kp, int64_t i0, int64_t j0, unsigned char* smem,
-                                             double (&out)[4][4][4])
+// Waits for the phase of `parity`, for about a second at most (failure: false, for every warp).
+__device__ __forceinline__ bool wait(Control& c, uint64_t* b, uint32_t parity)
 {
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int wm = (warp >> 2) * 64, wn = (warp & 3) * 32;
-    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
-    double* park = reinterpret_cast<double*>(smem + kRing) + tid;
-    float part[4][4][4];
-    long long acc[4][4][4];
-#pragma unroll
-    for (int x = 0; x < 4; ++x)
-#pragma unroll
-        for (int y = 0; y < 4; ++y)
-#pragma unroll
-            for (int h = 0; h < 4; ++h) {
-                acc[x][y][h] = 0;
-                part[x][y][h] = 0.0f;
-            }
-    const int ksteps = (int)(kp / BK);
-    // this thread's pieces of a tile: rows tid / 8 + 32 q
-    const int lr = tid >> 3, lc = tid & 7;
-    const uint32_t dst = piece(lr, lc);   // 32 rows further is 4096 bytes further
-    const __nv_bfloat16* a0 = A + (i0 + lr) * kp + lc * 8;
-    const __nv_bfloat16* b0 = B + (j0 + lr) * kp + lc * 8;
-    auto load = [&](const Schedule& q, int stage) {
-        const uint32_t sa = sbase + stage * 2 * kTileBytes + dst, sb = sa + kTileBytes;
-        const int64_t ko = (int64_t)q.ks * BK;
-        const __nv_bfloat16* a = a0 + q.s * rows * kp + ko;
-        const __nv_bfloat16* b = b0 + (q.l - q.s) * rows * kp + ko;
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            cp_async16(sa + 4096 * t, a + 32 * t * kp);
-            cp_async16(sb + 4096 * t, b + 32 * t * kp);
+    if (mbar_try(b, parity)) return true;
+    const long long t0 = clock64();
+    while (!mbar_try(b, parity)) {
+        if (*(volatile int*)&c.failed) return false;
+        if (clock64() - t0 > 2000000000ll) {
+            *(volatile int*)&c.failed = 1;
+            return false;
         }
-    };
-    Schedule cur, pre;
-    cur.begin(ksteps);
-    pre.begin(ksteps);
-#pragma unroll
-    for (int st = 0; st < STAGES - 1; ++st) {
-        if (!pre.done()) {
-            load(pre, st);
-            pre.next();
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    int stage = 0;
-    while (!cur.done()) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
-        __syncthreads();
-        {
-            const int ls = (stage + STAGES - 1) % STAGES;
-            if (!pre.done()) {
-                load(pre, ls);
-                pre.next();
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        }
-        const uint32_t sa = sbase + stage * 2 * kTileBytes, sb = sa + kTileBytes;
-#pragma unroll
-        for (int kk = 0; kk < BK / 16; ++kk) {
-            uint32_t bf[2][4];
-#pragma unroll
-            for (int y = 0; y < 2; ++y)   // columns 16 y .. 16 y + 15: matrices (n 0-7, k 0-7), (n 0-7, k 8-15), (n 8-15, ..)
-                ldmatrix4(bf[y], sb + piece(wn + 16 * y + (lane & 7) + ((lane >> 4) << 3), 2 * kk + ((lane >> 3) & 1)));
-#pragma unroll
-            for (int x = 0; x < 4; ++x) {
-                uint32_t af[4];
-                ldmatrix4(af, sa + piece(wm + 16 * x + (lane & 15), 2 * kk + (lane >> 4)));
-#pragma unroll
-                for (int y = 0; y < 4; ++y) mma(part[x][y], af, bf[y >> 1][2 * (y & 1)], bf[y >> 1][2 * (y & 1) + 1]);
-            }
-        }
-        const int l = cur.l;
-        if (cur.next()) {
-            // the level's chunk is complete: into the integers
-            const int w = 1 << 7 * (l >= kSmallLevels ? S - 1 - l : kSmallLevels - 1 - l);
-#pragma unroll
-            for (int x = 0; x < 4; ++x)
-#pragma unroll
-                for (int y = 0; y < 4; ++y)
-#pragma unroll
-                    for (int h = 0; h < 4; ++h) {
-                        acc[x][y][h] += (long long)__float2int_rn(part[x][y][h]) * w;
-                        part[x][y][h] = 0.0f;
-                    }
-            if (l == kSmallLevels && cur.l < l) {
-#pragma unroll
-                for (int x = 0; x < 4; ++x)
-#pragma unroll
-                    for (int y = 0; y < 4; ++y)
-#pragma unroll
-                        for (int h = 0; h < 4; ++h) {
-                            park[(16 * x + 4 * y + h) * kThreads] = __ll2double_rn(acc[x][y][h]);
-                            acc[x][y][h] = 0;
-                        }
-            }
-        }
-        stage = (stage + 1) % STAGES;
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();   // the ring is free for the caller
-    constexpr double kSmall = 1.0 / (1ull << (12 + 7 * (S - 1) - 28)) / (1ull << 28);
-    constexpr double kLarge = 1.0 / (1ull << (12 + 7 * (kSmallLevels - 1)));
-#pragma unroll
-    for (int x = 0; x < 4; ++x)
-#pragma unroll
-        for (int y = 0; y < 4; ++y)
-#pragma unroll
-            for (int h = 0; h < 4; ++h)
-                out[x][y][h] = fma(__ll2double_rn(acc[x][y][h]), kLarge, park[(16 * x + 4 * y + h) * kThreads] * kSmall);
+    return true;
 }
 
-__device__ __forceinline__ int tile_row(int x, int h)
+// A K-major operand tile with the 128-byte swizzle: 8 rows are 1024 bytes.
+__device__ __forceinline__ uint64_t operand_desc(uint32_t addr)
 {
-    return ((int)threadIdx.x >> 7) * 64 + 16 * x + (((int)threadIdx.x & 31) >> 2) + 8 * (h >> 1);
+    return (uint64_t)((addr & 0x3FFFF) >> 4) | (uint64_t)1 << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 |
+           (uint64_t)2 << 61;
 }
-__device__ __forceinline__ int tile_col(int y, int h)
+
+// The copying thread: all tiles of the passes, in order.  Returns once what it started has landed.
+__device__ __forceinline__ void copy_tiles(Control& c, uint32_t tiles, const __nv_bfloat16* A, const __nv_bfloat16* B,
+                                           int64_t plane, int blocks)
 {
-    return (((int)threadIdx.x >> 5) & 3) * 32 + 8 * y + 2 * ((int)threadIdx.x & 3) + (h & 1);
+    uint32_t g = 0;
+    bool ok = true;
+    auto load = [&](const __nv_bfloat16* src) {
+        const uint32_t slot = g % kSlots, turn = g / kSlots;
+        if (turn > 0) ok = wait(c, &c.empty[slot], (turn - 1) & 1);
+        if (!ok) return;
+        mbar_expect(&c.full[slot], kTileBytes);
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                         tiles + slot * kTileBytes),
+                     "l"(src), "r"(kTileBytes), "r"(smem_addr(&c.full[slot])) : "memory");
+        ++g;
+    };
+    for (int p = 0; p < kPasses && ok; ++p) {
+        const Pass q = pass_of(p);
+        for (int kb = 0; kb < blocks && ok; ++kb) {
+            const int64_t o = (int64_t)kb * kTileValues;
+            for (int s = 0; s <= q.hi && ok; ++s) {
+                load(A + s * plane + o);
+                if (s == 0) {
+                    for (int t = q.hi; t >= q.lo && ok; --t) load(B + t * plane + o);
+                } else if (q.lo - s >= 0 && ok) {
+                    load(B + (q.lo - s) * plane + o);
+                }
+            }
+        }
+    }
+    // the last tile of each slot (on failure too: none may land after the block has gone)
+    for (uint32_t k = 0; k < kSlots && k < g; ++k) {
+        const uint32_t last = g - 1 - k;
+        const long long t0 = clock64();
+        while (!mbar_try(&c.full[last % kSlots], (last / kSlots) & 1))
+            if (clock64() - t0 > 2000000000ll) break;
+    }
 }
+
+// The issuing thread, a pass unrolled: what it computes per product has to stay below the 256 cycles
+// that the tensor core takes for it.  (With the loops rolled and a wait per operand a product took 640.)
+__device__ __forceinline__ void commit(uint64_t* b)
+{
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(b)) : "memory");
+}
+
+struct Ring {
+    uint32_t slot, turn;   // of the block's first tile
+    __device__ __forceinline__ Ring at(uint32_t index) const
+    {
+        Ring r{slot + index, turn};
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+            if (r.slot >= kSlots) {
+                r.slot -= kSlots;
+                ++r.turn;
+            }
+        return r;
+    }
+};
+static_assert(2 * S + kSlots - 1 < 3 * kSlots, "two wraps");
+
+template <int LO, int HI>
+__device__ __forceinline__ bool issue_pass(Control& c, uint64_t desc0, uint32_t tmem, int blocks, Ring& ring, uint32_t& chunk)
+{
+    constexpr uint32_t idesc = 1u << 4 | 1u << 7 | 1u << 10 | (uint32_t)(BN >> 3) << 17 | (uint32_t)(BM >> 4) << 24;
+    const Pass q{LO, HI};
+    const int step = q.chunk_blocks();
+    for (int k0 = 0; k0 < blocks; k0 += step, ++chunk) {
+        if (chunk > 0 && !wait(c, &c.sums_empty, (chunk - 1) & 1)) return false;
+        const int k1 = min(k0 + step, blocks);
+        for (int kb = k0; kb < k1; ++kb, ring = ring.at(q.loads())) {
+#pragma unroll
+            for (int s = 0; s <= HI; ++s) {
+                const Ring ra = ring.at(q.index_a(s));
+                bool ok = wait(c, &c.full[ra.slot], ra.turn & 1);
+#pragma unroll
+                for (int t = HI; t >= 0; --t)   // the tiles of B that came in with A_s
+                    if (s == 0 ? t >= LO : t == LO - s) {
+                        const Ring rb = ring.at(q.index_b(t));
+                        ok = ok && wait(c, &c.full[rb.slot], rb.turn & 1);
+                    }
+                if (!ok) return false;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t da = desc0 + ra.slot * (kTileBytes >> 4);
+#pragma unroll
+                for (int t = HI - s; t >= (s < LO ? LO - s : 0); --t) {
+                    const uint64_t db = desc0 + ring.at(q.index_b(t)).slot * (kTileBytes >> 4);
+                    const uint32_t d = tmem + (uint32_t)(s + t - LO) * BN;
+#pragma unroll
+                    for (int kk = 0; kk < BK / 16; ++kk) {
+                        const uint32_t add = s > 0 || kk > 0 || kb > k0;
+                        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                                     "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+                                     "l"(da + 2 * kk), "l"(db + 2 * kk), "r"(idesc), "r"(add) : "memory");
+                    }
+                }
+                commit(&c.empty[ra.slot]);
+                commit(&c.empty[ring.at(q.index_b(HI - s)).slot]);
+            }
+        }
+        commit(&c.sums_full);
+    }
+    return true;
+}
+
+__device__ __forceinline__ void issue_products(Control& c, uint32_t tiles, uint32_t tmem, int blocks)
+{
+    Ring ring{0, 0};
+    uint32_t chunk = 0;
+    const uint64_t desc0 = operand_desc(tiles);
+    if (issue_pass<kSmallLevels, S - 1>(c, desc0, tmem, blocks, ring, chunk) &&
+        issue_pass<1, kSmallLevels - 1>(c, desc0, tmem, blocks, ring, chunk))
+        issue_pass<0, 0>(c, desc0, tmem, blocks, ring, chunk);
+    // nothing may be in flight when the accumulators are given back
+    commit(&c.drained);
+    const long long t0 = clock64();
+    while (!mbar_try(&c.drained, 0))
+        if (clock64() - t0 > 2000000000ll) break;
+}
+
+// One 128 x 128 tile of sum_{s+t<S} 2^(-12-7(s+t)) A_s B_t^T, rows i0 .. of A's planes by rows j0 .. of B's.
+// Thread t < kEpiThreads gets row tile_row(), columns tile_col() .. + 63.  park: 128 KB of memory for this
+// tile.  False, for all threads, if a wait ran out; call it with all kThreads.
+__device__ __forceinline__ bool tile_product(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B,
+                                             int64_t rows, int64_t kp, int64_t i0, int64_t j0, unsigned char* smem,
+                                             double* __restrict__ park, double (&out)[64])
+{
+    __shared__ Control c;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t tiles = (smem_addr(smem) + 1023) & ~1023u;
+    const int blocks = (int)(kp / BK);
+    const int64_t plane = rows * kp;
+    if (warp == 9) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_addr(&c.tmem)) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 0) {
+        for (int k = 0; k < kSlots; ++k) {
+            mbar_init(&c.full[k], 1);
+            mbar_init(&c.empty[k], 1);
+        }
+        mbar_init(&c.sums_full, 1);
+        mbar_init(&c.drained, 1);
+        mbar_init(&c.sums_empty, kEpiThreads / 32);
+        c.failed = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = c.tmem;
+    if (warp == 8) {
+        if (lane == 0)
+            copy_tiles(c, tiles, A + i0 / BM * (kp / BK) * kTileValues, B + j0 / BN * (kp / BK) * kTileValues, plane, blocks);
+        __syncwarp();
+    } else if (warp == 9) {
+        if (lane == 0) issue_products(c, tiles, tmem, blocks);
+        __syncwarp();
+    } else {
+        long long acc[64];
+#pragma unroll
+        for (int q = 0; q < 64; ++q) acc[q] = 0;
+        const uint32_t mine = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 64 * (warp >> 2);
+        uint32_t chunk = 0;
+        bool ok = true;
+        for (int p = 0; p < kPasses && ok; ++p) {
+            const Pass q = pass_of(p);
+            const int step = q.chunk_blocks(), top = p == 0 ? S - 1 : kSmallLevels - 1;
+            for (int k0 = 0; k0 < blocks; k0 += step, ++chunk) {
+                ok = __all_sync(0xffffffffu, wait(c, &c.sums_full, chunk & 1));
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (int l = q.lo; l <= q.hi; ++l) {
+                    const int w = 1 << 7 * (top - l);
+#pragma unroll
+                    for (int h = 0; h < 4; ++h) {
+                        uint32_t v[16];
+                        // one statement, so that no use of v moves above the wait
+                        asm volatile(
+                            "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
+                            "tcgen05.wait::ld.sync.aligned;"
+                            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                              "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
+                              "=r"(v[15])
+                            : "r"(mine + (uint32_t)(l - q.lo) * BN + 16 * h) : "memory");
+#pragma unroll
+                        for (int e = 0; e < 16; ++e)
+                            acc[16 * h + e] += (long long)__float2int_rn(__uint_as_float(v[e])) * w;
+                    }
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&c.sums_empty);
+            }
+            if (p == 0) {
+#pragma unroll
+                for (int q2 = 0; q2 < 64; ++q2) {
+                    park[q2 * kEpiThreads + tid] = __ll2double_rn(acc[q2]);
+                    acc[q2] = 0;
+                }
+            }
+        }
+        constexpr double kSmall = 1.0 / (1ull << (12 + 7 * (S - 1) - 28)) / (1ull << 28);
+        constexpr double kLarge = 1.0 / (1ull << (12 + 7 * (kSmallLevels - 1)));
+#pragma unroll
+        for (int q = 0; q < 64; ++q)
+            out[q] = fma(__ll2double_rn(acc[q]), kLarge, park[q * kEpiThreads + tid] * kSmall);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 9) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+    }
+    return !*(volatile int*)&c.failed;
+}
+
+__device__ __forceinline__ int tile_row() { return (int)threadIdx.x & 127; }
+__device__ __forceinline__ int tile_col() { return ((int)threadIdx.x >> 7) * 64; }
 
 }  // namespace sliced
 }  // namespace symeig

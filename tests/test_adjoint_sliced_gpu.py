@@ -1,4 +1,4 @@
-"""The adjoint's products by bf16 slices (orders from 192): edges of the 128-wide tiles and of the
+"""The adjoint's products by bf16 slices (orders from 96): edges of the 128-wide tiles and of the
 64-deep steps, batches beside single matrices, operands that fall back to the FP64 MMA.
 
 Tolerance: with u = 2^-53 a length-n FP64 product x.y is off by at most n u |x| |y| (2-norms) in either
@@ -53,7 +53,7 @@ def run(torch, pkg, lam, Q, glam, gQ):
     return gd.cpu().numpy(), ge.cpu().numpy()
 
 
-@pytest.mark.parametrize("n,kind", [(191, "plain"), (192, "plain"), (255, "plain"), (256, "plain"), (257, "plain"), (287, "graded"),
+@pytest.mark.parametrize("n,kind", [(95, "plain"), (96, "plain"), (128, "graded"), (129, "plain"), (191, "plain"), (192, "plain"), (255, "plain"), (256, "plain"), (257, "plain"), (287, "graded"),
                                     (289, "plain"), (320, "localized"), (321, "graded"),
                                     (384, "plain"), (385, "localized"), (511, "graded")])
 def test_sliced_adjoint(cuda, pkg, n, kind):
@@ -65,6 +65,25 @@ def test_sliced_adjoint(cuda, pkg, n, kind):
     # the gradient is linear: exact under a power of two
     sd, se = run(cuda, pkg, lam, Q, glam * 2.0 ** 300, gQ * 2.0 ** 300)
     assert np.array_equal(sd, gd * 2.0 ** 300) and np.array_equal(se, ge * 2.0 ** 300)
+
+
+@pytest.mark.parametrize("n,bits,signed", [(200, 9, True), (513, 8, True), (1100, 6, True), (700, 4, False)])
+def test_sliced_adjoint_integers(cuda, pkg, n, bits, signed):
+    """Integer Q and gQ with gaps of 0 and +-1: every product and sum is an integer below 2^53, so the
+    gradient is exact, whatever the order of its sums."""
+    rng = np.random.default_rng(n)
+    top = 2 ** bits
+    ints = lambda: rng.integers(-top + 1 if signed else 1, top, (n, n))  # noqa: E731
+    Q, gQ, glam = ints(), ints(), rng.integers(-9, 10, n)
+    lam = (rng.random(n) < 0.5).astype(np.int64)
+    M = (Q.T @ gQ) * (lam[None, :] - lam[:, None])
+    np.fill_diagonal(M, glam)
+    P = Q @ M
+    assert (np.abs(P) @ np.abs(Q).max(axis=0)).max() < 2 ** 52
+    f = lambda x: x.astype(np.float64)  # noqa: E731
+    gd, ge = run(cuda, pkg, f(lam), f(Q), f(glam), f(gQ))
+    assert np.array_equal(gd, (P * Q).sum(1))
+    assert np.array_equal(ge, (P[:-1] * Q[1:]).sum(1) + (P[1:] * Q[:-1]).sum(1))
 
 
 def test_sliced_adjoint_batch(cuda, pkg):
