@@ -287,13 +287,13 @@ __global__ void adjoint_lambda_only_kernel(const double* __restrict__ Q, int64_t
 
 }  // namespace
 
-// From this order on the products run on the bf16 tensor cores; below it the padding to 128 x 128
-// tiles, the slicing and its launches cost more than the FP64 pipe takes.  FP64 MMA against sliced, one
-// matrix: n = 64 239 / 234 us, 96 312 / 257, 130 427 / 299, 256 700 / 328, 512 1314 / 428, 1024 4.78 / 0.67 ms,
-// 2047 32.8 / 2.05, 4096 252 / 10.9; batches: 64 of n = 64 235 / 436 us, of 80 462 / 468, of 96 538 / 500,
-// of 130 1769 / 878, 25 of 257 3226 / 958.  The rule leaves the count out, so that a matrix has the
-// same bits alone and in a batch.
-static constexpr int64_t kSlicedMin = 96;
+// From this order on the products run on the bf16 tensor cores where Q is spread out.  FP64 MMA against
+// sliced, one matrix: n = 130 427 / 308 us, 256 700 / 336, 512 1314 / 430, 1024 4.78 / 0.66 ms, 2047 32.8 / 2.0,
+// 4096 252 / 10.8; 25 of n = 257 3226 / 957 us, 4 of 700 6590 / 692.  A localized Q pays for the question and the kernels
+// that return at once: 45 us of 810 at n = 300, 60 of 4700 at 1000, 100 us of 32.8 ms at 2047; below
+// n = 256 it would be above 6 %.  The rule leaves the count out, so that a matrix has the same bits
+// alone and in a batch.
+static constexpr int64_t kSlicedMin = 256;
 // Matrices sliced at once: their planes take at most this many bytes (one matrix always fits).
 static constexpr int64_t kSlicedBytes = (int64_t)512 << 20;
 
@@ -302,18 +302,19 @@ static constexpr int64_t kSlicedMax = 65408;
 
 bool adjoint_sliced(int64_t n) { return n >= kSlicedMin && n <= kSlicedMax; }
 
+// (and 32767 at most: blockIdx.z counts two operands)
 static int64_t sliced_group(int64_t count, int64_t n)
 {
     const int64_t per = 2 * 2 * sliced::plane_values(n, n);
-    return std::max<int64_t>(1, std::min<int64_t>(count, kSlicedBytes / per));
+    return std::max<int64_t>(1, std::min(std::min<int64_t>(count, 32767), kSlicedBytes / per));
 }
 
-// The scratch after M and the partials: two operands' planes, the tiles' small sums, the operands' exponents, two
-// flags a matrix.
+// The scratch after M and the partials: two operands' planes, the tiles' small sums, the operands' exponents, a
+// flag a matrix.
 static int64_t sliced_scratch_doubles(int64_t count, int64_t n)
 {
     const int64_t g = sliced_group(count, n), r = sliced::pad_rows(n);
-    return g * (2 * sliced::plane_values(n, n) * 2 + r * r * (int64_t)sizeof(double) + 2 * (n + 1) * (int64_t)sizeof(int)) / 8 + 64;
+    return g * (2 * sliced::plane_values(n, n) * 2 + r * r * (int64_t)sizeof(double) + (2 * n + 1) * (int64_t)sizeof(int)) / 8 + 64;
 }
 
 // Device-pointer adjoint for `count` matrices of order n stored back to back (Q, gQ with
@@ -362,21 +363,20 @@ int adjoint_dev(cudaStream_t s, int64_t count, int64_t n, const double* lam, con
         double* gez = ge ? ge + z * (n - 1) : nullptr;
         const dim3 fgrid(grid.x, grid.y, g), sgrid((unsigned)ntiles, (unsigned)ntiles, g);
         const dim3 cgrid((unsigned)((kp / 8 + 255) / 256), (unsigned)rows, g);
-        if (cudaMemsetAsync(flag, 0, 2 * group * sizeof(int), s) != cudaSuccess) return SYMEIG_ERR_CUDA;
-        sliced::column_exponents_kernel<<<dim3((unsigned)n, g), 256, 0, s>>>(Qz, n, n, strideQ, ea, n, true, flag);
-        sliced::column_exponents_kernel<<<dim3((unsigned)n, g), 256, 0, s>>>(Gz, n, n, strideQ, eb, n, false, flag);
-        sliced::slice_columns_kernel<<<cgrid, 256, 0, s>>>(Qz, n, n, strideQ, ea, n, rows, kp, PA, pstride, flag);
-        sliced::slice_columns_kernel<<<cgrid, 256, 0, s>>>(Gz, n, n, strideQ, eb, n, rows, kp, PB, pstride, flag);
+        const sliced::Operand oq{Qz, ea, PA, true}, og{Gz, eb, PB, false}, om{Mz, eb, PB, false};
+        if (cudaMemsetAsync(flag, 0, group * sizeof(int), s) != cudaSuccess) return SYMEIG_ERR_CUDA;
+        sliced::column_exponents_kernel<<<dim3((unsigned)n, g, 2), 256, 0, s>>>(oq, og, n, flag);
+        sliced::slice_columns_kernel<<<dim3(cgrid.x, cgrid.y, 2 * g), 256, 0, s>>>(oq, og, (int)g, n, rows, kp, pstride, flag);
         sliced_m_kernel<<<sgrid, sliced::kThreads, sliced::kSmem, s>>>(PA, PB, ea, eb, lz, glz, n, rows, kp, pstride, Mz, park, flag);
         adjoint_m_kernel<<<fgrid, kAdjThreads, 0, s>>>(Qz, n, Gz, n, lz, glz, n, Mz, strideQ, strideQ, strideM, flag);
-        sliced::row_exponents_kernel<<<dim3((unsigned)((n + 31) / 32), g), 256, 0, s>>>(Qz, n, n, strideQ, ea, n, true, flag + group);
-        sliced::column_exponents_kernel<<<dim3((unsigned)n, g), 256, 0, s>>>(Mz, n, n, strideM, eb, n, false, flag + group);
+        sliced::row_exponents_kernel<<<dim3((unsigned)((n + 31) / 32), g), 1024, 0, s>>>(Qz, n, ea, flag);
+        sliced::column_exponents_kernel<<<dim3((unsigned)n, g, 1), 256, 0, s>>>(om, om, n, flag);
         sliced::slice_rows_kernel<<<dim3((unsigned)((kp + 63) / 64), (unsigned)((rows + 31) / 32), g), 256, 0, s>>>(
-            Qz, n, n, strideQ, ea, n, rows, kp, PA, pstride, flag + group);
-        sliced::slice_columns_kernel<<<cgrid, 256, 0, s>>>(Mz, n, n, strideM, eb, n, rows, kp, PB, pstride, flag + group);
-        sliced_p_kernel<<<sgrid, sliced::kThreads, sliced::kSmem, s>>>(PA, PB, ea, eb, Qz, n, rows, kp, pstride, pz, stridePart, park, flag + group);
-        adjoint_p_kernel<<<fgrid, kAdjThreads, 0, s>>>(Qz, n, Mz, n, pz, strideQ, strideM, stridePart, flag + group);
-        adjoint_reduce_kernel<<<dim3((unsigned)((n + 255) / 256), g), 256, 0, s>>>(pz, n, gd + z * n, gez, stridePart, flag + group);
+            Qz, n, ea, rows, kp, PA, pstride, flag);
+        sliced::slice_columns_kernel<<<cgrid, 256, 0, s>>>(om, om, (int)g, n, rows, kp, pstride, flag);
+        sliced_p_kernel<<<sgrid, sliced::kThreads, sliced::kSmem, s>>>(PA, PB, ea, eb, Qz, n, rows, kp, pstride, pz, stridePart, park, flag);
+        adjoint_p_kernel<<<fgrid, kAdjThreads, 0, s>>>(Qz, n, Mz, n, pz, strideQ, strideM, stridePart, flag);
+        adjoint_reduce_kernel<<<dim3((unsigned)((n + 255) / 256), g), 256, 0, s>>>(pz, n, gd + z * n, gez, stridePart, flag);
     }
     return cudaGetLastError() == cudaSuccess ? SYMEIG_OK : SYMEIG_ERR_CUDA;
 }

@@ -13,11 +13,11 @@
 //     thread at the FP64 pipe's two lanes a clock, 16k cycles; as integers it is 512.)
 // What is dropped (digits past 2^-63, levels past S - 1) is 2^-63 of the row's maximum times the
 // column's for each term, where FP64 rounds each by 2^-53 of its own size.  That is the smaller of the two
-// while one operand's rows are spread out, their maximum no more than some hundred times a typical
-// entry; the caller's other operand may be anything.  The exponent kernels check it for the operand that
-// is asked to be (kMaxOverRms).  Measured against longer
-// arithmetic, gradients of Toeplitz eigenvectors n = 257 .. 2047: 1.4e-16 .. 2.3e-16 of their norm, FP64 MMA
-// 6.0e-16 .. 1.9e-15; Gaussian orthogonal Q, n = 600: 1.6e-16 against 1.9e-15.
+// while one operand is spread out (kMaxOverRms, checked by the exponent kernels), so that a large entry of the
+// other meets an entry of ordinary size.  Measured against longer arithmetic, gradients of Toeplitz
+// eigenvectors n = 257 .. 2047: 1.4e-16 .. 2.3e-16 of their norm, FP64 MMA 6.0e-16 .. 1.9e-15; Gaussian orthogonal Q,
+// n = 600: 1.7e-16 against 1.9e-15.  Localized eigenvectors with close eigenvalues (random diagonal, n = 1000)
+// would give 2.6e-15 against 2.6e-16: they stay with the FP64 MMA.
 // A localized operand, an infinity or a NaN sets the matrix's flag word: the sliced
 // kernels return at once for it and the caller's FP64 MMA kernels, launched behind them
 // with the opposite test, do the work.
@@ -92,22 +92,32 @@ __device__ __forceinline__ uint32_t pack(int lo, int hi)
 }
 
 // `spread` operands: n max^2 <= kMaxOverRms^2 sum x^2 per row or column (entries of an eigenvector of
-// a Toeplitz matrix reach 1.4 times their rms, Gaussian ones 4 to 5, a localized one's sqrt(n)).
-// Where the squares leave the FP64 range the answer is no.
-constexpr double kMaxOverRms = 16.0;
+// a Toeplitz matrix reach 1.4 times their rms, Gaussian ones 4 to 5, a localized one's about sqrt(n), 16 for
+// the smallest order).  Where the squares leave the FP64 range the answer is no.
+constexpr double kMaxOverRms = 6.0;
 __device__ __forceinline__ bool spread(double mx, double sum, int64_t n)
 {
     return mx == 0.0 || (mx > 1e-140 && mx < 1e140 && mx * mx * (double)n <= kMaxOverRms * kMaxOverRms * sum);
 }
 
-// exps[i] of the columns of X (n x cols, leading dimension ld): one block per column.
+// Two operands of one launch (blockIdx.z, or its part beyond the matrices, picks one): a launch saved
+// where Q is localized and the FP64 MMA does the work after all.
+struct Operand {
+    const double* x;
+    int* exps;
+    __nv_bfloat16* planes;
+    bool must_spread;
+};
+
+// exps[i] of the columns of X (n x n): one block per column, blockIdx.y = matrix.
 static __global__ void __launch_bounds__(256)
-column_exponents_kernel(const double* __restrict__ X, int64_t ld, int64_t n, int64_t stride, int* __restrict__ exps,
-                        int64_t estride, bool must_spread, int* __restrict__ flag)
+column_exponents_kernel(Operand o0, Operand o1, int64_t n, int* __restrict__ flag)
 {
+    if (__syncthreads_or(flag[blockIdx.y])) return;
     __shared__ unsigned long long sh[8];
     __shared__ double ss[8];
-    const double* x = X + blockIdx.y * stride + (int64_t)blockIdx.x * ld;
+    const Operand& o = blockIdx.z == 0 ? o0 : o1;
+    const double* x = o.x + (blockIdx.y * n + blockIdx.x) * n;
     unsigned long long m = 0;
     double sum = 0.0;
     for (int64_t k = threadIdx.x; k < n; k += blockDim.x) {
@@ -116,9 +126,9 @@ column_exponents_kernel(const double* __restrict__ X, int64_t ld, int64_t n, int
         sum = fma(v, v, sum);
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-        sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    for (int d = 16; d > 0; d >>= 1) {
+        m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
+        sum += __shfl_xor_sync(0xffffffffu, sum, d);
     }
     if ((threadIdx.x & 31) == 0) {
         sh[threadIdx.x >> 5] = m;
@@ -131,40 +141,45 @@ column_exponents_kernel(const double* __restrict__ X, int64_t ld, int64_t n, int
             sum += ss[w];
         }
         const int e = magnitude_exponent(m);
-        exps[blockIdx.y * estride + blockIdx.x] = e;
-        if (e == kNoScale || (must_spread && !spread(__longlong_as_double((long long)m), sum, n))) flag[blockIdx.y] = 1;
+        o.exps[blockIdx.y * n + blockIdx.x] = e;
+        if (e == kNoScale || (o.must_spread && !spread(__longlong_as_double((long long)m), sum, n))) flag[blockIdx.y] = 1;
     }
 }
 
-// exps[i] of the rows of X (n x n): 32 rows per block.
-static __global__ void __launch_bounds__(256)
-row_exponents_kernel(const double* __restrict__ X, int64_t ld, int64_t n, int64_t stride, int* __restrict__ exps,
-                     int64_t estride, bool must_spread, int* __restrict__ flag)
+// exps[i] of the rows of X (n x n), which must spread: 32 rows per block, its 32 warps take every 32nd column.
+static __global__ void __launch_bounds__(1024)
+row_exponents_kernel(const double* __restrict__ X, int64_t n, int* __restrict__ exps, int* __restrict__ flag)
 {
-    __shared__ unsigned long long sh[8][32];
-    __shared__ double ss[8][32];
+    if (__syncthreads_or(flag[blockIdx.y])) return;
+    __shared__ unsigned long long sh[32][33];
+    __shared__ double ss[32][33];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t i = (int64_t)blockIdx.x * 32 + lane;
-    const double* x = X + blockIdx.y * stride;
+    const double* x = X + blockIdx.y * n * n;
     unsigned long long m = 0;
     double sum = 0.0;
     if (i < n)
-        for (int64_t k = w; k < n; k += 8) {
-            const double v = x[i + k * ld];
+        for (int64_t k = w; k < n; k += 32) {
+            const double v = x[i + k * n];
             m = max(m, (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull);
             sum = fma(v, v, sum);
         }
     sh[w][lane] = m;
     ss[w][lane] = sum;
     __syncthreads();
-    if (w == 0 && i < n) {
-        for (int q = 1; q < 8; ++q) {
-            m = max(m, sh[q][lane]);
-            sum += ss[q][lane];
-        }
+    // warp w sums row w
+    m = sh[lane][w];
+    sum = ss[lane][w];
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+        m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
+        sum += __shfl_xor_sync(0xffffffffu, sum, d);
+    }
+    const int64_t r = (int64_t)blockIdx.x * 32 + w;
+    if (lane == 0 && r < n) {
         const int e = magnitude_exponent(m);
-        exps[blockIdx.y * estride + i] = e;
-        if (e == kNoScale || (must_spread && !spread(__longlong_as_double((long long)m), sum, n))) flag[blockIdx.y] = 1;
+        exps[blockIdx.y * n + r] = e;
+        if (e == kNoScale || !spread(__longlong_as_double((long long)m), sum, n)) flag[blockIdx.y] = 1;
     }
 }
 
@@ -176,18 +191,20 @@ __device__ __forceinline__ int64_t plane_offset(int s, int64_t i, int64_t k0, in
     return ((s * (rows / BM) + i / BM) * (kp / BK) + k0 / BK) * kTileValues + r * BK + ((c ^ (r & 7)) << 3);
 }
 
-// Planes of the columns of X (rows, kp padded; zeros outside).  One thread per 8 inner indices.
+// Planes of the columns of X (rows, kp padded; zeros outside).  One thread per 8 inner indices;
+// blockIdx.z = matrix, from `count` on the second operand's.
 static __global__ void __launch_bounds__(256)
-slice_columns_kernel(const double* __restrict__ X, int64_t ld, int64_t n, int64_t stride, const int* __restrict__ exps,
-                     int64_t estride, int64_t rows, int64_t kp, __nv_bfloat16* __restrict__ planes, int64_t pstride,
+slice_columns_kernel(Operand o0, Operand o1, int count, int64_t n, int64_t rows, int64_t kp, int64_t pstride,
                      const int* __restrict__ flag)
 {
-    if (flag[blockIdx.z]) return;
+    const Operand& o = (int)blockIdx.z < count ? o0 : o1;
+    const int64_t z = (int)blockIdx.z < count ? blockIdx.z : blockIdx.z - count;
+    if (flag[z]) return;
     const int64_t k0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
     const int64_t i = blockIdx.y;
     if (k0 >= kp) return;
-    const double* x = X + blockIdx.z * stride + i * ld;
-    const int e = i < n ? exps[blockIdx.z * estride + i] : 0;
+    const double* x = o.x + (z * n + i) * n;
+    const int e = i < n ? o.exps[z * n + i] : 0;
     uint32_t out[S][4];
     int d0[S], d1[S];
 #pragma unroll
@@ -198,7 +215,7 @@ slice_columns_kernel(const double* __restrict__ X, int64_t ld, int64_t n, int64_
 #pragma unroll
         for (int s = 0; s < S; ++s) out[s][q] = pack(d0[s], d1[s]);
     }
-    __nv_bfloat16* p = planes + blockIdx.z * pstride + plane_offset(0, i, k0, rows, kp);
+    __nv_bfloat16* p = o.planes + z * pstride + plane_offset(0, i, k0, rows, kp);
 #pragma unroll
     for (int s = 0; s < S; ++s)
         *reinterpret_cast<uint4*>(p + s * rows * kp) = make_uint4(out[s][0], out[s][1], out[s][2], out[s][3]);
@@ -207,23 +224,22 @@ slice_columns_kernel(const double* __restrict__ X, int64_t ld, int64_t n, int64_
 // Planes of the rows of X (n x n): as slice_columns_kernel on the transpose, through a 32 x 64
 // shared tile.
 static __global__ void __launch_bounds__(256)
-slice_rows_kernel(const double* __restrict__ X, int64_t ld, int64_t n, int64_t stride, const int* __restrict__ exps,
-                  int64_t estride, int64_t rows, int64_t kp, __nv_bfloat16* __restrict__ planes, int64_t pstride,
+slice_rows_kernel(const double* __restrict__ X, int64_t n, const int* __restrict__ exps, int64_t rows, int64_t kp, __nv_bfloat16* __restrict__ planes, int64_t pstride,
                   const int* __restrict__ flag)
 {
     if (flag[blockIdx.z]) return;
     __shared__ double tile[64][33];   // [inner][row]
     const int64_t i0 = (int64_t)blockIdx.y * 32, k0 = (int64_t)blockIdx.x * 64;
-    const double* x = X + blockIdx.z * stride;
+    const double* x = X + blockIdx.z * n * n;
     for (int t = threadIdx.x; t < 64 * 32; t += blockDim.x) {
         const int r = t & 31, c = t >> 5;
-        tile[c][r] = i0 + r < n && k0 + c < n ? x[i0 + r + (k0 + c) * ld] : 0.0;
+        tile[c][r] = i0 + r < n && k0 + c < n ? x[i0 + r + (k0 + c) * n] : 0.0;
     }
     __syncthreads();
     const int r = threadIdx.x >> 3, c = (threadIdx.x & 7) * 8;
     const int64_t i = i0 + r;
     if (i >= rows || k0 + c >= kp) return;
-    const int e = i < n ? exps[blockIdx.z * estride + i] : 0;
+    const int e = i < n ? exps[blockIdx.z * n + i] : 0;
     uint32_t out[S][4];
     int d0[S], d1[S];
 #pragma unroll
