@@ -908,7 +908,7 @@ def measure_adjoint(pkg, n=4096, K=64, chase_mode=3, batched=True, with_cpu=True
     ref_s = time.perf_counter() - tr0
     g = np.concatenate([td.grad.cpu().numpy(), te.grad.cpu().numpy()])
     rel = float(np.linalg.norm(g - g_ref) / np.linalg.norm(g_ref))
-    # the adjoint kernels alone (two FP64 tensor-core GEMMs with fused epilogues)
+    # the adjoint kernels alone (two FP64 GEMMs with fused epilogues; FP64 MMA for localized Q)
     glam = torch.randn(n, device=dev, dtype=torch.float64)
     gQ = torch.randn(n, n, device=dev, dtype=torch.float64)
     lam_d, Q_d = lam.detach(), Q.detach()

@@ -257,8 +257,11 @@ int symeig_batched_tuning(int64_t* split, int32_t* shape_small, int32_t* shape_l
  * for a loss of the eigenvalues only).  Writes dL/dd (gd, n each) and dL/de (ge, n-1 each):
  *   M = diag(glam) + F o (Q^T gQ), F_ij = 1/(lam_j - lam_i) (0 on the diagonal and where
  *   lam_i == lam_j), Abar = Q M Q^T, dL/dd_i = Abar_ii, dL/de_i = Abar_{i,i+1} + Abar_{i+1,i}.
- * Q^T gQ and Q M run on the FP64 tensor cores (mma.sync .f64) with the F-masking and the
- * (off-)diagonal extraction fused into their epilogues; Abar is never formed. */
+ * Q^T gQ and Q M run on the tensor cores with the F-masking and the (off-)diagonal extraction
+ * fused into their epilogues; Abar is never formed.  From n = 256 a spread-out Q takes exact bf16
+ * slices (tcgen05), any other the FP64 MMA (mma.sync .f64).  The choice is made on the device, per
+ * matrix.  Scratch of the handle: 8 bytes per element of the batch, and for the slices up to 44 more
+ * for each of at most 512 MiB worth of matrices; without room for these the FP64 MMA runs. */
 int symeig_eig_adjoint_f64(symeig_handle h, int64_t count, int64_t n, const double* lam,
                            const double* Q, const double* glam, const double* gQ, double* gd,
                            double* ge);

@@ -14,7 +14,7 @@ and three additions without a reference counterpart:
 
     qr_algorithm_batched!(Hs::Vector{SymTridiagonal{Float64}}, Qs; max_layers, tol, maxiter_factor)
     tridiag_eigen(d, e) -> (lam, Q), differentiable through a ChainRulesCore rrule whose
-        pullback is the library's adjoint (FP64 tensor-core GEMMs with fused epilogues)
+        pullback is the library's adjoint (tensor-core GEMMs with fused epilogues)
     bulk_wave_order_2x2_lmul!(A, givens)                      # bulk form of lmul!, src/simple_givens.jl:38
     get_rotation(f, g) -> (c, s, r), elementwise               # src/simple_givens.jl:20
     syev!(A) -> (lam, V): dense symmetric eigensolve (sytrd, orgtr, qr_algorithm!)
