@@ -288,8 +288,8 @@ __global__ void adjoint_lambda_only_kernel(const double* __restrict__ Q, int64_t
 }  // namespace
 
 // From this order on the products run on the bf16 tensor cores where Q is spread out.  FP64 MMA against
-// sliced, one matrix: n = 130 427 / 308 us, 256 700 / 336, 512 1314 / 430, 1024 4.78 / 0.66 ms, 2047 32.8 / 2.0,
-// 4096 252 / 10.8; 25 of n = 257 3226 / 957 us, 4 of 700 6590 / 692.  A localized Q pays for the question and the kernels
+// sliced, one matrix: n = 130 427 / 308 us, 256 700 / 324, 512 1314 / 407, 1024 4.78 / 0.61 ms, 2047 32.8 / 1.73,
+// 4096 252 / 10.0; 25 of n = 257 3226 / 752 us, 4 of 700 6590 / 573.  A localized Q pays for the question and the kernels
 // that return at once: 45 us of 810 at n = 300, 60 of 4700 at 1000, 100 us of 32.8 ms at 2047; below
 // n = 256 it would be above 6 %.  The rule leaves the count out, so that a matrix has the same bits
 // alone and in a batch.

@@ -26,8 +26,8 @@
 // in memory as the tensor core wants them, 128 x 64 tiles of 16 KB with the 128-byte swizzle, so one
 // bulk copy brings each.  Four levels at a time have a 128-column accumulator each, so that a plane's
 // tile is read once for all of them, 37 bytes a clock and SM at the tensor core's rate (one product at a
-// time would take 128).  Two products at n = 2047 take 2.0 ms with everything (mma.sync with 128 x 128 tiles of
-// the same operands: 5.4), at n = 4096 10.9 ms, 1130 TFLOP/s in bf16 counted over the whole call.  At
+// time would take 128).  Two products at n = 2047 take 1.73 ms with everything (mma.sync with 128 x 128 tiles of
+// the same operands: 5.4), at n = 4096 10.0 ms, 1240 TFLOP/s in bf16 counted over the whole call.  At
 // n = 2047 256 tiles on 152 SMs are two waves, 84 % full; a tile's own time is the products (256 cycles
 // each, 1440 of them), the sums' way out of TMEM (18 times, between which the tensor core waits) and the
 // epilogue's FP64 division.
@@ -65,12 +65,19 @@ __device__ __forceinline__ int magnitude_exponent(uint64_t abs_bits)
 
 constexpr int kFixedBits = 6 + 7 * (S - 1);
 
-// x 2^(kFixedBits - e) rounded to an integer (|x| < 2^e, so at most 2^62)
+// x 2^(kFixedBits - e) rounded to an integer (|x| < 2^e, so below 2^62), from the bits: in FP64 the
+// scaling and the conversion kept the slicing kernels on the 2-lane FP64 pipe (80 % busy; the whole adjoint
+// of n = 2047 1.94 ms, 1.73 from the bits).
 __device__ __forceinline__ long long fixed_point(double x, int e)
 {
-    // in two exact steps, so that the scale factors stay normal
-    const int sh = kFixedBits - e, h = sh / 2;
-    return __double2ll_rn(scalbn(scalbn(x, h), sh - h));
+    const uint64_t b = (uint64_t)__double_as_longlong(x);
+    const int ef = (int)(b >> 52) & 0x7FF;
+    uint64_t m = b & 0x000FFFFFFFFFFFFFull;
+    if (ef) m |= 0x0010000000000000ull;
+    const int sh = max(ef, 1) - 1075 + kFixedBits - e;   // |x| = m 2^(max(ef, 1) - 1075); m << sh < 2^62
+    const int down = min(-sh, 60);                       // m < 2^53: from 55 on the result is 0
+    m = sh >= 0 ? m << sh : (m + (1ull << (down - 1))) >> down;
+    return (long long)b < 0 ? -(long long)m : (long long)m;
 }
 
 // the S balanced digits of v, plane s at d[s]
@@ -123,7 +130,7 @@ column_exponents_kernel(Operand o0, Operand o1, int64_t n, int* __restrict__ fla
     for (int64_t k = threadIdx.x; k < n; k += blockDim.x) {
         const double v = x[k];
         m = max(m, (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull);
-        sum = fma(v, v, sum);
+        if (o.must_spread) sum = fma(v, v, sum);
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
