@@ -11,8 +11,8 @@
 // is stored.
 //
 // Two FP64 GEMMs with fused epilogues, on the bf16 tensor cores by exact slices (sliced_gemm.cuh)
-// from n = kSlicedMin on, else (and where Q is localized or an operand holds an infinity or NaN,
-// which the device decides) on the FP64 MMA
+// from n = kSlicedMin on, else (and where Q is localized, the slices would lose accuracy or an operand
+// holds an infinity or NaN, which the device decides) on the FP64 MMA
 // (dmma_tile.cuh: mma.sync m8n8k4 .f64; tcgen05 has no f64 kind):
 //   1. G = Q^T gQ, epilogue M_ij = i == j ? glam_i : G_ij / (lam_j - lam_i), M stored.
 //   2. P = Q M, epilogue: per row i the partial sums over the CTA's columns k of
@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 
 #include "symeig.h"
 #include "symeig_common.cuh"
@@ -164,6 +165,109 @@ __global__ void adjoint_reduce_kernel(const double* __restrict__ part, int64_t n
 
 // ---- the same on the bf16 tensor cores (sliced_gemm.cuh) -------------------------------------
 
+// Before 1.: whether the slices keep FP64's accuracy in every entry of Q^T gQ (sliced_gemm.cuh; a column
+// of zeros is exact, and M's diagonal takes none).  `need`: the least L.
+__global__ void __launch_bounds__(sliced::kThreads, 1)
+sliced_m_check_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B, const int* __restrict__ ea,
+                      const int* __restrict__ eb, int64_t n, int64_t rows, int64_t kp, int64_t pstride, float need,
+                      int* __restrict__ fallback)
+{
+    extern __shared__ __align__(1024) unsigned char smem[];
+    const int64_t z = blockIdx.z;
+    const bool skip = fallback[z] != 0;
+    if (__syncthreads_or(skip)) return;
+    const int64_t i0 = (int64_t)blockIdx.y * sliced::BM, j0 = (int64_t)blockIdx.x * sliced::BN;
+    float L[64];
+    bool poor = !sliced::tile_product<true>(A + z * pstride, B + z * pstride, rows, kp, i0, j0, smem, nullptr, L);
+    const int64_t i = i0 + sliced::tile_row();
+    if (threadIdx.x < sliced::kEpiThreads && i < n && ea[z * n + i] != sliced::kZeroScale) {
+#pragma unroll
+        for (int q = 0; q < 64; ++q) {
+            const int64_t j = j0 + sliced::tile_col() + q;
+            if (j < n && j != i && L[q] < need && eb[z * n + j] != sliced::kZeroScale) poor = true;
+        }
+    }
+    if (__syncthreads_or(poor) && threadIdx.x == 0) fallback[z] = 1;
+}
+
+// Before 2.: whether they keep it in the gradient's entries.  dd_i = sum_k Q_ik P_ik has from P = Q M the errors
+//   FP64    2^-53 sum_k |Q_ik| sum_j |Q_ij| |M_jk| >= 2^(-65 + ea_i) sum_k |Q_ik| 2^eb_k L_ik,
+//   slices  sqrt(n) 2^-63 2^ea_i sum_k |Q_ik| 2^eb_k
+// (as scales, and n for both as bounds), so  sum_k |Q_ik| 2^eb_k (L_ik - need) >= 0  is asked of every row, and the
+// same with the weights |Q_{i+1,k}| and |Q_{i-1,k}| for de_i and de_{i-1}.  A CTA leaves its columns'
+// part of the three sums in `margin`; the last one of a row of tiles adds them up.  The terms are in FP32
+// about the tile's largest column, on the safe side: a weight below 2^-60 of its row's largest counts as
+// 2^-60 against and as 0 for the slices, and a column below 2^-60 of the tile's largest fails.
+__global__ void __launch_bounds__(sliced::kThreads, 1)
+sliced_p_check_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B, const int* __restrict__ ea,
+                      const int* __restrict__ eb, const double* __restrict__ Q, int64_t n, int64_t rows, int64_t kp,
+                      int64_t pstride, float need, double* __restrict__ margin, int64_t stride_margin,
+                      int* __restrict__ done, int* __restrict__ fallback)
+{
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ float red[3][2][sliced::BM], scale[sliced::BN];
+    __shared__ int top, last;
+    const int64_t z = blockIdx.z;
+    const bool skip = fallback[z] != 0;
+    if (__syncthreads_or(skip)) return;
+    Q += z * n * n;
+    margin += z * stride_margin;
+    ea += z * n;
+    eb += z * n;
+    const int64_t i0 = (int64_t)blockIdx.y * sliced::BM, k0 = (int64_t)blockIdx.x * sliced::BN;
+    if (threadIdx.x == 0) top = sliced::kZeroScale;
+    __syncthreads();
+    int e = sliced::kZeroScale;
+    if (threadIdx.x < sliced::BN && k0 + threadIdx.x < n) e = eb[k0 + threadIdx.x];
+    if (threadIdx.x < sliced::BN) atomicMax(&top, e);
+    __syncthreads();
+    bool poor = e != sliced::kZeroScale && e < top - 60;
+    if (threadIdx.x < sliced::BN) scale[threadIdx.x] = e == sliced::kZeroScale || poor ? 0.0f : exp2f((float)(e - top));
+    float L[64];
+    if (!sliced::tile_product<true>(A + z * pstride, B + z * pstride, rows, kp, i0, k0, smem, nullptr, L)) poor = true;
+    if (__syncthreads_or(poor)) {
+        if (threadIdx.x == 0) fallback[z] = 1;
+        return;
+    }
+    const int r = sliced::tile_row();
+    const int64_t i = i0 + r;
+    if (threadIdx.x < sliced::kEpiThreads) {
+#pragma unroll
+        for (int t = 0; t < 3; ++t) {
+            const int64_t w = t == 0 ? i : t == 1 ? i + 1 : i - 1;   // the row whose entries weigh
+            float m = 0.0f;
+            if (i < n && w >= 0 && w < n) {
+                const int ew = ea[w];
+#pragma unroll
+                for (int q = 0; q < 64; ++q) {
+                    const int64_t k = k0 + sliced::tile_col() + q;
+                    if (k < n) m += sliced::weighted(Q[w + k * n], ew, (L[q] - need) * scale[sliced::tile_col() + q]);
+                }
+            }
+            red[t][threadIdx.x >> 7][r] = m;
+        }
+    }
+    __syncthreads();
+    const int64_t tiles = gridDim.x;
+    if (threadIdx.x < sliced::BM && i < n)
+#pragma unroll
+        for (int t = 0; t < 3; ++t)
+            margin[((int64_t)t * tiles + blockIdx.x) * n + i] = scalbn((double)red[t][0][r] + (double)red[t][1][r], top);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(&done[z * gridDim.y + blockIdx.y], 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    if (threadIdx.x < sliced::BM && i < n)
+        for (int t = 0; t < 3; ++t) {
+            double m = 0.0;
+            for (int64_t b = 0; b < tiles; ++b) m += __ldcg(&margin[((int64_t)t * tiles + b) * n + i]);
+            poor |= !(m >= 0.0);
+        }
+    if (__syncthreads_or(poor) && threadIdx.x == 0) fallback[z] = 1;
+}
+
 // 1. as adjoint_m_kernel.  A: planes of Q's columns with exponents ea; B: of gQ's columns with eb.
 __global__ void __launch_bounds__(sliced::kThreads, 1)
 sliced_m_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B, const int* __restrict__ ea,
@@ -181,7 +285,7 @@ sliced_m_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __rest
     park += ((z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * sliced::BM * sliced::BN;
     const int64_t i0 = (int64_t)blockIdx.y * sliced::BM, j0 = (int64_t)blockIdx.x * sliced::BN;
     double acc[64];
-    if (!sliced::tile_product(A + z * pstride, B + z * pstride, rows, kp, i0, j0, smem, park, acc)) {
+    if (!sliced::tile_product<false>(A + z * pstride, B + z * pstride, rows, kp, i0, j0, smem, park, acc)) {
         if (threadIdx.x == 0) fallback[z] = 1;
         return;
     }
@@ -221,7 +325,7 @@ sliced_p_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __rest
     park += ((z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * sliced::BM * sliced::BN;
     const int64_t i0 = (int64_t)blockIdx.y * sliced::BM, k0 = (int64_t)blockIdx.x * sliced::BN;
     double acc[64];
-    if (!sliced::tile_product(A + z * pstride, B + z * pstride, rows, kp, i0, k0, smem, park, acc)) {
+    if (!sliced::tile_product<false>(A + z * pstride, B + z * pstride, rows, kp, i0, k0, smem, park, acc)) {
         if (threadIdx.x == 0) fallback[z] = 1;
         return;
     }
@@ -310,11 +414,11 @@ static int64_t sliced_group(int64_t count, int64_t n)
 }
 
 // The scratch after M and the partials: two operands' planes, the tiles' small sums, the operands' exponents, a
-// flag a matrix.
+// flag a matrix and a counter a row of tiles.
 static int64_t sliced_scratch_doubles(int64_t count, int64_t n)
 {
     const int64_t g = sliced_group(count, n), r = sliced::pad_rows(n);
-    return g * (2 * sliced::plane_values(n, n) * 2 + r * r * (int64_t)sizeof(double) + (2 * n + 1) * (int64_t)sizeof(int)) / 8 + 64;
+    return g * (2 * sliced::plane_values(n, n) * 2 + r * r * (int64_t)sizeof(double) + (2 * n + 1 + r / sliced::BM) * (int64_t)sizeof(int)) / 8 + 64;
 }
 
 // Device-pointer adjoint for `count` matrices of order n stored back to back (Q, gQ with
@@ -342,9 +446,10 @@ int adjoint_dev(cudaStream_t s, int64_t count, int64_t n, const double* lam, con
         adjoint_reduce_kernel<<<dim3((unsigned)((n + 255) / 256), (unsigned)count), 256, 0, s>>>(part, n, gd, ge, stridePart, nullptr);
         return cudaGetLastError() == cudaSuccess ? SYMEIG_OK : SYMEIG_ERR_CUDA;
     }
-    if (cudaFuncSetAttribute(sliced_m_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sliced::kSmem) != cudaSuccess ||
-        cudaFuncSetAttribute(sliced_p_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sliced::kSmem) != cudaSuccess)
-        return SYMEIG_ERR_CUDA;
+    for (const void* k : {(const void*)sliced_m_kernel, (const void*)sliced_p_kernel, (const void*)sliced_m_check_kernel,
+                          (const void*)sliced_p_check_kernel})
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sliced::kSmem) != cudaSuccess)
+            return SYMEIG_ERR_CUDA;
     const int64_t group = sliced_group(count, n), rows = sliced::pad_rows(n), kp = sliced::pad_k(n);
     const int64_t pstride = sliced::plane_values(n, n);
     // 256-byte aligned: the planes' 16-byte pieces
@@ -356,6 +461,8 @@ int adjoint_dev(cudaStream_t s, int64_t count, int64_t n, const double* lam, con
     int* eb = ea + group * n;
     int* flag = eb + group * n;
     const int64_t ntiles = (n + sliced::BN - 1) / sliced::BN;
+    int* done = flag + group;
+    const float need = (float)(sliced::kLeadFactor * std::sqrt((double)n));
     for (int64_t z = 0; z < count; z += group) {
         const unsigned g = (unsigned)std::min<int64_t>(group, count - z);
         const double *Qz = Q + z * strideQ, *Gz = gQ + z * strideQ, *lz = lam + z * n, *glz = glam + z * n;
@@ -364,9 +471,10 @@ int adjoint_dev(cudaStream_t s, int64_t count, int64_t n, const double* lam, con
         const dim3 fgrid(grid.x, grid.y, g), sgrid((unsigned)ntiles, (unsigned)ntiles, g);
         const dim3 cgrid((unsigned)((kp / 8 + 255) / 256), (unsigned)rows, g);
         const sliced::Operand oq{Qz, ea, PA, true}, og{Gz, eb, PB, false}, om{Mz, eb, PB, false};
-        if (cudaMemsetAsync(flag, 0, group * sizeof(int), s) != cudaSuccess) return SYMEIG_ERR_CUDA;
+        if (cudaMemsetAsync(flag, 0, group * (1 + ntiles) * sizeof(int), s) != cudaSuccess) return SYMEIG_ERR_CUDA;
         sliced::column_exponents_kernel<<<dim3((unsigned)n, g, 2), 256, 0, s>>>(oq, og, n, flag);
         sliced::slice_columns_kernel<<<dim3(cgrid.x, cgrid.y, 2 * g), 256, 0, s>>>(oq, og, (int)g, n, rows, kp, pstride, flag);
+        sliced_m_check_kernel<<<sgrid, sliced::kThreads, sliced::kSmem, s>>>(PA, PB, ea, eb, n, rows, kp, pstride, need, flag);
         sliced_m_kernel<<<sgrid, sliced::kThreads, sliced::kSmem, s>>>(PA, PB, ea, eb, lz, glz, n, rows, kp, pstride, Mz, park, flag);
         adjoint_m_kernel<<<fgrid, kAdjThreads, 0, s>>>(Qz, n, Gz, n, lz, glz, n, Mz, strideQ, strideQ, strideM, flag);
         sliced::row_exponents_kernel<<<dim3((unsigned)((n + 31) / 32), g), 1024, 0, s>>>(Qz, n, ea, flag);
@@ -374,6 +482,9 @@ int adjoint_dev(cudaStream_t s, int64_t count, int64_t n, const double* lam, con
         sliced::slice_rows_kernel<<<dim3((unsigned)((kp + 63) / 64), (unsigned)((rows + 31) / 32), g), 256, 0, s>>>(
             Qz, n, ea, rows, kp, PA, pstride, flag);
         sliced::slice_columns_kernel<<<cgrid, 256, 0, s>>>(om, om, (int)g, n, rows, kp, pstride, flag);
+        // (pz: the margins, before the partial sums take their place)
+        sliced_p_check_kernel<<<sgrid, sliced::kThreads, sliced::kSmem, s>>>(PA, PB, ea, eb, Qz, n, rows, kp, pstride, need, pz,
+                                                                            stridePart, done, flag);
         sliced_p_kernel<<<sgrid, sliced::kThreads, sliced::kSmem, s>>>(PA, PB, ea, eb, Qz, n, rows, kp, pstride, pz, stridePart, park, flag);
         adjoint_p_kernel<<<fgrid, kAdjThreads, 0, s>>>(Qz, n, Mz, n, pz, strideQ, strideM, stridePart, flag);
         adjoint_reduce_kernel<<<dim3((unsigned)((n + 255) / 256), g), 256, 0, s>>>(pz, n, gd + z * n, gez, stridePart, flag);

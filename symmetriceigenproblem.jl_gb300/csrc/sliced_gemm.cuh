@@ -11,14 +11,23 @@
 //   * each chunk's sums go to 64-bit integers, levels S-1 .. 5 to one, 4 .. 0 to another, still exactly,
 //     and those two to FP64 at the end: two roundings in all.  (FP64 sums per chunk cost 128 instructions a
 //     thread at the FP64 pipe's two lanes a clock, 16k cycles; as integers it is 512.)
-// What is dropped (digits past 2^-63, levels past S - 1) is 2^-63 of the row's maximum times the
-// column's for each term, where FP64 rounds each by 2^-53 of its own size.  That is the smaller of the two
-// while one operand is spread out (kMaxOverRms, checked by the exponent kernels), so that a large entry of the
-// other meets an entry of ordinary size.  Measured against longer arithmetic, gradients of Toeplitz
-// eigenvectors n = 257 .. 2047: 1.4e-16 .. 2.3e-16 of their norm, FP64 MMA 6.0e-16 .. 1.9e-15; Gaussian orthogonal Q,
-// n = 600: 1.7e-16 against 1.9e-15.  Localized eigenvectors with close eigenvalues (random diagonal, n = 1000)
-// would give 2.6e-15 against 2.6e-16: they stay with the FP64 MMA.
-// A localized operand, an infinity or a NaN sets the matrix's flag word: the sliced
+// What is dropped (digits past 2^-63, levels past S - 1) is at most 10 n 2^-63 of the row's maximum times the
+// column's, and about sqrt(n) 2^-63 of them where the digits' signs are mixed, whatever the entries that
+// meet.  FP64 rounds each term by 2^-53 of its own size: its error is on the scale of 2^-53 sum |a_k| |b_k|, and
+// that sum is far below n max max where the large entries of one operand meet small ones or zeros of the other.
+// So the sum is measured: one more plane holds the leading digit of each magnitude, floor(64 |a| 2^-ea), and the
+// product of the leading planes, L, bounds it from below, sum |a_k| |b_k| >= 2^(ea + eb - 12) L.  With
+//   L >= kLeadFactor sqrt(n),  kLeadFactor = 4,
+// sqrt(n) 2^-63 max max is below 2^-53 sum |a_k| |b_k|, and 10 n 2^-63 max max below FP64's bound
+// n 2^-53 sum |a_k| |b_k| (n >= 100).  The caller asks that of every entry of the first product, and of the
+// second one summed over a row with the weights its entries enter the gradient with.  Errors of the gradient's
+// entries over 2^-53 times their FP64 scale, against longer arithmetic, FP64 -> sliced: Toeplitz eigenvectors n = 256 .. 1100
+// (L from 130 sqrt(n)) 0.6-1.5 -> 0.2-0.35; Gaussian orthogonal Q, n = 600 (10.8) 4.8 -> 1.1; a gradient of one
+// eigenvector (0.7) 15 -> 5; localized eigenvectors (random diagonal as large as the couplings, 0.05)
+// 12 -> 14: equal at about a hundredth of the line.  Without the question two uncoupled chains with spectra 1e-10 apart
+// (L = 0: 1 / gap of a pair from both chains meets a zero of Q) gave 1e5 where FP64 gives 1.
+// Localized Q is turned away before that, from its rows' and columns' norms (kMaxOverRms): it would mostly fail.
+// A localized operand, an L too small, an infinity or a NaN sets the matrix's flag word: the sliced
 // kernels return at once for it and the caller's FP64 MMA kernels, launched behind them
 // with the opposite test, do the work.
 //
@@ -50,17 +59,19 @@ static_assert(BM == 128 && BN == 128, "a tile is one tcgen05 shape");
 
 inline int64_t pad_rows(int64_t n) { return (n + BM - 1) / BM * BM; }
 inline int64_t pad_k(int64_t n) { return (n + BK - 1) / BK * BK; }
-// bf16 values of one operand's planes
-inline int64_t plane_values(int64_t rows, int64_t k) { return S * pad_rows(rows) * pad_k(k); }
+// bf16 values of one operand's planes: the digits and, plane S, the magnitudes' leading digits
+constexpr int kPlanes = S + 1;
+inline int64_t plane_values(int64_t rows, int64_t k) { return kPlanes * pad_rows(rows) * pad_k(k); }
+constexpr double kLeadFactor = 4.0;
 
-// A magnitude's exponent e with |x| < 2^e, or kNoScale for infinity and NaN (0 gives -1075).
-constexpr int kNoScale = 1 << 20;
+// A magnitude's exponent e with |x| < 2^e, or kNoScale for infinity and NaN, kZeroScale for 0.
+constexpr int kNoScale = 1 << 20, kZeroScale = -1075;
 __device__ __forceinline__ int magnitude_exponent(uint64_t abs_bits)
 {
     if (abs_bits >= 0x7FF0000000000000ull) return kNoScale;
     const int ef = (int)(abs_bits >> 52);
     if (ef > 0) return ef - 1022;
-    return abs_bits == 0 ? -1075 : -1010 - (__clzll((long long)abs_bits));   // subnormal: 2^-1074 * 2^(64 - clz)
+    return abs_bits == 0 ? kZeroScale : -1010 - (__clzll((long long)abs_bits));   // subnormal: 2^-1074 * 2^(64 - clz)
 }
 
 constexpr int kFixedBits = 6 + 7 * (S - 1);
@@ -80,9 +91,10 @@ __device__ __forceinline__ long long fixed_point(double x, int e)
     return (long long)b < 0 ? -(long long)m : (long long)m;
 }
 
-// the S balanced digits of v, plane s at d[s]
-__device__ __forceinline__ void digits(long long v, int (&d)[S])
+// the S balanced digits of v, plane s at d[s], and |v|'s leading digit
+__device__ __forceinline__ void digits(long long v, int (&d)[kPlanes])
 {
+    d[S] = (int)(llabs(v) >> 7 * (S - 1));
 #pragma unroll
     for (int s = S - 1; s > 0; --s) {
         const int t = (int)((v + 64) & 127) - 64;
@@ -100,11 +112,23 @@ __device__ __forceinline__ uint32_t pack(int lo, int hi)
 
 // `spread` operands: n max^2 <= kMaxOverRms^2 sum x^2 per row or column (entries of an eigenvector of
 // a Toeplitz matrix reach 1.4 times their rms, Gaussian ones 4 to 5, a localized one's about sqrt(n), 16 for
-// the smallest order).  Where the squares leave the FP64 range the answer is no.
+// the smallest order).  Where the squares leave the FP64 range the answer is no.  This spares a
+// localized Q the slicing; what the slices are good for, L decides.
 constexpr double kMaxOverRms = 6.0;
 __device__ __forceinline__ bool spread(double mx, double sum, int64_t n)
 {
     return mx == 0.0 || (mx > 1e-140 && mx < 1e140 && mx * mx * (double)n <= kMaxOverRms * kMaxOverRms * sum);
+}
+
+// |x| 2^-e v for |x| < 2^e, never more: a weight |x| 2^-e below 2^-60 (but not 0) counts as 2^-60 where v is
+// negative and as 0 where it is not.
+__device__ __forceinline__ float weighted(double x, int e, float v)
+{
+    const int hi = __double2hiint(x) & 0x7FFFFFFF, lo = __double2loint(x);
+    if ((hi | lo) == 0) return 0.0f;
+    const int d = (hi >> 20) - 1022 - e;   // |x| in [2^(d-1), 2^d) 2^e
+    if (d <= -60) return v < 0.0f ? v * 0x1p-60f : 0.0f;
+    return v * __int_as_float((d + 126) << 23 | (hi & 0xFFFFF) << 3 | (int)((uint32_t)lo >> 29));
 }
 
 // Two operands of one launch (blockIdx.z, or its part beyond the matrices, picks one): a launch saved
@@ -212,19 +236,19 @@ slice_columns_kernel(Operand o0, Operand o1, int count, int64_t n, int64_t rows,
     if (k0 >= kp) return;
     const double* x = o.x + (z * n + i) * n;
     const int e = i < n ? o.exps[z * n + i] : 0;
-    uint32_t out[S][4];
-    int d0[S], d1[S];
+    uint32_t out[kPlanes][4];
+    int d0[kPlanes], d1[kPlanes];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const int64_t k = k0 + 2 * q;
         digits(i < n && k < n ? fixed_point(x[k], e) : 0, d0);
         digits(i < n && k + 1 < n ? fixed_point(x[k + 1], e) : 0, d1);
 #pragma unroll
-        for (int s = 0; s < S; ++s) out[s][q] = pack(d0[s], d1[s]);
+        for (int s = 0; s < kPlanes; ++s) out[s][q] = pack(d0[s], d1[s]);
     }
     __nv_bfloat16* p = o.planes + z * pstride + plane_offset(0, i, k0, rows, kp);
 #pragma unroll
-    for (int s = 0; s < S; ++s)
+    for (int s = 0; s < kPlanes; ++s)
         *reinterpret_cast<uint4*>(p + s * rows * kp) = make_uint4(out[s][0], out[s][1], out[s][2], out[s][3]);
 }
 
@@ -247,18 +271,18 @@ slice_rows_kernel(const double* __restrict__ X, int64_t n, const int* __restrict
     const int64_t i = i0 + r;
     if (i >= rows || k0 + c >= kp) return;
     const int e = i < n ? exps[blockIdx.z * n + i] : 0;
-    uint32_t out[S][4];
-    int d0[S], d1[S];
+    uint32_t out[kPlanes][4];
+    int d0[kPlanes], d1[kPlanes];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         digits(i < n ? fixed_point(tile[c + 2 * q][r], e) : 0, d0);
         digits(i < n ? fixed_point(tile[c + 2 * q + 1][r], e) : 0, d1);
 #pragma unroll
-        for (int s = 0; s < S; ++s) out[s][q] = pack(d0[s], d1[s]);
+        for (int s = 0; s < kPlanes; ++s) out[s][q] = pack(d0[s], d1[s]);
     }
     __nv_bfloat16* p = planes + blockIdx.z * pstride + plane_offset(0, i, k0 + c, rows, kp);
 #pragma unroll
-    for (int s = 0; s < S; ++s)
+    for (int s = 0; s < kPlanes; ++s)
         *reinterpret_cast<uint4*>(p + s * rows * kp) = make_uint4(out[s][0], out[s][1], out[s][2], out[s][3]);
 }
 
@@ -303,6 +327,7 @@ struct Pass {
     // blocks whose sums stay below 2^23: (hi + 1) 64 2^12 each
     __device__ __forceinline__ int chunk_blocks() const { return 32 / (hi + 1); }
 };
+// The last pass alone, on the planes S, gives the leading digits' product L (LEAD).
 constexpr int kPasses = 3;
 __device__ __forceinline__ Pass pass_of(int p)
 {
@@ -339,6 +364,7 @@ __device__ __forceinline__ uint64_t operand_desc(uint32_t addr)
 }
 
 // The copying thread: all tiles of the passes, in order.  Returns once what it started has landed.
+template <bool LEAD>
 __device__ __forceinline__ void copy_tiles(Control& c, uint32_t tiles, const __nv_bfloat16* A, const __nv_bfloat16* B,
                                            int64_t plane, int blocks)
 {
@@ -354,7 +380,7 @@ __device__ __forceinline__ void copy_tiles(Control& c, uint32_t tiles, const __n
                      "l"(src), "r"(kTileBytes), "r"(smem_addr(&c.full[slot])) : "memory");
         ++g;
     };
-    for (int p = 0; p < kPasses && ok; ++p) {
+    for (int p = LEAD ? kPasses - 1 : 0; p < kPasses && ok; ++p) {
         const Pass q = pass_of(p);
         for (int kb = 0; kb < blocks && ok; ++kb) {
             const int64_t o = (int64_t)kb * kTileValues;
@@ -444,14 +470,17 @@ __device__ __forceinline__ bool issue_pass(Control& c, uint64_t desc0, uint32_t 
     return true;
 }
 
+template <bool LEAD>
 __device__ __forceinline__ void issue_products(Control& c, uint32_t tiles, uint32_t tmem, int blocks)
 {
     Ring ring{0, 0};
     uint32_t chunk = 0;
     const uint64_t desc0 = operand_desc(tiles);
-    if (issue_pass<kSmallLevels, S - 1>(c, desc0, tmem, blocks, ring, chunk) &&
-        issue_pass<1, kSmallLevels - 1>(c, desc0, tmem, blocks, ring, chunk))
-        issue_pass<0, 0>(c, desc0, tmem, blocks, ring, chunk);
+    bool ok = true;
+    if constexpr (!LEAD)
+        ok = issue_pass<kSmallLevels, S - 1>(c, desc0, tmem, blocks, ring, chunk) &&
+             issue_pass<1, kSmallLevels - 1>(c, desc0, tmem, blocks, ring, chunk);
+    if (ok) issue_pass<0, 0>(c, desc0, tmem, blocks, ring, chunk);
     // nothing may be in flight when the accumulators are given back
     commit(&c.drained);
     const long long t0 = clock64();
@@ -459,18 +488,24 @@ __device__ __forceinline__ void issue_products(Control& c, uint32_t tiles, uint3
         if (clock64() - t0 > 2000000000ll) break;
 }
 
-// One 128 x 128 tile of sum_{s+t<S} 2^(-12-7(s+t)) A_s B_t^T, rows i0 .. of A's planes by rows j0 .. of B's.
+// One 128 x 128 tile of sum_{s+t<S} 2^(-12-7(s+t)) A_s B_t^T, rows i0 .. of A's planes by rows j0 .. of B's; with
+// LEAD of the leading digits' product A_S B_S^T, which is an integer below 2^28.
 // Thread t < kEpiThreads gets row tile_row(), columns tile_col() .. + 63.  park: 128 KB of memory for this
-// tile.  False, for all threads, if a wait ran out; call it with all kThreads.
+// tile (not with LEAD).  False, for all threads, if a wait ran out; call it with all kThreads.
+template <bool LEAD, typename Out>
 __device__ __forceinline__ bool tile_product(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B,
                                              int64_t rows, int64_t kp, int64_t i0, int64_t j0, unsigned char* smem,
-                                             double* __restrict__ park, double (&out)[64])
+                                             double* __restrict__ park, Out (&out)[64])
 {
     __shared__ Control c;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t tiles = (smem_addr(smem) + 1023) & ~1023u;
     const int blocks = (int)(kp / BK);
     const int64_t plane = rows * kp;
+    if (LEAD) {
+        A += S * plane;
+        B += S * plane;
+    }
     if (warp == 9) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_addr(&c.tmem)) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -492,10 +527,10 @@ __device__ __forceinline__ bool tile_product(const __nv_bfloat16* __restrict__ A
     const uint32_t tmem = c.tmem;
     if (warp == 8) {
         if (lane == 0)
-            copy_tiles(c, tiles, A + i0 / BM * (kp / BK) * kTileValues, B + j0 / BN * (kp / BK) * kTileValues, plane, blocks);
+            copy_tiles<LEAD>(c, tiles, A + i0 / BM * (kp / BK) * kTileValues, B + j0 / BN * (kp / BK) * kTileValues, plane, blocks);
         __syncwarp();
     } else if (warp == 9) {
-        if (lane == 0) issue_products(c, tiles, tmem, blocks);
+        if (lane == 0) issue_products<LEAD>(c, tiles, tmem, blocks);
         __syncwarp();
     } else {
         long long acc[64];
@@ -504,7 +539,7 @@ __device__ __forceinline__ bool tile_product(const __nv_bfloat16* __restrict__ A
         const uint32_t mine = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 64 * (warp >> 2);
         uint32_t chunk = 0;
         bool ok = true;
-        for (int p = 0; p < kPasses && ok; ++p) {
+        for (int p = LEAD ? kPasses - 1 : 0; p < kPasses && ok; ++p) {
             const Pass q = pass_of(p);
             const int step = q.chunk_blocks(), top = p == 0 ? S - 1 : kSmallLevels - 1;
             for (int k0 = 0; k0 < blocks; k0 += step, ++chunk) {
@@ -512,7 +547,7 @@ __device__ __forceinline__ bool tile_product(const __nv_bfloat16* __restrict__ A
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 for (int l = q.lo; l <= q.hi; ++l) {
-                    const int w = 1 << 7 * (top - l);
+                    const int w = LEAD ? 1 : 1 << 7 * (top - l);
 #pragma unroll
                     for (int h = 0; h < 4; ++h) {
                         uint32_t v[16];
@@ -534,7 +569,7 @@ __device__ __forceinline__ bool tile_product(const __nv_bfloat16* __restrict__ A
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&c.sums_empty);
             }
-            if (p == 0) {
+            if (!LEAD && p == 0) {
 #pragma unroll
                 for (int q2 = 0; q2 < 64; ++q2) {
                     park[q2 * kEpiThreads + tid] = __ll2double_rn(acc[q2]);
@@ -545,8 +580,10 @@ __device__ __forceinline__ bool tile_product(const __nv_bfloat16* __restrict__ A
         constexpr double kSmall = 1.0 / (1ull << (12 + 7 * (S - 1) - 28)) / (1ull << 28);
         constexpr double kLarge = 1.0 / (1ull << (12 + 7 * (kSmallLevels - 1)));
 #pragma unroll
-        for (int q = 0; q < 64; ++q)
-            out[q] = fma(__ll2double_rn(acc[q]), kLarge, park[q * kEpiThreads + tid] * kSmall);
+        for (int q = 0; q < 64; ++q) {
+            if constexpr (LEAD) out[q] = (Out)acc[q];
+            else out[q] = fma(__ll2double_rn(acc[q]), kLarge, park[q * kEpiThreads + tid] * kSmall);
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
