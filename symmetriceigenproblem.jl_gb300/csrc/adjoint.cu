@@ -232,20 +232,33 @@ sliced_p_check_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* 
     const int r = sliced::tile_row();
     const int64_t i = i0 + r;
     if (threadIdx.x < sliced::kEpiThreads) {
+        // the neighbouring rows' weights are the neighbouring lanes'; past a warp's ends lanes 0 and 31 read them
+        const int lane = threadIdx.x & 31;
+        const int64_t edge = lane == 0 ? i - 1 : i + 1;
+        const bool ok = i < n, edge_ok = (lane == 0 || lane == 31) && edge >= 0 && edge < n;
+        const int e_row = ok ? ea[i] : 0, e_edge = edge_ok ? ea[edge] : 0;
+        // L through shared memory (the operand tiles are done with) and a loop: unrolled, the code that each
+        // CTA runs once cost its fetches, 44 us at n = 300
+        float* Ls = reinterpret_cast<float*>(smem) + sliced::tile_col() * sliced::BM + r;
 #pragma unroll
-        for (int t = 0; t < 3; ++t) {
-            const int64_t w = t == 0 ? i : t == 1 ? i + 1 : i - 1;   // the row whose entries weigh
-            float m = 0.0f;
-            if (i < n && w >= 0 && w < n) {
-                const int ew = ea[w];
-#pragma unroll
-                for (int q = 0; q < 64; ++q) {
-                    const int64_t k = k0 + sliced::tile_col() + q;
-                    if (k < n) m += sliced::weighted(Q[w + k * n], ew, (L[q] - need) * scale[sliced::tile_col() + q]);
-                }
-            }
-            red[t][threadIdx.x >> 7][r] = m;
+        for (int q = 0; q < 64; ++q) Ls[q * sliced::BM] = L[q];
+        const double* x = Q + i + (k0 + sliced::tile_col()) * n;
+        const int64_t to_edge = edge - i;
+        const int cols = (int)max((int64_t)0, min((int64_t)64, n - k0 - sliced::tile_col()));
+        float m0 = 0.0f, mu = 0.0f, ml = 0.0f;
+#pragma unroll 8
+        for (int q = 0; q < cols; ++q) {
+            const float v = (Ls[q * sliced::BM] - need) * scale[sliced::tile_col() + q];
+            const float w = sliced::weight(ok ? x[q * n] : 0.0, e_row), we = sliced::weight(edge_ok ? x[q * n + to_edge] : 0.0, e_edge);
+            const float wu = __shfl_down_sync(0xffffffffu, w, 1), wl = __shfl_up_sync(0xffffffffu, w, 1);
+            m0 += sliced::weighted(w, v);
+            mu += sliced::weighted(lane == 31 ? we : wu, v);
+            ml += sliced::weighted(lane == 0 ? we : wl, v);
         }
+        const int half = threadIdx.x >> 7;
+        red[0][half][r] = m0;
+        red[1][half][r] = mu;
+        red[2][half][r] = ml;
     }
     __syncthreads();
     const int64_t tiles = gridDim.x;

@@ -120,16 +120,16 @@ __device__ __forceinline__ bool spread(double mx, double sum, int64_t n)
     return mx == 0.0 || (mx > 1e-140 && mx < 1e140 && mx * mx * (double)n <= kMaxOverRms * kMaxOverRms * sum);
 }
 
-// |x| 2^-e v for |x| < 2^e, never more: a weight |x| 2^-e below 2^-60 (but not 0) counts as 2^-60 where v is
-// negative and as 0 where it is not.
-__device__ __forceinline__ float weighted(double x, int e, float v)
+// The weight |x| 2^-e of |x| < 2^e in FP32, -2^-60 for one below 2^-60 (but not 0).
+__device__ __forceinline__ float weight(double x, int e)
 {
     const int hi = __double2hiint(x) & 0x7FFFFFFF, lo = __double2loint(x);
-    if ((hi | lo) == 0) return 0.0f;
     const int d = (hi >> 20) - 1022 - e;   // |x| in [2^(d-1), 2^d) 2^e
-    if (d <= -60) return v < 0.0f ? v * 0x1p-60f : 0.0f;
-    return v * __int_as_float((d + 126) << 23 | (hi & 0xFFFFF) << 3 | (int)((uint32_t)lo >> 29));
+    const float w = d <= -60 ? -0x1p-60f : __int_as_float((d + 126) << 23 | (hi & 0xFFFFF) << 3 | (int)((uint32_t)lo >> 29));
+    return (hi | lo) == 0 ? 0.0f : w;
 }
+// weight times v, never more: a weight below 2^-60 counts as 2^-60 where v is negative and as 0 where it is not
+__device__ __forceinline__ float weighted(float w, float v) { return fabsf(w) * (w < 0.0f ? fminf(v, 0.0f) : v); }
 
 // Two operands of one launch (blockIdx.z, or its part beyond the matrices, picks one): a launch saved
 // where Q is localized and the FP64 MMA does the work after all.
