@@ -10,7 +10,8 @@
 // decides by the exact remainder, so the results are always the correctly rounded ones.
 //
 // Method.  x = 2^(2k) X, X in [1, 4) with 54 bits; y = 1/sqrt(X) in (1/2, 1], R = sqrt(X) = X y.
-//   y0  the hardware's seed (rsqrt.approx.ftz.f64, 21 bits), e = 1 - X y0^2, |e| < 2^-18,
+//   y0  the hardware's seed (rsqrt.approx.ftz.f64, 21 bits), e = 1 - X y0^2, |e| < 2^-18 (tested: a
+//       seed further off takes the reference form),
 //   y   = y0 (1 + e/2 + 3/8 e^2 + 5/16 e^3), the binomial series of (1 - e)^(-1/2); the next
 //         term is below 2^-73.
 // All products are exact integers or truncated towards a known side.  In units of 2^-64,
@@ -128,7 +129,8 @@ __device__ __forceinline__ void givens_int(double f, double g, double x, double&
     const int32_t E = (int32_t)__funnelshift_r(eql, (uint32_t)eqh, 18);
     const int32_t e2 = __mulhi(E, E);
     const int32_t e3 = __mulhi(e2, E);
-    const int32_t qs = ((3 * e2) >> 1) + (((e3 >> 4) * 5) >> 15);    // units 2^-68
+    // units 2^-68; 0 <= e2 <= 2^30, so 3 e2 needs the unsigned word
+    const int32_t qs = (int32_t)((3u * (uint32_t)e2) >> 1) + (((e3 >> 4) * 5) >> 15);
     const int64_t w = (int64_t)mulw(eql, y0) + (int64_t)qs * (int64_t)(int32_t)y0;
     const int64_t v = (int64_t)eqh * (int64_t)(int32_t)y0 + (int64_t)((uint64_t)(y0 << 4) << 32);
     const uint64_t y = ((uint64_t)v << 7) + (uint64_t)(w >> 25) - 1;
