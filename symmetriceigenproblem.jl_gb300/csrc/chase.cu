@@ -35,13 +35,21 @@ __device__ __forceinline__ bool is_small(const double* dv, const double* ev, int
 }
 
 // False only where is_small is false, from the exponent fields: |e| >= 2^(xe-1023), while
-// tol (|d_j| + |d_j+1|) < 2^(xt-1023+1) 2^(max(xd)-1023+2).  An FP64 instruction costs 64 cycles,
-// so the scan runs the exact test only where this cannot decide.
+// tol (|d_j| + |d_j+1|) < 2^(xt-1023+1) 2^(max(xd)-1023+2), unless the sum is infinite (xd >= 2046, where
+// every xe below xt + 1026 passes the second test and those from there on the first, with xe = 0) or tol is
+// (kNoTol).  An FP64 instruction costs 64 cycles, so the scan runs the exact test only where this cannot
+// decide.
+constexpr int32_t kNoTol = 4096;   // above every xe
+__device__ __forceinline__ int32_t tol_exponent(double tol)
+{
+    const int32_t xt = (__double2hiint(tol) >> 20) & 0x7FF;
+    return xt == 0x7FF ? kNoTol : xt;
+}
 __device__ __forceinline__ bool maybe_small(double e, double d0, double d1, int32_t xt)
 {
     const int32_t xe = (__double2hiint(e) >> 20) & 0x7FF;
     const int32_t xd = max((__double2hiint(d0) >> 20) & 0x7FF, (__double2hiint(d1) >> 20) & 0x7FF);
-    return xe == 0 || xe < xt + xd - 1020;
+    return (uint32_t)(xe - 1) >= (uint32_t)(xt + 1025) || xe < xt + xd - 1020;
 }
 
 // Wilkinson shift from the trailing 2x2 block [a c; c b] (src/bulge_chasing.jl:239-265), by a
@@ -348,7 +356,7 @@ __device__ __forceinline__ int64_t block_start(const double* dv, const double* e
                                                double tol)
 {
     const int lane = threadIdx.x & 31;
-    const int32_t xt = (__double2hiint(tol) >> 20) & 0x7FF;
+    const int32_t xt = tol_exponent(tol);
     for (int64_t base = to - 1; base >= start; base -= 32 * kScanUnroll) {
         bool may[kScanUnroll];
 #pragma unroll
