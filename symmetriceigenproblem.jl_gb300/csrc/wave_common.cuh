@@ -244,6 +244,15 @@ struct Staging {
 // tile to Q is first checked against the pass's extent (rows [0, m), columns [0, n_loc)); an
 // access outside it is skipped and sets bit 1 (value 2) of the kernel's error word, which the
 // host reports as SYMEIG_ERR_DEVICE.  The default build compiles the checks away.
+// Whether the element at offset `off` of Q is one of rows [0, m), columns [0, n), element (row, col)
+// being at row * rs + col * ldq with rs or ldq 1: decoded from the offset alone, so that it tests
+// the address of an access and not the index it was meant to have.
+__host__ __device__ inline bool offset_in_extent(int64_t off, int64_t ldq, int64_t rs, int64_t m, int64_t n)
+{
+    if (off < 0) return false;
+    const int64_t col = rs == 1 ? off / ldq : off % rs, row = rs == 1 ? off % ldq : off / rs;
+    return row < m && col < n;
+}
 #ifdef SYMEIG_DEVICE_CHECKS
 __device__ __forceinline__ bool index_ok(int* check, bool ok)
 {

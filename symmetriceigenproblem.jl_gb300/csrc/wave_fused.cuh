@@ -16,7 +16,7 @@
 // share of the rows needs (kSms), in the fewest equal rounds when that exceeds what fits
 // (max_warps), so no SM carries more rows than another by more than one warp.
 //
-// KB and G are chosen per pass (fused_shape): the layers of a pass are padded to G * KB with KB
+// KB and G are chosen per pass (choose, apply_fused.cuh): the layers of a pass are padded to G * KB with KB
 // even (or, FP64, 1), not to 64, and a short Q takes more lane groups (32 / G rows per warp).
 //
 // FP64 (SHIFT): the products run on the integer pipes (int_mul.cuh), about 1550 instructions per
@@ -180,10 +180,11 @@ __device__ __forceinline__ bool tile(T* __restrict__ Q, int64_t ldq, int64_t m, 
                 bulk_load(ring + b * S::CHUNK, table + (int64_t)(c_begin + b) * S::CHUNK, S::CHUNK, &bar[b]);
     }
     __syncthreads();
+    // checked builds test every address of Q that is read or written
 #ifdef SYMEIG_DEVICE_CHECKS
-    auto in_extent = [&](bool ok) { return wave::index_ok(check, ok); };
+    auto in_extent = [&](const T* p) { return wave::index_ok(check, wave::offset_in_extent(p - Q, ldq, rs, m, n)); };
 #else
-    auto in_extent = [](bool) { return true; };
+    auto in_extent = [](const T*) { return true; };
 #endif
     const int64_t row = row0 + (int64_t)(tid >> 5) * RPW + rl;
     const bool row_ok = row < m;
@@ -198,7 +199,10 @@ __device__ __forceinline__ bool tile(T* __restrict__ Q, int64_t ldq, int64_t m, 
 #pragma unroll
         for (int a = 0; a < PD; ++a)
 #pragma unroll
-            for (int f = 0; f < F; ++f) ahead[a][f] = a * F + f < n ? q0[(int64_t)(a * F + f) * ldq] : T(0);
+            for (int f = 0; f < F; ++f) {
+                const T* p = q0 + (int64_t)(a * F + f) * ldq;
+                ahead[a][f] = a * F + f < n && in_extent(p) ? *p : T(0);
+            }
     } else {
         const T* s = state + tid;   // value-major
         const int nt = blockDim.x;
@@ -232,7 +236,7 @@ __device__ __forceinline__ bool tile(T* __restrict__ Q, int64_t ldq, int64_t m, 
                     const T up = __shfl_up_sync(0xffffffffu, xout[f], RPW);
                     win[(KB + f + base) % W] = g == 0 ? ahead[a][f] : up;
                     T next = T(0);
-                    if (ld_col + f < n && in_extent(ld_col + f >= 0)) next = lp[f * ldq];
+                    if (ld_col + f < n && in_extent(lp + f * ldq)) next = lp[f * ldq];
                     ahead[a][f] = next;
                 }
                 ld_col += F;
@@ -242,7 +246,7 @@ __device__ __forceinline__ bool tile(T* __restrict__ Q, int64_t ldq, int64_t m, 
                 for (int f = 0; f < F; ++f) {
                     xout[f] = win[(f + base) % W];
                     const bool in = storer && (uint32_t)(st_col + f) < (uint32_t)n;
-                    st_pred(sp + f * ldq, xout[f], in && in_extent(!in || st_col + f < n));
+                    st_pred(sp + f * ldq, xout[f], in && in_extent(sp + f * ldq));
                 }
                 st_col += F;
                 sp += F * ldq;
