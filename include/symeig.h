@@ -121,7 +121,8 @@ int symeig_set_apply_form(symeig_handle h, int32_t form);
  * entry points return SYMEIG_ERR_TIMEOUT (device_errors = 1 in the statistics).  In chase
  * mode 3 the first bulge of each batch also stops releasing its progress, so the next bulge's
  * wait runs out the same way.  Q (and, in mode 3, H) is then unspecified; the handle and the
- * context stay usable.  0 (default) turns it off. */
+ * context stay usable.  The adjoint's sliced products stop copying operand tiles from that one on
+ * (waits of about 1 s); its gradients stay right, by the FP64 MMA, and the error is reported.  0 (default) turns it off. */
 int symeig_set_test_stall(symeig_handle h, int32_t chunk);
 /* Record CUDA events around every wave-kernel launch so symeig_get_stats can report their
  * device time (wave_kernel_ms).  Off by default.  symeig_get_stats waits for the last
@@ -268,6 +269,9 @@ int symeig_eig_adjoint_f64(symeig_handle h, int64_t count, int64_t n, const doub
 int symeig_eig_adjoint_f64_dev(symeig_handle h, int64_t count, int64_t n, const double* lam,
                                const double* Q, const double* glam, const double* gQ, double* gd,
                                double* ge);
+/* Waits for the device and returns how many matrices of the handle's last call, an adjoint, ran on
+ * the bf16 slices. */
+int symeig_adjoint_sliced(symeig_handle h, int64_t* count);
 
 /* ---- bulk apply without any allocation -------------------------------------------------- *
  * No counterpart in the reference.  For callers that cannot allocate device memory at call

@@ -77,6 +77,7 @@ SIGNATURES = {
     "symeig_apply_tuning": (ctypes.c_int, [c_i32, P_i32, c_i32]),
     "symeig_eig_adjoint_f64": (ctypes.c_int, [c_vp, c_i64, c_i64, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp]),
     "symeig_eig_adjoint_f64_dev": (ctypes.c_int, [c_vp, c_i64, c_i64, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp]),
+    "symeig_adjoint_sliced": (ctypes.c_int, [c_vp, P_i64]),
     "symeig_eigen_decomp_f64": (ctypes.c_int, [c_vp, c_vp, c_vp, c_i64, c_vp, c_i64, P_i32, P_i64]),
 }
 
@@ -173,6 +174,12 @@ class Handle:
         s = Stats()
         check("symeig_get_stats", self._lib.symeig_get_stats(self.ptr, ctypes.byref(s)))
         return s.as_dict()
+
+    def adjoint_sliced(self) -> int:
+        """Matrices of the last call, an eig_adjoint, whose products ran on bf16 slices."""
+        c = c_i64()
+        check("symeig_adjoint_sliced", self._lib.symeig_adjoint_sliced(self.ptr, ctypes.byref(c)))
+        return c.value
 
     def set_kernel_timing(self, on: bool):
         check("symeig_set_kernel_timing", self._lib.symeig_set_kernel_timing(self.ptr, int(bool(on))))

@@ -143,11 +143,13 @@ adjoint_p_kernel(const double* __restrict__ Q, int64_t ldq, const double* __rest
 }
 
 // 3. dd_i = sum_tiles part0[i];  de_i = sum_tiles (part1[i] + part2[i+1]).
-// part holds the FP64 MMA's column tiles, or with `fallback` given and clear the sliced kernel's.
+// part holds the FP64 MMA's column tiles, or with `fallback` given and clear the sliced kernel's (counted).
 __global__ void adjoint_reduce_kernel(const double* __restrict__ part, int64_t n, double* __restrict__ gd,
-                                      double* __restrict__ ge, int64_t stridePart, const int* __restrict__ fallback)
+                                      double* __restrict__ ge, int64_t stridePart, const int* __restrict__ fallback,
+                                      int* __restrict__ sliced_count)
 {
     const int64_t z = blockIdx.y;
+    if (fallback && blockIdx.x == 0 && threadIdx.x == 0 && !fallback[z]) atomicAdd(sliced_count, 1);
     part += z * stridePart;
     gd += z * n;
     ge += z * (n > 1 ? n - 1 : 0);
@@ -170,7 +172,7 @@ __global__ void adjoint_reduce_kernel(const double* __restrict__ part, int64_t n
 __global__ void __launch_bounds__(sliced::kThreads, 1)
 sliced_m_check_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B, const int* __restrict__ ea,
                       const int* __restrict__ eb, int64_t n, int64_t rows, int64_t kp, int64_t pstride, float need,
-                      int* __restrict__ fallback)
+                      int* __restrict__ fallback, sliced::Report report)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
     const int64_t z = blockIdx.z;
@@ -178,7 +180,11 @@ sliced_m_check_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* 
     if (__syncthreads_or(skip)) return;
     const int64_t i0 = (int64_t)blockIdx.y * sliced::BM, j0 = (int64_t)blockIdx.x * sliced::BN;
     float L[64];
-    bool poor = !sliced::tile_product<true>(A + z * pstride, B + z * pstride, rows, kp, i0, j0, smem, nullptr, L);
+    bool poor = false;
+    if (!sliced::tile_product<true>(A + z * pstride, B + z * pstride, rows, kp, i0, j0, smem, nullptr, L, report.stall)) {
+        if (threadIdx.x == 0) report.timeout(fallback[z]);
+        return;
+    }
     const int64_t i = i0 + sliced::tile_row();
     if (threadIdx.x < sliced::kEpiThreads && i < n && ea[z * n + i] != sliced::kZeroScale) {
 #pragma unroll
@@ -202,7 +208,7 @@ __global__ void __launch_bounds__(sliced::kThreads, 1)
 sliced_p_check_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B, const int* __restrict__ ea,
                       const int* __restrict__ eb, const double* __restrict__ Q, int64_t n, int64_t rows, int64_t kp,
                       int64_t pstride, float need, double* __restrict__ margin, int64_t stride_margin,
-                      int* __restrict__ done, int* __restrict__ fallback)
+                      int* __restrict__ done, int* __restrict__ fallback, sliced::Report report)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ float red[3][2][sliced::BM], scale[sliced::BN];
@@ -224,7 +230,10 @@ sliced_p_check_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* 
     bool poor = e != sliced::kZeroScale && e < top - 60;
     if (threadIdx.x < sliced::BN) scale[threadIdx.x] = e == sliced::kZeroScale || poor ? 0.0f : exp2f((float)(e - top));
     float L[64];
-    if (!sliced::tile_product<true>(A + z * pstride, B + z * pstride, rows, kp, i0, k0, smem, nullptr, L)) poor = true;
+    if (!sliced::tile_product<true>(A + z * pstride, B + z * pstride, rows, kp, i0, k0, smem, nullptr, L, report.stall)) {
+        if (threadIdx.x == 0) report.timeout(fallback[z]);
+        return;
+    }
     if (__syncthreads_or(poor)) {
         if (threadIdx.x == 0) fallback[z] = 1;
         return;
@@ -286,7 +295,7 @@ __global__ void __launch_bounds__(sliced::kThreads, 1)
 sliced_m_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B, const int* __restrict__ ea,
                 const int* __restrict__ eb, const double* __restrict__ lam, const double* __restrict__ glam, int64_t n,
                 int64_t rows, int64_t kp, int64_t pstride, double* __restrict__ Mout, double* __restrict__ park,
-                int* __restrict__ fallback)
+                int* __restrict__ fallback, sliced::Report report)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
     const int64_t z = blockIdx.z;
@@ -298,8 +307,8 @@ sliced_m_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __rest
     park += ((z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * sliced::BM * sliced::BN;
     const int64_t i0 = (int64_t)blockIdx.y * sliced::BM, j0 = (int64_t)blockIdx.x * sliced::BN;
     double acc[64];
-    if (!sliced::tile_product<false>(A + z * pstride, B + z * pstride, rows, kp, i0, j0, smem, park, acc)) {
-        if (threadIdx.x == 0) fallback[z] = 1;
+    if (!sliced::tile_product<false>(A + z * pstride, B + z * pstride, rows, kp, i0, j0, smem, park, acc, report.stall)) {
+        if (threadIdx.x == 0) report.timeout(fallback[z]);
         return;
     }
     const int64_t i = i0 + sliced::tile_row();
@@ -326,7 +335,7 @@ __global__ void __launch_bounds__(sliced::kThreads, 1)
 sliced_p_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B, const int* __restrict__ ea,
                 const int* __restrict__ eb, const double* __restrict__ Q, int64_t n, int64_t rows, int64_t kp,
                 int64_t pstride, double* __restrict__ part, int64_t stridePart, double* __restrict__ park,
-                int* __restrict__ fallback)
+                int* __restrict__ fallback, sliced::Report report)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ double red[3][2][sliced::BM];
@@ -338,8 +347,8 @@ sliced_p_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __rest
     park += ((z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * sliced::BM * sliced::BN;
     const int64_t i0 = (int64_t)blockIdx.y * sliced::BM, k0 = (int64_t)blockIdx.x * sliced::BN;
     double acc[64];
-    if (!sliced::tile_product<false>(A + z * pstride, B + z * pstride, rows, kp, i0, k0, smem, park, acc)) {
-        if (threadIdx.x == 0) fallback[z] = 1;
+    if (!sliced::tile_product<false>(A + z * pstride, B + z * pstride, rows, kp, i0, k0, smem, park, acc, report.stall)) {
+        if (threadIdx.x == 0) report.timeout(fallback[z]);
         return;
     }
     const int r = sliced::tile_row();
@@ -437,9 +446,10 @@ static int64_t sliced_scratch_doubles(int64_t count, int64_t n)
 // Device-pointer adjoint for `count` matrices of order n stored back to back (Q, gQ with
 // leading dimension n and stride n*n; lam, glam, gd with stride n; ge with stride n-1).
 // scratch: adjoint_scratch_doubles(count, n, use_sliced) doubles; use_sliced only where adjoint_sliced(n).
+// err[0]: the handle's error word; err[1] counts the matrices that took the slices.
 int adjoint_dev(cudaStream_t s, int64_t count, int64_t n, const double* lam, const double* Q,
                 const double* glam, const double* gQ, double* gd, double* ge, double* scratch,
-                bool use_sliced)
+                bool use_sliced, int* err, int32_t stall)
 {
     if (count <= 0 || n <= 0) return SYMEIG_OK;
     const int64_t tiles = (n + BN - 1) / BN;
@@ -456,13 +466,14 @@ int adjoint_dev(cudaStream_t s, int64_t count, int64_t n, const double* lam, con
     if (!use_sliced) {
         adjoint_m_kernel<<<grid, kAdjThreads, 0, s>>>(Q, n, gQ, n, lam, glam, n, Mbuf, strideQ, strideQ, strideM, nullptr);
         adjoint_p_kernel<<<grid, kAdjThreads, 0, s>>>(Q, n, Mbuf, n, part, strideQ, strideM, stridePart, nullptr);
-        adjoint_reduce_kernel<<<dim3((unsigned)((n + 255) / 256), (unsigned)count), 256, 0, s>>>(part, n, gd, ge, stridePart, nullptr);
+        adjoint_reduce_kernel<<<dim3((unsigned)((n + 255) / 256), (unsigned)count), 256, 0, s>>>(part, n, gd, ge, stridePart, nullptr, nullptr);
         return cudaGetLastError() == cudaSuccess ? SYMEIG_OK : SYMEIG_ERR_CUDA;
     }
     for (const void* k : {(const void*)sliced_m_kernel, (const void*)sliced_p_kernel, (const void*)sliced_m_check_kernel,
                           (const void*)sliced_p_check_kernel})
         if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sliced::kSmem) != cudaSuccess)
             return SYMEIG_ERR_CUDA;
+    const sliced::Report report{err, stall > 0 ? (uint32_t)stall : 0xffffffffu};
     const int64_t group = sliced_group(count, n), rows = sliced::pad_rows(n), kp = sliced::pad_k(n);
     const int64_t pstride = sliced::plane_values(n, n);
     // 256-byte aligned: the planes' 16-byte pieces
@@ -487,8 +498,8 @@ int adjoint_dev(cudaStream_t s, int64_t count, int64_t n, const double* lam, con
         if (cudaMemsetAsync(flag, 0, group * (1 + ntiles) * sizeof(int), s) != cudaSuccess) return SYMEIG_ERR_CUDA;
         sliced::column_exponents_kernel<<<dim3((unsigned)n, g, 2), 256, 0, s>>>(oq, og, n, flag);
         sliced::slice_columns_kernel<<<dim3(cgrid.x, cgrid.y, 2 * g), 256, 0, s>>>(oq, og, (int)g, n, rows, kp, pstride, flag);
-        sliced_m_check_kernel<<<sgrid, sliced::kThreads, sliced::kSmem, s>>>(PA, PB, ea, eb, n, rows, kp, pstride, need, flag);
-        sliced_m_kernel<<<sgrid, sliced::kThreads, sliced::kSmem, s>>>(PA, PB, ea, eb, lz, glz, n, rows, kp, pstride, Mz, park, flag);
+        sliced_m_check_kernel<<<sgrid, sliced::kThreads, sliced::kSmem, s>>>(PA, PB, ea, eb, n, rows, kp, pstride, need, flag, report);
+        sliced_m_kernel<<<sgrid, sliced::kThreads, sliced::kSmem, s>>>(PA, PB, ea, eb, lz, glz, n, rows, kp, pstride, Mz, park, flag, report);
         adjoint_m_kernel<<<fgrid, kAdjThreads, 0, s>>>(Qz, n, Gz, n, lz, glz, n, Mz, strideQ, strideQ, strideM, flag);
         sliced::row_exponents_kernel<<<dim3((unsigned)((n + 31) / 32), g), 1024, 0, s>>>(Qz, n, ea, flag);
         sliced::column_exponents_kernel<<<dim3((unsigned)n, g, 1), 256, 0, s>>>(om, om, n, flag);
@@ -497,10 +508,10 @@ int adjoint_dev(cudaStream_t s, int64_t count, int64_t n, const double* lam, con
         sliced::slice_columns_kernel<<<cgrid, 256, 0, s>>>(om, om, (int)g, n, rows, kp, pstride, flag);
         // (pz: the margins, before the partial sums take their place)
         sliced_p_check_kernel<<<sgrid, sliced::kThreads, sliced::kSmem, s>>>(PA, PB, ea, eb, Qz, n, rows, kp, pstride, need, pz,
-                                                                            stridePart, done, flag);
-        sliced_p_kernel<<<sgrid, sliced::kThreads, sliced::kSmem, s>>>(PA, PB, ea, eb, Qz, n, rows, kp, pstride, pz, stridePart, park, flag);
+                                                                            stridePart, done, flag, report);
+        sliced_p_kernel<<<sgrid, sliced::kThreads, sliced::kSmem, s>>>(PA, PB, ea, eb, Qz, n, rows, kp, pstride, pz, stridePart, park, flag, report);
         adjoint_p_kernel<<<fgrid, kAdjThreads, 0, s>>>(Qz, n, Mz, n, pz, strideQ, strideM, stridePart, flag);
-        adjoint_reduce_kernel<<<dim3((unsigned)((n + 255) / 256), g), 256, 0, s>>>(pz, n, gd + z * n, gez, stridePart, flag);
+        adjoint_reduce_kernel<<<dim3((unsigned)((n + 255) / 256), g), 256, 0, s>>>(pz, n, gd + z * n, gez, stridePart, flag, err + 1);
     }
     return cudaGetLastError() == cudaSuccess ? SYMEIG_OK : SYMEIG_ERR_CUDA;
 }

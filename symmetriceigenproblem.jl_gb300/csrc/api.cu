@@ -66,7 +66,7 @@ struct symeig_context {
     // kernel done
     cudaEvent_t seg_in[kPipeBlocks] = {}, seg_done[kPipeBlocks] = {};
     DevBuf grid[2], thick[2], place[2], table, state, d, e, q, cs, bak, rot, dense, dense_io, bulge, seg_state;
-    int* derr = nullptr;   // device error word of the wave kernels (bounded waits)
+    int* derr = nullptr;   // device error word (bounded waits), and the adjoint's count of sliced matrices
     int32_t exact_order = 1;  // rotation placement of the qr driver
     int32_t chase_mode = 0;   // symeig_set_chase_mode
     int32_t apply_form = 0;   // symeig_set_apply_form
@@ -165,7 +165,7 @@ void begin_call(symeig_handle h)
     h->kused = 0;
     h->kpending = false;
     // the error word of the bounded waits reports on this call only
-    cudaMemsetAsync(h->derr, 0, sizeof(int), h->stream);
+    cudaMemsetAsync(h->derr, 0, 2 * sizeof(int), h->stream);
 }
 
 // After a synchronous call: SYMEIG_ERR_TIMEOUT if a wave kernel's bounded wait gave up.
@@ -711,8 +711,8 @@ int symeig_create(symeig_handle* out, int device)
     }
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_main, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaMallocHost((void**)&h->h_state, sizeof(ChaseState));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&h->derr, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(h->derr, 0, sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc((void**)&h->derr, 2 * sizeof(int));
+    if (e == cudaSuccess) e = cudaMemset(h->derr, 0, 2 * sizeof(int));
     if (e != cudaSuccess) {
         symeig_destroy(h);
         return cuda_status(e);
@@ -1038,7 +1038,7 @@ int symeig_eig_adjoint_f64_dev(symeig_handle h, int64_t count, int64_t n, const 
     }
     if (gQ && !use_sliced) CK(h->cs.ensure((size_t)adjoint_scratch_doubles(count, n, false) * sizeof(double)));
     auto t0 = std::chrono::steady_clock::now();
-    rc = adjoint_dev(h->stream, count, n, lam, Q, glam, gQ, gd, ge, (double*)h->cs.ptr, use_sliced);
+    rc = adjoint_dev(h->stream, count, n, lam, Q, glam, gQ, gd, ge, (double*)h->cs.ptr, use_sliced, h->derr, h->test_stall);
     h->stats.total_ms =
         std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     return rc;
@@ -1074,6 +1074,18 @@ int symeig_eig_adjoint_f64(symeig_handle h, int64_t count, int64_t n, const doub
     CK(cudaMemcpyAsync(gd, dgd, nv * sizeof(double), cudaMemcpyDeviceToHost, s));
     if (ne) CK(cudaMemcpyAsync(ge, dge, ne * sizeof(double), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
+    return check_device_error(h);
+}
+
+int symeig_adjoint_sliced(symeig_handle h, int64_t* count)
+{
+    int rc = check_handle(h);
+    if (rc) return rc;
+    if (!count) return SYMEIG_ERR_NULL;
+    int c = 0;
+    CK(cudaDeviceSynchronize());
+    CK(cudaMemcpy(&c, h->derr + 1, sizeof(int), cudaMemcpyDeviceToHost));
+    *count = c;
     return SYMEIG_OK;
 }
 

@@ -341,6 +341,18 @@ struct Control {
     int failed;
 };
 
+// Where a wait that ran out is reported (the handle's error word) and the test hook.
+struct Report {
+    int* err;
+    uint32_t stall;   // tiles copied before the copies stop
+    // the FP64 MMA takes the matrix
+    __device__ __forceinline__ void timeout(int& fallback) const
+    {
+        fallback = 1;
+        atomicOr(err, 1);
+    }
+};
+
 // Waits for the phase of `parity`, for about a second at most (failure: false, for every warp).
 __device__ __forceinline__ bool wait(Control& c, uint64_t* b, uint32_t parity)
 {
@@ -363,16 +375,18 @@ __device__ __forceinline__ uint64_t operand_desc(uint32_t addr)
            (uint64_t)2 << 61;
 }
 
-// The copying thread: all tiles of the passes, in order.  Returns once what it started has landed.
+// The copying thread: all tiles of the passes, in order.  Returns once what it started has landed.  `stall`
+// (the test hook): tiles from that one on are not copied, so that the waits for them run out.
 template <bool LEAD>
 __device__ __forceinline__ void copy_tiles(Control& c, uint32_t tiles, const __nv_bfloat16* A, const __nv_bfloat16* B,
-                                           int64_t plane, int blocks)
+                                           int64_t plane, int blocks, uint32_t stall)
 {
     uint32_t g = 0;
     bool ok = true;
     auto load = [&](const __nv_bfloat16* src) {
         const uint32_t slot = g % kSlots, turn = g / kSlots;
-        if (turn > 0) ok = wait(c, &c.empty[slot], (turn - 1) & 1);
+        if (g >= stall) ok = false;
+        else if (turn > 0) ok = wait(c, &c.empty[slot], (turn - 1) & 1);
         if (!ok) return;
         mbar_expect(&c.full[slot], kTileBytes);
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
@@ -495,7 +509,7 @@ __device__ __forceinline__ void issue_products(Control& c, uint32_t tiles, uint3
 template <bool LEAD, typename Out>
 __device__ __forceinline__ bool tile_product(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B,
                                              int64_t rows, int64_t kp, int64_t i0, int64_t j0, unsigned char* smem,
-                                             double* __restrict__ park, Out (&out)[64])
+                                             double* __restrict__ park, Out (&out)[64], uint32_t stall)
 {
     __shared__ Control c;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -527,7 +541,8 @@ __device__ __forceinline__ bool tile_product(const __nv_bfloat16* __restrict__ A
     const uint32_t tmem = c.tmem;
     if (warp == 8) {
         if (lane == 0)
-            copy_tiles<LEAD>(c, tiles, A + i0 / BM * (kp / BK) * kTileValues, B + j0 / BN * (kp / BK) * kTileValues, plane, blocks);
+            copy_tiles<LEAD>(c, tiles, A + i0 / BM * (kp / BK) * kTileValues, B + j0 / BN * (kp / BK) * kTileValues, plane, blocks,
+                             stall);
         __syncwarp();
     } else if (warp == 9) {
         if (lane == 0) issue_products<LEAD>(c, tiles, tmem, blocks);
