@@ -170,12 +170,13 @@ __global__ void adjoint_reduce_kernel(const double* __restrict__ part, int64_t n
 // Before 1.: whether the slices keep FP64's accuracy in every entry of Q^T gQ (sliced_gemm.cuh; a column
 // of zeros is exact, and M's diagonal takes none).  `need`: the least L.
 __global__ void __launch_bounds__(sliced::kThreads, 1)
-sliced_m_check_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B, const int* __restrict__ ea,
-                      const int* __restrict__ eb, int64_t n, int64_t rows, int64_t kp, int64_t pstride, float need,
+sliced_m_check_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B, const int* ea,
+                      const int* eb, int64_t n, int64_t rows, int64_t kp, int64_t pstride, float need,
                       int* __restrict__ fallback, sliced::Report report)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
     const int64_t z = blockIdx.z;
+    wait_previous_launch();
     const bool skip = fallback[z] != 0;
     if (__syncthreads_or(skip)) return;
     const int64_t i0 = (int64_t)blockIdx.y * sliced::BM, j0 = (int64_t)blockIdx.x * sliced::BN;
@@ -205,8 +206,8 @@ sliced_m_check_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* 
 // about the tile's largest column, on the safe side: a weight below 2^-60 of its row's largest counts as
 // 2^-60 against and as 0 for the slices, and a column below 2^-60 of the tile's largest fails.
 __global__ void __launch_bounds__(sliced::kThreads, 1)
-sliced_p_check_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B, const int* __restrict__ ea,
-                      const int* __restrict__ eb, const double* __restrict__ Q, int64_t n, int64_t rows, int64_t kp,
+sliced_p_check_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B, const int* ea,
+                      const int* eb, const double* __restrict__ Q, int64_t n, int64_t rows, int64_t kp,
                       int64_t pstride, float need, double* __restrict__ margin, int64_t stride_margin,
                       int* __restrict__ done, int* __restrict__ fallback, sliced::Report report)
 {
@@ -214,6 +215,7 @@ sliced_p_check_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* 
     __shared__ float red[3][2][sliced::BM], scale[sliced::BN];
     __shared__ int top, last;
     const int64_t z = blockIdx.z;
+    wait_previous_launch();
     const bool skip = fallback[z] != 0;
     if (__syncthreads_or(skip)) return;
     Q += z * n * n;
@@ -292,13 +294,14 @@ sliced_p_check_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* 
 
 // 1. as adjoint_m_kernel.  A: planes of Q's columns with exponents ea; B: of gQ's columns with eb.
 __global__ void __launch_bounds__(sliced::kThreads, 1)
-sliced_m_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B, const int* __restrict__ ea,
-                const int* __restrict__ eb, const double* __restrict__ lam, const double* __restrict__ glam, int64_t n,
+sliced_m_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B, const int* ea,
+                const int* eb, const double* __restrict__ lam, const double* __restrict__ glam, int64_t n,
                 int64_t rows, int64_t kp, int64_t pstride, double* __restrict__ Mout, double* __restrict__ park,
                 int* __restrict__ fallback, sliced::Report report)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
     const int64_t z = blockIdx.z;
+    wait_previous_launch();
     const bool skip = fallback[z] != 0;
     if (__syncthreads_or(skip)) return;
     lam += z * n;
@@ -332,14 +335,15 @@ sliced_m_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __rest
 
 // 2. as adjoint_p_kernel.  A: planes of Q's rows with exponents ea; B: of M's columns with eb.
 __global__ void __launch_bounds__(sliced::kThreads, 1)
-sliced_p_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B, const int* __restrict__ ea,
-                const int* __restrict__ eb, const double* __restrict__ Q, int64_t n, int64_t rows, int64_t kp,
+sliced_p_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B, const int* ea,
+                const int* eb, const double* __restrict__ Q, int64_t n, int64_t rows, int64_t kp,
                 int64_t pstride, double* __restrict__ part, int64_t stridePart, double* __restrict__ park,
                 int* __restrict__ fallback, sliced::Report report)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ double red[3][2][sliced::BM];
     const int64_t z = blockIdx.z;
+    wait_previous_launch();
     const bool skip = fallback[z] != 0;
     if (__syncthreads_or(skip)) return;
     Q += z * n * n;
@@ -435,12 +439,13 @@ static int64_t sliced_group(int64_t count, int64_t n)
     return std::max<int64_t>(1, std::min(std::min<int64_t>(count, 32767), kSlicedBytes / per));
 }
 
-// The scratch after M and the partials: two operands' planes, the tiles' small sums, the operands' exponents, a
-// flag a matrix and a counter a row of tiles.
+// The scratch after M and the partials: of a group two operands' planes and the tiles' small sums; of all matrices the
+// operands' exponents, a flag and a counter a row of tiles.
 static int64_t sliced_scratch_doubles(int64_t count, int64_t n)
 {
     const int64_t g = sliced_group(count, n), r = sliced::pad_rows(n);
-    return g * (2 * sliced::plane_values(n, n) * 2 + r * r * (int64_t)sizeof(double) + (2 * n + 1 + r / sliced::BM) * (int64_t)sizeof(int)) / 8 + 64;
+    return (g * (2 * sliced::plane_values(n, n) * 2 + r * r * (int64_t)sizeof(double)) +
+            count * (2 * n + 1 + r / sliced::BM) * (int64_t)sizeof(int)) / 8 + 64;
 }
 
 // Device-pointer adjoint for `count` matrices of order n stored back to back (Q, gQ with
@@ -481,38 +486,52 @@ int adjoint_dev(cudaStream_t s, int64_t count, int64_t n, const double* lam, con
     __nv_bfloat16* PA = (__nv_bfloat16*)base;
     __nv_bfloat16* PB = PA + group * pstride;
     double* park = (double*)(PB + group * pstride);
-    int* ea = (int*)(park + group * rows * rows);
-    int* eb = ea + group * n;
-    int* flag = eb + group * n;
+    int* ea = (int*)(park + group * rows * rows);   // from here on of all matrices
+    int* eb = ea + count * n;
+    int* flag = eb + count * n;
+    int* done = flag + count;
     const int64_t ntiles = (n + sliced::BN - 1) / sliced::BN;
-    int* done = flag + group;
     const float need = (float)(sliced::kLeadFactor * std::sqrt((double)n));
+    const unsigned all = (unsigned)count;
+    const unsigned kblocks = (unsigned)((kp / 8 + 255) / 256);
+    // The FP64 MMA takes the matrices that fall back in one launch each, whatever the groups: by groups the last waves of
+    // their tiles cost 3 % of 256 matrices of n = 512.  In a chain (launch_after) the launches that return at
+    // once overlap.
+    if (cudaMemsetAsync(flag, 0, count * (1 + ntiles) * sizeof(int), s) != cudaSuccess) return SYMEIG_ERR_CUDA;
+    sliced::column_exponents_kernel<<<dim3((unsigned)n, all, 2), 256, 0, s>>>(sliced::Operand{Q, ea, PA, true},
+                                                                            sliced::Operand{gQ, eb, PB, false}, n, flag);
     for (int64_t z = 0; z < count; z += group) {
         const unsigned g = (unsigned)std::min<int64_t>(group, count - z);
-        const double *Qz = Q + z * strideQ, *Gz = gQ + z * strideQ, *lz = lam + z * n, *glz = glam + z * n;
-        double *Mz = Mbuf + z * strideM, *pz = part + z * stridePart;
-        double* gez = ge ? ge + z * (n - 1) : nullptr;
-        const dim3 fgrid(grid.x, grid.y, g), sgrid((unsigned)ntiles, (unsigned)ntiles, g);
-        const dim3 cgrid((unsigned)((kp / 8 + 255) / 256), (unsigned)rows, g);
-        const sliced::Operand oq{Qz, ea, PA, true}, og{Gz, eb, PB, false}, om{Mz, eb, PB, false};
-        if (cudaMemsetAsync(flag, 0, group * (1 + ntiles) * sizeof(int), s) != cudaSuccess) return SYMEIG_ERR_CUDA;
-        sliced::column_exponents_kernel<<<dim3((unsigned)n, g, 2), 256, 0, s>>>(oq, og, n, flag);
-        sliced::slice_columns_kernel<<<dim3(cgrid.x, cgrid.y, 2 * g), 256, 0, s>>>(oq, og, (int)g, n, rows, kp, pstride, flag);
-        sliced_m_check_kernel<<<sgrid, sliced::kThreads, sliced::kSmem, s>>>(PA, PB, ea, eb, n, rows, kp, pstride, need, flag, report);
-        sliced_m_kernel<<<sgrid, sliced::kThreads, sliced::kSmem, s>>>(PA, PB, ea, eb, lz, glz, n, rows, kp, pstride, Mz, park, flag, report);
-        adjoint_m_kernel<<<fgrid, kAdjThreads, 0, s>>>(Qz, n, Gz, n, lz, glz, n, Mz, strideQ, strideQ, strideM, flag);
-        sliced::row_exponents_kernel<<<dim3((unsigned)((n + 31) / 32), g), 1024, 0, s>>>(Qz, n, ea, flag);
-        sliced::column_exponents_kernel<<<dim3((unsigned)n, g, 1), 256, 0, s>>>(om, om, n, flag);
-        sliced::slice_rows_kernel<<<dim3((unsigned)((kp + 63) / 64), (unsigned)((rows + 31) / 32), g), 256, 0, s>>>(
-            Qz, n, ea, rows, kp, PA, pstride, flag);
-        sliced::slice_columns_kernel<<<cgrid, 256, 0, s>>>(om, om, (int)g, n, rows, kp, pstride, flag);
-        // (pz: the margins, before the partial sums take their place)
-        sliced_p_check_kernel<<<sgrid, sliced::kThreads, sliced::kSmem, s>>>(PA, PB, ea, eb, Qz, n, rows, kp, pstride, need, pz,
-                                                                            stridePart, done, flag, report);
-        sliced_p_kernel<<<sgrid, sliced::kThreads, sliced::kSmem, s>>>(PA, PB, ea, eb, Qz, n, rows, kp, pstride, pz, stridePart, park, flag, report);
-        adjoint_p_kernel<<<fgrid, kAdjThreads, 0, s>>>(Qz, n, Mz, n, pz, strideQ, strideM, stridePart, flag);
-        adjoint_reduce_kernel<<<dim3((unsigned)((n + 255) / 256), g), 256, 0, s>>>(pz, n, gd + z * n, gez, stridePart, flag, err + 1);
+        const dim3 sgrid((unsigned)ntiles, (unsigned)ntiles, g);
+        launch_after(sliced::slice_columns_kernel, dim3(kblocks, (unsigned)rows, 2 * g), 256, 0, s,
+                     sliced::Operand{Q + z * strideQ, ea + z * n, PA, true}, sliced::Operand{gQ + z * strideQ, eb + z * n, PB, false},
+                     (int)g, n, rows, kp, pstride, flag + z);
+        launch_after(sliced_m_check_kernel, sgrid, sliced::kThreads, sliced::kSmem, s, PA, PB, ea + z * n, eb + z * n, n, rows, kp,
+                     pstride, need, flag + z, report);
+        launch_after(sliced_m_kernel, sgrid, sliced::kThreads, sliced::kSmem, s, PA, PB, ea + z * n, eb + z * n, lam + z * n,
+                     glam + z * n, n, rows, kp, pstride, Mbuf + z * strideM, park, flag + z, report);
     }
+    adjoint_m_kernel<<<grid, kAdjThreads, 0, s>>>(Q, n, gQ, n, lam, glam, n, Mbuf, strideQ, strideQ, strideM, flag);
+    launch_after(sliced::row_exponents_kernel, dim3((unsigned)((n + 31) / 32), all), 1024, 0, s, Q, n, ea, flag);
+    const sliced::Operand om{Mbuf, eb, PB, false};
+    launch_after(sliced::column_exponents_kernel, dim3((unsigned)n, all, 1), 256, 0, s, om, om, n, flag);
+    for (int64_t z = 0; z < count; z += group) {
+        const unsigned g = (unsigned)std::min<int64_t>(group, count - z);
+        const dim3 sgrid((unsigned)ntiles, (unsigned)ntiles, g);
+        const sliced::Operand oz{Mbuf + z * strideM, eb + z * n, PB, false};
+        double* pz = part + z * stridePart;
+        launch_after(sliced::slice_rows_kernel, dim3((unsigned)((kp + 63) / 64), (unsigned)((rows + 31) / 32), g), 256, 0, s,
+                     Q + z * strideQ, n, ea + z * n, rows, kp, PA, pstride, flag + z);
+        launch_after(sliced::slice_columns_kernel, dim3(kblocks, (unsigned)rows, g), 256, 0, s, oz, oz, (int)g, n, rows, kp, pstride,
+                     flag + z);
+        // (pz: the margins, before the partial sums take their place)
+        launch_after(sliced_p_check_kernel, sgrid, sliced::kThreads, sliced::kSmem, s, PA, PB, ea + z * n, eb + z * n,
+                     Q + z * strideQ, n, rows, kp, pstride, need, pz, stridePart, done + z * ntiles, flag + z, report);
+        launch_after(sliced_p_kernel, sgrid, sliced::kThreads, sliced::kSmem, s, PA, PB, ea + z * n, eb + z * n, Q + z * strideQ, n,
+                     rows, kp, pstride, pz, stridePart, park, flag + z, report);
+    }
+    adjoint_p_kernel<<<grid, kAdjThreads, 0, s>>>(Q, n, Mbuf, n, part, strideQ, strideM, stridePart, flag);
+    adjoint_reduce_kernel<<<dim3((unsigned)((n + 255) / 256), all), 256, 0, s>>>(part, n, gd, ge, stridePart, flag, err + 1);
     return cudaGetLastError() == cudaSuccess ? SYMEIG_OK : SYMEIG_ERR_CUDA;
 }
 

@@ -42,6 +42,8 @@
 // epilogue's FP64 division.
 #pragma once
 #include <cuda_bf16.h>
+
+#include "launch_after.cuh"
 #include <cstdint>
 
 namespace symeig {
@@ -144,6 +146,7 @@ struct Operand {
 static __global__ void __launch_bounds__(256)
 column_exponents_kernel(Operand o0, Operand o1, int64_t n, int* __restrict__ flag)
 {
+    wait_previous_launch();
     if (__syncthreads_or(flag[blockIdx.y])) return;
     __shared__ unsigned long long sh[8];
     __shared__ double ss[8];
@@ -181,6 +184,7 @@ column_exponents_kernel(Operand o0, Operand o1, int64_t n, int* __restrict__ fla
 static __global__ void __launch_bounds__(1024)
 row_exponents_kernel(const double* __restrict__ X, int64_t n, int* __restrict__ exps, int* __restrict__ flag)
 {
+    wait_previous_launch();
     if (__syncthreads_or(flag[blockIdx.y])) return;
     __shared__ unsigned long long sh[32][33];
     __shared__ double ss[32][33];
@@ -226,8 +230,10 @@ __device__ __forceinline__ int64_t plane_offset(int s, int64_t i, int64_t k0, in
 // blockIdx.z = matrix, from `count` on the second operand's.
 static __global__ void __launch_bounds__(256)
 slice_columns_kernel(Operand o0, Operand o1, int count, int64_t n, int64_t rows, int64_t kp, int64_t pstride,
-                     const int* __restrict__ flag)
+                     const int* flag)
 {
+    wait_previous_launch();
+    wait_previous_launch();
     const Operand& o = (int)blockIdx.z < count ? o0 : o1;
     const int64_t z = (int)blockIdx.z < count ? blockIdx.z : blockIdx.z - count;
     if (flag[z]) return;
@@ -255,8 +261,9 @@ slice_columns_kernel(Operand o0, Operand o1, int count, int64_t n, int64_t rows,
 // Planes of the rows of X (n x n): as slice_columns_kernel on the transpose, through a 32 x 64
 // shared tile.
 static __global__ void __launch_bounds__(256)
-slice_rows_kernel(const double* __restrict__ X, int64_t n, const int* __restrict__ exps, int64_t rows, int64_t kp, __nv_bfloat16* __restrict__ planes, int64_t pstride,
-                  const int* __restrict__ flag)
+slice_rows_kernel(const double* __restrict__ X, int64_t n, const int* exps, int64_t rows, int64_t kp,
+                  __nv_bfloat16* __restrict__ planes, int64_t pstride,
+                  const int* flag)
 {
     if (flag[blockIdx.z]) return;
     __shared__ double tile[64][33];   // [inner][row]

@@ -35,6 +35,7 @@
 #include <cuda_runtime.h>
 
 #include "dmma_tile.cuh"
+#include "launch_after.cuh"
 #include "symeig.h"
 #include "symeig_common.cuh"
 
@@ -74,29 +75,6 @@ __device__ __forceinline__ double warp_sum_of(const double* __restrict__ a, int 
     }
     if (k < n) s0 += a[k];
     return warp_sum(s0 + s1);
-}
-
-// Programmatic dependent launch: a column kernel's blocks may be resident before the launch ahead
-// has finished; they read nothing until it has completed.
-__device__ __forceinline__ void wait_previous_launch()
-{
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
-template <typename... Params, typename... Args>
-void launch_after(void (*kernel)(Params...), dim3 grid, int threads, cudaStream_t s, Args... args)
-{
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.stream = s;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
 }
 
 // The scratch of one panel, shared by the column kernels.
@@ -200,7 +178,7 @@ products_kernel(Panel P, int64_t j, int i, int nparts, int chunks, double* __res
     wait_previous_launch();
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     const int64_t n = P.n, m = n - j - 1;
-    const double* __restrict__ col = P.A + j * P.lda;
+    const double* col = P.A + j * P.lda;
     if (wp == 0) {
         const double s = warp_sum_of(P.part, nparts);
         double tau, scale, beta;
@@ -225,7 +203,7 @@ products_kernel(Panel P, int64_t j, int i, int nparts, int chunks, double* __res
         // dot products: the blocks' warps over t = 0 .. 2 i - 1
         const int first = ((int)(blockIdx.y - chunks) * (int)gridDim.x + (int)blockIdx.x) * (2 * SR / 32) + wp;
         for (int t = first; t < 2 * i; t += (int)(gridDim.y - chunks) * (int)gridDim.x * (2 * SR / 32)) {
-            const double* __restrict__ x = P.VW + (int64_t)(t < i ? t : P.pb + t - i) * n;
+            const double* x = P.VW + (int64_t)(t < i ? t : P.pb + t - i) * n;
             double s0 = lane == 0 ? x[j + 1] : 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
             int64_t r = j + 2 + lane;
             for (; r + 96 < n; r += 128) {
@@ -249,7 +227,7 @@ products_kernel(Panel P, int64_t j, int i, int nparts, int chunks, double* __res
     const int64_t r = j + 1 + (int64_t)blockIdx.x * SR + rl;
     double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
     if (r < n) {
-        const double* __restrict__ a = P.A + r + c0 * P.lda;
+        const double* a = P.A + r + c0 * P.lda;
         int c = h * (gch / 2);
         const int end = min(len, c + gch / 2);
 #pragma unroll 4
@@ -666,12 +644,12 @@ int sytrd_dev(cudaStream_t s, int64_t n, double* A, int64_t lda, double* d, doub
             const unsigned chunks = blocks_for(m, symv_cols(m));
             // blocks for the 2 i dot products beside the chunks'
             const unsigned extra = i > 0 ? blocks_for(blocks_for(2 * i, 2 * SR / 32), (int)sr) : 0;
-            launch_after(column_kernel, dim3(blocks), RB * RG, s, P, j, i, (int)blocks, 0);
-            launch_after(products_kernel, dim3(sr, chunks + extra), 2 * SR, s, P, j, i, (int)blocks, (int)chunks, d, e, tau);
-            launch_after(w_kernel, dim3(blocks1), RB * RG, s, P, j, i, (int)chunks);
+            launch_after(column_kernel, dim3(blocks), RB * RG, 0, s, P, j, i, (int)blocks, 0);
+            launch_after(products_kernel, dim3(sr, chunks + extra), 2 * SR, 0, s, P, j, i, (int)blocks, (int)chunks, d, e, tau);
+            launch_after(w_kernel, dim3(blocks1), RB * RG, 0, s, P, j, i, (int)chunks);
         }
         const int64_t q = p + pb;
-        launch_after(column_kernel, dim3(blocks_for(n - q, RB)), RB * RG, s, P, q, pb, (int)blocks_for(n - q, RB), 1);
+        launch_after(column_kernel, dim3(blocks_for(n - q, RB)), RB * RG, 0, s, P, q, pb, (int)blocks_for(n - q, RB), 1);
         const unsigned t = blocks_for(n - q, dmma::BM);
         trailing_update_kernel<<<dim3(t, t), dmma::kThreads, 0, s>>>(A, lda, n, q, pb, P.VW, P.WV);
     }
