@@ -14,8 +14,8 @@ namespace symeig {
 
 __device__ __forceinline__ void wait_previous_launch()
 {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 template <typename... Params, typename... Args>
