@@ -418,21 +418,21 @@ __global__ void adjoint_lambda_only_kernel(const double* __restrict__ Q, int64_t
 }  // namespace
 
 // From this order on the products run on the bf16 tensor cores where Q is spread out.  FP64 MMA against
-// sliced, one matrix: n = 130 427 / 308 us, 256 700 / 324, 512 1314 / 407, 1024 4.78 / 0.61 ms, 2047 32.8 / 1.73,
-// 4096 252 / 10.0; 25 of n = 257 3226 / 752 us, 4 of 700 6590 / 573.  A localized Q pays for the question and the kernels
-// that return at once: 45 us of 810 at n = 300, 60 of 4700 at 1000, 100 us of 32.8 ms at 2047; below
-// n = 256 it would be above 6 %.  The rule leaves the count out, so that a matrix has the same bits
+// sliced, one matrix: n = 256 694 / 335 us, 300 810 / 354, 512 1304 / 428, 1000 4693 / 634, 2047 32.8 / 1.89 ms;
+// 25 of n = 300 3612 / 745 us, 256 of n = 512 127 / 13.6 ms.  A localized Q pays for the question and the kernels that return
+// at once: 20 us of 700 at n = 256, 24 of 810 at 300, 28 of 4690 at 1000, 0.6 ms of 127 for 256 of n = 512; below
+// n = 256 it would be above 3 %.  The rule leaves the count out, so that a matrix has the same bits
 // alone and in a batch.
 static constexpr int64_t kSlicedMin = 256;
 // Matrices sliced at once: their planes take at most this many bytes (one matrix always fits).
 static constexpr int64_t kSlicedBytes = (int64_t)512 << 20;
 
-// Above it the rows leave the grid's y range (slice_columns_kernel).
+// The planes of larger orders would take 160 GB and more.
 static constexpr int64_t kSlicedMax = 65408;
 
 bool adjoint_sliced(int64_t n) { return n >= kSlicedMin && n <= kSlicedMax; }
 
-// (and 32767 at most: blockIdx.z counts two operands)
+// (and 32767 at most: slice_columns_kernel's blockIdx.y counts two operands)
 static int64_t sliced_group(int64_t count, int64_t n)
 {
     const int64_t per = 2 * 2 * sliced::plane_values(n, n);
@@ -493,17 +493,18 @@ int adjoint_dev(cudaStream_t s, int64_t count, int64_t n, const double* lam, con
     const int64_t ntiles = (n + sliced::BN - 1) / sliced::BN;
     const float need = (float)(sliced::kLeadFactor * std::sqrt((double)n));
     const unsigned all = (unsigned)count;
-    const unsigned kblocks = (unsigned)((kp / 8 + 255) / 256);
+    const unsigned cblocks = (unsigned)((rows * (kp / 8) + 255) / 256);
+    const unsigned eblocks = (unsigned)((n + sliced::kExpWarps - 1) / sliced::kExpWarps);
     // The FP64 MMA takes the matrices that fall back in one launch each, whatever the groups: by groups the last waves of
     // their tiles cost 3 % of 256 matrices of n = 512.  In a chain (launch_after) the launches that return at
     // once overlap.
     if (cudaMemsetAsync(flag, 0, count * (1 + ntiles) * sizeof(int), s) != cudaSuccess) return SYMEIG_ERR_CUDA;
-    sliced::column_exponents_kernel<<<dim3((unsigned)n, all, 2), 256, 0, s>>>(sliced::Operand{Q, ea, PA, true},
+    sliced::column_exponents_kernel<<<dim3(eblocks, all, 2), 32 * sliced::kExpWarps, 0, s>>>(sliced::Operand{Q, ea, PA, true},
                                                                             sliced::Operand{gQ, eb, PB, false}, n, flag);
     for (int64_t z = 0; z < count; z += group) {
         const unsigned g = (unsigned)std::min<int64_t>(group, count - z);
         const dim3 sgrid((unsigned)ntiles, (unsigned)ntiles, g);
-        launch_after(sliced::slice_columns_kernel, dim3(kblocks, (unsigned)rows, 2 * g), 256, 0, s,
+        launch_after(sliced::slice_columns_kernel, dim3(cblocks, 2 * g), 256, 0, s,
                      sliced::Operand{Q + z * strideQ, ea + z * n, PA, true}, sliced::Operand{gQ + z * strideQ, eb + z * n, PB, false},
                      (int)g, n, rows, kp, pstride, flag + z);
         launch_after(sliced_m_check_kernel, sgrid, sliced::kThreads, sliced::kSmem, s, PA, PB, ea + z * n, eb + z * n, n, rows, kp,
@@ -514,7 +515,7 @@ int adjoint_dev(cudaStream_t s, int64_t count, int64_t n, const double* lam, con
     adjoint_m_kernel<<<grid, kAdjThreads, 0, s>>>(Q, n, gQ, n, lam, glam, n, Mbuf, strideQ, strideQ, strideM, flag);
     launch_after(sliced::row_exponents_kernel, dim3((unsigned)((n + 31) / 32), all), 1024, 0, s, Q, n, ea, flag);
     const sliced::Operand om{Mbuf, eb, PB, false};
-    launch_after(sliced::column_exponents_kernel, dim3((unsigned)n, all, 1), 256, 0, s, om, om, n, flag);
+    launch_after(sliced::column_exponents_kernel, dim3(eblocks, all, 1), 32 * sliced::kExpWarps, 0, s, om, om, n, flag);
     for (int64_t z = 0; z < count; z += group) {
         const unsigned g = (unsigned)std::min<int64_t>(group, count - z);
         const dim3 sgrid((unsigned)ntiles, (unsigned)ntiles, g);
@@ -522,7 +523,7 @@ int adjoint_dev(cudaStream_t s, int64_t count, int64_t n, const double* lam, con
         double* pz = part + z * stridePart;
         launch_after(sliced::slice_rows_kernel, dim3((unsigned)((kp + 63) / 64), (unsigned)((rows + 31) / 32), g), 256, 0, s,
                      Q + z * strideQ, n, ea + z * n, rows, kp, PA, pstride, flag + z);
-        launch_after(sliced::slice_columns_kernel, dim3(kblocks, (unsigned)rows, g), 256, 0, s, oz, oz, (int)g, n, rows, kp, pstride,
+        launch_after(sliced::slice_columns_kernel, dim3(cblocks, g), 256, 0, s, oz, oz, (int)g, n, rows, kp, pstride,
                      flag + z);
         // (pz: the margins, before the partial sums take their place)
         launch_after(sliced_p_check_kernel, sgrid, sliced::kThreads, sliced::kSmem, s, PA, PB, ea + z * n, eb + z * n,

@@ -142,40 +142,44 @@ struct Operand {
     bool must_spread;
 };
 
-// exps[i] of the columns of X (n x n): one block per column, blockIdx.y = matrix.
-static __global__ void __launch_bounds__(256)
+// exps[i] of the columns of X (n x n): one warp per column, blockIdx.y = matrix.  (A block per column, and one per
+// row in slice_columns_kernel, were mostly idle in batches of small orders: 25 of n = 300 844 us, 745 this way.)
+constexpr int kExpWarps = 8;
+static __global__ void __launch_bounds__(32 * kExpWarps)
 column_exponents_kernel(Operand o0, Operand o1, int64_t n, int* __restrict__ flag)
 {
     wait_previous_launch();
-    if (__syncthreads_or(flag[blockIdx.y])) return;
-    __shared__ unsigned long long sh[8];
-    __shared__ double ss[8];
+    const int64_t i = (int64_t)blockIdx.x * kExpWarps + (threadIdx.x >> 5);
+    if (i >= n || __any_sync(0xffffffffu, flag[blockIdx.y])) return;
     const Operand& o = blockIdx.z == 0 ? o0 : o1;
-    const double* x = o.x + (blockIdx.y * n + blockIdx.x) * n;
+    const double* x = o.x + (blockIdx.y * n + i) * n;
     unsigned long long m = 0;
-    double sum = 0.0;
-    for (int64_t k = threadIdx.x; k < n; k += blockDim.x) {
+    double s[4] = {};
+    int64_t k = threadIdx.x & 31;
+    for (; k + 96 < n; k += 128) {
+        double v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = x[k + 32 * u];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            m = max(m, (unsigned long long)__double_as_longlong(v[u]) & 0x7FFFFFFFFFFFFFFFull);
+            if (o.must_spread) s[u] = fma(v[u], v[u], s[u]);
+        }
+    }
+    for (; k < n; k += 32) {
         const double v = x[k];
         m = max(m, (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull);
-        if (o.must_spread) sum = fma(v, v, sum);
+        if (o.must_spread) s[0] = fma(v, v, s[0]);
     }
+    double sum = (s[0] + s[1]) + (s[2] + s[3]);
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
         m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
-        sum += __shfl_xor_sync(0xffffffffu, sum, d);
+        if (o.must_spread) sum += __shfl_xor_sync(0xffffffffu, sum, d);
     }
     if ((threadIdx.x & 31) == 0) {
-        sh[threadIdx.x >> 5] = m;
-        ss[threadIdx.x >> 5] = sum;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < 8; ++w) {
-            m = max(m, sh[w]);
-            sum += ss[w];
-        }
         const int e = magnitude_exponent(m);
-        o.exps[blockIdx.y * n + blockIdx.x] = e;
+        o.exps[blockIdx.y * n + i] = e;
         if (e == kNoScale || (o.must_spread && !spread(__longlong_as_double((long long)m), sum, n))) flag[blockIdx.y] = 1;
     }
 }
@@ -226,20 +230,20 @@ __device__ __forceinline__ int64_t plane_offset(int s, int64_t i, int64_t k0, in
     return ((s * (rows / BM) + i / BM) * (kp / BK) + k0 / BK) * kTileValues + r * BK + ((c ^ (r & 7)) << 3);
 }
 
-// Planes of the columns of X (rows, kp padded; zeros outside).  One thread per 8 inner indices;
-// blockIdx.z = matrix, from `count` on the second operand's.
+// Planes of the columns of X (rows, kp padded; zeros outside).  One thread per 8 inner indices, a column's
+// beside each other; blockIdx.y = matrix, from `count` on the second operand's.
 static __global__ void __launch_bounds__(256)
 slice_columns_kernel(Operand o0, Operand o1, int count, int64_t n, int64_t rows, int64_t kp, int64_t pstride,
                      const int* flag)
 {
     wait_previous_launch();
     wait_previous_launch();
-    const Operand& o = (int)blockIdx.z < count ? o0 : o1;
-    const int64_t z = (int)blockIdx.z < count ? blockIdx.z : blockIdx.z - count;
+    const Operand& o = (int)blockIdx.y < count ? o0 : o1;
+    const int64_t z = (int)blockIdx.y < count ? blockIdx.y : blockIdx.y - count;
     if (flag[z]) return;
-    const int64_t k0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
-    const int64_t i = blockIdx.y;
-    if (k0 >= kp) return;
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t i = t / (kp / 8), k0 = t % (kp / 8) * 8;
+    if (i >= rows) return;
     const double* x = o.x + (z * n + i) * n;
     const int e = i < n ? o.exps[z * n + i] : 0;
     uint32_t out[kPlanes][4];
