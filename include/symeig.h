@@ -260,9 +260,11 @@ int symeig_batched_tuning(int64_t* split, int32_t* shape_small, int32_t* shape_l
  *   lam_i == lam_j), Abar = Q M Q^T, dL/dd_i = Abar_ii, dL/de_i = Abar_{i,i+1} + Abar_{i+1,i}.
  * Q^T gQ and Q M run on the tensor cores with the F-masking and the (off-)diagonal extraction
  * fused into their epilogues; Abar is never formed.  From n = 256 a spread-out Q takes exact bf16
- * slices (tcgen05), any other the FP64 MMA (mma.sync .f64).  The choice is made on the device, per
- * matrix.  Scratch of the handle: 8 bytes per element of the batch, and for the slices up to 44 more
- * for each of at most 512 MiB worth of matrices; without room for these the FP64 MMA runs. */
+ * slices (tcgen05), any other, and one whose gradient the slices would give less accurately, the FP64
+ * MMA (mma.sync .f64).  The choice is made on the device, per matrix.  Scratch of the handle: 8 bytes
+ * per element of the batch, and for the slices 48 more for one matrix or for a group of them with 512 MiB
+ * of planes; above 4 GiB (n = 9450) these are given back after the call.  Without room for them the FP64
+ * MMA runs. */
 int symeig_eig_adjoint_f64(symeig_handle h, int64_t count, int64_t n, const double* lam,
                            const double* Q, const double* glam, const double* gQ, double* gd,
                            double* ge);

@@ -439,22 +439,23 @@ static int64_t sliced_group(int64_t count, int64_t n)
     return std::max<int64_t>(1, std::min(std::min<int64_t>(count, 32767), kSlicedBytes / per));
 }
 
-// The scratch after M and the partials: of a group two operands' planes and the tiles' small sums; of all matrices the
+// The slices' own scratch: of a group two operands' planes and the tiles' small sums; of all matrices the
 // operands' exponents, a flag and a counter a row of tiles.
-static int64_t sliced_scratch_doubles(int64_t count, int64_t n)
+size_t adjoint_planes_bytes(int64_t count, int64_t n)
 {
     const int64_t g = sliced_group(count, n), r = sliced::pad_rows(n);
-    return (g * (2 * sliced::plane_values(n, n) * 2 + r * r * (int64_t)sizeof(double)) +
-            count * (2 * n + 1 + r / sliced::BM) * (int64_t)sizeof(int)) / 8 + 64;
+    return (size_t)(g * (2 * sliced::plane_values(n, n) * 2 + r * r * (int64_t)sizeof(double)) +
+                    count * (2 * n + 1 + r / sliced::BM) * (int64_t)sizeof(int) + 512);
 }
 
 // Device-pointer adjoint for `count` matrices of order n stored back to back (Q, gQ with
 // leading dimension n and stride n*n; lam, glam, gd with stride n; ge with stride n-1).
-// scratch: adjoint_scratch_doubles(count, n, use_sliced) doubles; use_sliced only where adjoint_sliced(n).
+// scratch: adjoint_scratch_doubles(count, n) doubles.  planes: adjoint_planes_bytes(count, n) bytes, only where
+// adjoint_sliced(n), or null for the FP64 MMA.
 // err[0]: the handle's error word; err[1] counts the matrices that took the slices.
 int adjoint_dev(cudaStream_t s, int64_t count, int64_t n, const double* lam, const double* Q,
                 const double* glam, const double* gQ, double* gd, double* ge, double* scratch,
-                bool use_sliced, int* err, int32_t stall)
+                void* planes, int* err, int32_t stall)
 {
     if (count <= 0 || n <= 0) return SYMEIG_OK;
     const int64_t tiles = (n + BN - 1) / BN;
@@ -468,7 +469,7 @@ int adjoint_dev(cudaStream_t s, int64_t count, int64_t n, const double* lam, con
     double* Mbuf = scratch;
     double* part = scratch + count * strideM;
     const dim3 grid((unsigned)tiles, (unsigned)((n + BM - 1) / BM), (unsigned)count);
-    if (!use_sliced) {
+    if (!planes) {
         adjoint_m_kernel<<<grid, kAdjThreads, 0, s>>>(Q, n, gQ, n, lam, glam, n, Mbuf, strideQ, strideQ, strideM, nullptr);
         adjoint_p_kernel<<<grid, kAdjThreads, 0, s>>>(Q, n, Mbuf, n, part, strideQ, strideM, stridePart, nullptr);
         adjoint_reduce_kernel<<<dim3((unsigned)((n + 255) / 256), (unsigned)count), 256, 0, s>>>(part, n, gd, ge, stridePart, nullptr, nullptr);
@@ -482,7 +483,7 @@ int adjoint_dev(cudaStream_t s, int64_t count, int64_t n, const double* lam, con
     const int64_t group = sliced_group(count, n), rows = sliced::pad_rows(n), kp = sliced::pad_k(n);
     const int64_t pstride = sliced::plane_values(n, n);
     // 256-byte aligned: the planes' 16-byte pieces
-    unsigned char* base = (unsigned char*)(((uintptr_t)(part + count * stridePart) + 255) & ~(uintptr_t)255);
+    unsigned char* base = (unsigned char*)(((uintptr_t)planes + 255) & ~(uintptr_t)255);
     __nv_bfloat16* PA = (__nv_bfloat16*)base;
     __nv_bfloat16* PB = PA + group * pstride;
     double* park = (double*)(PB + group * pstride);
@@ -536,10 +537,10 @@ int adjoint_dev(cudaStream_t s, int64_t count, int64_t n, const double* lam, con
     return cudaGetLastError() == cudaSuccess ? SYMEIG_OK : SYMEIG_ERR_CUDA;
 }
 
-int64_t adjoint_scratch_doubles(int64_t count, int64_t n, bool use_sliced)
+int64_t adjoint_scratch_doubles(int64_t count, int64_t n)
 {
     const int64_t tiles = (n + BN - 1) / BN;
-    return count * (n * n + 3 * tiles * n) + (use_sliced ? sliced_scratch_doubles(count, n) : 0);
+    return count * (n * n + 3 * tiles * n);
 }
 
 }  // namespace symeig

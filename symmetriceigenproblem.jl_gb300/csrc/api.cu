@@ -48,6 +48,10 @@ struct DevBuf {
     }
 };
 
+// The adjoint's planes that a handle keeps (48 bytes an element of a matrix: n = 9450).  Above, taking them anew
+// costs a call a few ms of 110 and more.
+static constexpr size_t kKeepPlanes = (size_t)4 << 30;
+
 struct symeig_context {
     int device = 0;
     int sm_count = 0, cc_major = 0, cc_minor = 0;
@@ -65,7 +69,7 @@ struct symeig_context {
     // the column-segment pipeline of the host-pointer apply: per segment, columns copied in and
     // kernel done
     cudaEvent_t seg_in[kPipeBlocks] = {}, seg_done[kPipeBlocks] = {};
-    DevBuf grid[2], thick[2], place[2], table, state, d, e, q, cs, bak, rot, dense, dense_io, bulge, seg_state;
+    DevBuf grid[2], thick[2], place[2], table, state, d, e, q, cs, bak, rot, dense, dense_io, bulge, seg_state, planes;
     int* derr = nullptr;   // device error word (bounded waits), and the adjoint's count of sliced matrices
     int32_t exact_order = 1;  // rotation placement of the qr driver
     int32_t chase_mode = 0;   // symeig_set_chase_mode
@@ -738,7 +742,7 @@ int symeig_destroy(symeig_handle h)
     }
     h->table.release(); h->state.release(); h->d.release(); h->e.release();
     h->q.release(); h->cs.release(); h->bak.release(); h->rot.release();
-    h->dense.release(); h->dense_io.release(); h->bulge.release(); h->seg_state.release();
+    h->dense.release(); h->dense_io.release(); h->bulge.release(); h->seg_state.release(); h->planes.release();
     if (h->ev_main) cudaEventDestroy(h->ev_main);
     for (int b = 0; b < kPipeBlocks; ++b) {
         if (h->pipe[b]) {
@@ -1026,19 +1030,27 @@ int symeig_eig_adjoint_f64_dev(symeig_handle h, int64_t count, int64_t n, const 
     if (count == 0 || n == 0) return SYMEIG_OK;
     if (!lam || !Q || !glam || !gd || (n > 1 && !ge)) return SYMEIG_ERR_NULL;
     begin_call(h);
-    bool use_sliced = gQ && adjoint_sliced(n);
-    if (use_sliced) {
-        const cudaError_t e = h->cs.ensure((size_t)adjoint_scratch_doubles(count, n, true) * sizeof(double));
+    if (gQ) CK(h->cs.ensure((size_t)adjoint_scratch_doubles(count, n) * sizeof(double)));
+    // the slices' planes: kept up to kKeepPlanes, else taken for this call and given back behind it on the stream;
+    // without room for them the FP64 MMA needs M alone
+    void* planes = nullptr;
+    bool give_back = false;
+    if (gQ && adjoint_sliced(n)) {
+        const size_t want = adjoint_planes_bytes(count, n);
+        give_back = want > kKeepPlanes;
+        const cudaError_t e = give_back ? cudaMallocAsync(&planes, want, h->stream) : h->planes.ensure(want);
         if (e == cudaErrorMemoryAllocation) {
-            (void)cudaGetLastError();   // no room for the planes: the FP64 MMA needs M alone
-            use_sliced = false;
+            (void)cudaGetLastError();
+            planes = nullptr;
+            give_back = false;
         } else {
             CK(e);
+            if (!give_back) planes = h->planes.ptr;
         }
     }
-    if (gQ && !use_sliced) CK(h->cs.ensure((size_t)adjoint_scratch_doubles(count, n, false) * sizeof(double)));
     auto t0 = std::chrono::steady_clock::now();
-    rc = adjoint_dev(h->stream, count, n, lam, Q, glam, gQ, gd, ge, (double*)h->cs.ptr, use_sliced, h->derr, h->test_stall);
+    rc = adjoint_dev(h->stream, count, n, lam, Q, glam, gQ, gd, ge, (double*)h->cs.ptr, planes, h->derr, h->test_stall);
+    if (give_back && cudaFreeAsync(planes, h->stream) != cudaSuccess && rc == SYMEIG_OK) rc = SYMEIG_ERR_CUDA;
     h->stats.total_ms =
         std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     return rc;

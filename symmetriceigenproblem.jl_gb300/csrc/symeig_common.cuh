@@ -261,9 +261,10 @@ int batched_autotune(int device, cudaStream_t stream, int64_t count, const int64
 // Adjoint of the eigensolve for count matrices of order n (adjoint.cu).
 int adjoint_dev(cudaStream_t s, int64_t count, int64_t n, const double* lam, const double* Q,
                 const double* glam, const double* gQ, double* gd, double* ge, double* scratch,
-                bool use_sliced, int* err, int32_t stall);
+                void* planes, int* err, int32_t stall);
 bool adjoint_sliced(int64_t n);
-int64_t adjoint_scratch_doubles(int64_t count, int64_t n, bool use_sliced);
+int64_t adjoint_scratch_doubles(int64_t count, int64_t n);
+size_t adjoint_planes_bytes(int64_t count, int64_t n);
 void batched_set_tuning(int fp64, int64_t split, int32_t shape0, int32_t shape1);
 void batched_get_tuning(int fp64, int64_t* split, int32_t* shape0, int32_t* shape1);
 int batched_num_tiles();
