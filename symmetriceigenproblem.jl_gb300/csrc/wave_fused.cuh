@@ -199,10 +199,8 @@ __device__ __forceinline__ bool tile(T* __restrict__ Q, int64_t ldq, int64_t m, 
 #pragma unroll
         for (int a = 0; a < PD; ++a)
 #pragma unroll
-            for (int f = 0; f < F; ++f) {
-                const T* p = q0 + (int64_t)(a * F + f) * ldq;
-                ahead[a][f] = a * F + f < n && in_extent(p) ? *p : T(0);
-            }
+            for (int f = 0; f < F; ++f)
+                ahead[a][f] = a * F + f < n && in_extent(q0 + (int64_t)(a * F + f) * ldq) ? q0[(int64_t)(a * F + f) * ldq] : T(0);
     } else {
         const T* s = state + tid;   // value-major
         const int nt = blockDim.x;
