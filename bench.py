@@ -45,7 +45,7 @@ sys.path.insert(0, str(ROOT))
 
 WORKLOAD = "bulk Givens apply: Q 16384x16384 column-major, k=64 layers of 16383 rotations (cos t, sin t)"
 METRIC = "Givens GFLOP/s (6 flops per rotation per row), bulk apply 16384x16384 k=64"
-TRAFFIC_FILE = ROOT / "profiles" / "wave_apply_f64_16384_k64.md"
+TRAFFIC_FILE = ROOT / "profiles" / "wave_fused.md"
 
 
 def parse_args():
@@ -393,7 +393,7 @@ def run_ours(args):
     if world > 1:
         dist.barrier()
     # each call is synchronous (the copies back are complete when it returns), so each step is
-    # timed on its own; the median of 5 is the value, because a call now and then stalls for
+    # timed on its own; the median of the 5 to 9 is the value, because a call now and then stalls for
     # tens of ms on the host side (measured: 105-109 ms against 72.6 ms, in builds with and
     # without any change to the path), and the mean is reported beside it
     e2e_steps = max(5, min(args.steps, 9))

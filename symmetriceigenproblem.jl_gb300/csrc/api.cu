@@ -3,7 +3,7 @@
 //
 // qr driver.  The reference's outer loop (src/bulge_chasing.jl:166-284) alternates a serial
 // chase that fills a (n-1) x max_layers rotation buffer with a bulk application of that
-// buffer to Q.  Here the chase is a two-warp kernel on a side stream and the apply is the
+// buffer to Q.  Here the chase is one CTA on a side stream and the apply is the
 // wave-window kernel on the main stream, ordered by events: chase f, apply f, chase f+1, ...
 // (the rotation grid is double-buffered so that a concurrent schedule is possible; see the
 // note in the flush loop for why it is not used).  After each chase the host reads its

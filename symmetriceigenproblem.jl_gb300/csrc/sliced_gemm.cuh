@@ -35,8 +35,8 @@
 // in memory as the tensor core wants them, 128 x 64 tiles of 16 KB with the 128-byte swizzle, so one
 // bulk copy brings each.  Four levels at a time have a 128-column accumulator each, so that a plane's
 // tile is read once for all of them, 37 bytes a clock and SM at the tensor core's rate (one product at a
-// time would take 128).  Two products at n = 2047 take 1.73 ms with everything (mma.sync with 128 x 128 tiles of
-// the same operands: 5.4), at n = 4096 10.0 ms, 1240 TFLOP/s in bf16 counted over the whole call.  At
+// time would take 128).  Two products at n = 2047 take 1.84 ms with everything (mma.sync with 128 x 128 tiles of
+// the same operands: 5.4), at n = 4096 10.5 ms.  At
 // n = 2047 256 tiles on 152 SMs are two waves, 84 % full; a tile's own time is the products (256 cycles
 // each, 1440 of them), the sums' way out of TMEM (18 times, between which the tensor core waits) and the
 // epilogue's FP64 division.
@@ -79,8 +79,8 @@ __device__ __forceinline__ int magnitude_exponent(uint64_t abs_bits)
 constexpr int kFixedBits = 6 + 7 * (S - 1);
 
 // x 2^(kFixedBits - e) rounded to an integer (|x| < 2^e, so below 2^62), from the bits: in FP64 the
-// scaling and the conversion kept the slicing kernels on the 2-lane FP64 pipe (80 % busy; the whole adjoint
-// of n = 2047 1.94 ms, 1.73 from the bits).
+// scaling and the conversion kept the slicing kernels on the 2-lane FP64 pipe (80 % busy; 0.2 ms of the whole
+// adjoint of n = 2047).
 __device__ __forceinline__ long long fixed_point(double x, int e)
 {
     const uint64_t b = (uint64_t)__double_as_longlong(x);
