@@ -237,7 +237,6 @@ slice_columns_kernel(Operand o0, Operand o1, int count, int64_t n, int64_t rows,
                      const int* flag)
 {
     wait_previous_launch();
-    wait_previous_launch();
     const Operand& o = (int)blockIdx.y < count ? o0 : o1;
     const int64_t z = (int)blockIdx.y < count ? blockIdx.y : blockIdx.y - count;
     if (flag[z]) return;
@@ -269,6 +268,7 @@ slice_rows_kernel(const double* __restrict__ X, int64_t n, const int* exps, int6
                   __nv_bfloat16* __restrict__ planes, int64_t pstride,
                   const int* flag)
 {
+    wait_previous_launch();
     if (flag[blockIdx.z]) return;
     __shared__ double tile[64][33];   // [inner][row]
     const int64_t i0 = (int64_t)blockIdx.y * 32, k0 = (int64_t)blockIdx.x * 64;

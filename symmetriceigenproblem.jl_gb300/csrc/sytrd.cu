@@ -17,7 +17,7 @@
 // nothing but these three orders waits on the whole grid, and each sum is split over enough
 // threads that no thread chains more than about 16 FP64 operations of 64 cycles.  At the sizes
 // that fit L2 the reduction is bound by these latencies, not by the FP64 pipe: n = 1300 takes
-// 28.0 ms (with programmatic dependent launches, which hide 5 us a column of launch latency),
+// 27.0 ms (with programmatic dependent launches, which hide 6 us a column of launch latency),
 // against 165 ms for six launches a column with one thread per row and a block reduction per
 // earlier reflector.
 // The trailing update is one FP64 tensor-core GEMM (dmma_tile.cuh) of inner dimension 2 pb.

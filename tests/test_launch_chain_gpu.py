@@ -27,6 +27,23 @@ def test_dense_reduction_repeats(cuda, pkg, n):
         assert all(np.array_equal(x, y) for x, y in zip(o, out[0]))
 
 
+def test_adjoint_groups(cuda, pkg):
+    """Four groups of planes with matrices that fall back among them: each has its bits alone."""
+    n, count = 512, 160
+    gen = cuda.Generator(device="cuda")
+    gen.manual_seed(n * 7 + count)
+    rnd = lambda *s: cuda.randn(*s, generator=gen, dtype=cuda.float64, device="cuda")  # noqa: E731
+    Q, lam, glam, gQ = (rnd(count, n, n) / n ** 0.5).transpose(1, 2), rnd(count, n), rnd(count, n), rnd(count, n, n).transpose(1, 2)
+    h = pkg.Handle(0)
+    runs = [pkg.eig_adjoint(lam, Q, glam, gQ, handle=h) for _ in range(3)]
+    assert 0 < h.adjoint_sliced() < count
+    for z in range(count):
+        gd, ge = pkg.eig_adjoint(lam[z], Q[z], glam[z], gQ[z], handle=h)
+        for bd, be in runs:
+            assert cuda.equal(bd[z], gd) and cuda.equal(be[z], ge), z
+    h.close()
+
+
 @pytest.mark.parametrize("n", [256, 257, 300, 513])
 def test_adjoint_repeats(cuda, pkg, n):
     rng = np.random.default_rng(n)
