@@ -15,6 +15,6 @@ def test_every_chained_kernel_waits_first(pkg):
         body = re.search(r"\b%s\([^)]*\)\s*\{(.*?)\n\}" % name, text, re.S).group(1)
         declarations, _, rest = body.partition("wait_previous_launch();")
         assert rest, name
-        # before it only declarations: shared memory and the names of constants
+        # before it only shared memory and indices of the block
         for line in filter(None, map(str.strip, declarations.splitlines())):
-            assert re.match(r"(extern )?__shared__ [^=]*;$|constexpr ", line), (name, line)
+            assert re.match(r"(extern )?__shared__ [^=]*;$|const int64_t \w+ = blockIdx\.\w;$", line), (name, line)
