@@ -418,10 +418,10 @@ __global__ void adjoint_lambda_only_kernel(const double* __restrict__ Q, int64_t
 }  // namespace
 
 // From this order on the products run on the bf16 tensor cores where Q is spread out.  FP64 MMA against
-// sliced, one matrix: n = 256 694 / 335 us, 300 810 / 354, 512 1304 / 428, 1000 4693 / 634, 2047 32.8 / 1.89 ms;
-// 25 of n = 300 3612 / 745 us, 256 of n = 512 127 / 13.6 ms.  A localized Q pays for the question and the kernels that return
-// at once: 20 us of 700 at n = 256, 24 of 810 at 300, 28 of 4690 at 1000, 0.6 ms of 127 for 256 of n = 512; below
-// n = 256 it would be above 3 %.  The rule leaves the count out, so that a matrix has the same bits
+// sliced, one matrix: n = 256 694 / 344 us, 300 810 / 363, 512 1304 / 427, 1000 4693 / 641, 2047 32.8 / 1.89 ms;
+// 25 of n = 300 3612 / 757 us, 256 of n = 512 127.5 / 14.0 ms.  A localized Q pays for the question and the kernels that
+// return at once: about 25 us, of 700 at n = 256 and 4690 at 1000, 0.3 ms of 127.5 for 256 of n = 512; below
+// n = 256 it would be above 4 %.  The rule leaves the count out, so that a matrix has the same bits
 // alone and in a batch.
 static constexpr int64_t kSlicedMin = 256;
 // Matrices sliced at once: their planes take at most this many bytes (one matrix always fits).

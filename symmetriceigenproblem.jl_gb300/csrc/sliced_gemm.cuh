@@ -35,8 +35,8 @@
 // in memory as the tensor core wants them, 128 x 64 tiles of 16 KB with the 128-byte swizzle, so one
 // bulk copy brings each.  Four levels at a time have a 128-column accumulator each, so that a plane's
 // tile is read once for all of them, 37 bytes a clock and SM at the tensor core's rate (one product at a
-// time would take 128).  Two products at n = 2047 take 1.84 ms with everything (mma.sync with 128 x 128 tiles of
-// the same operands: 5.4), at n = 4096 10.5 ms.  At
+// time would take 128).  Two products at n = 2047 take 1.85 ms with everything (mma.sync with 128 x 128 tiles of
+// the same operands: 5.4), at n = 4096 10.6 ms.  At
 // n = 2047 256 tiles on 152 SMs are two waves, 84 % full; a tile's own time is the products (256 cycles
 // each, 1440 of them), the sums' way out of TMEM (18 times, between which the tensor core waits) and the
 // epilogue's FP64 division.
@@ -143,7 +143,7 @@ struct Operand {
 };
 
 // exps[i] of the columns of X (n x n): one warp per column, blockIdx.y = matrix.  (A block per column, and one per
-// row in slice_columns_kernel, were mostly idle in batches of small orders: 25 of n = 300 844 us, 745 this way.)
+// row in slice_columns_kernel, were mostly idle in batches of small orders: 25 of n = 300 844 us, 757 this way.)
 constexpr int kExpWarps = 8;
 static __global__ void __launch_bounds__(32 * kExpWarps)
 column_exponents_kernel(Operand o0, Operand o1, int64_t n, int* __restrict__ flag)
